@@ -667,8 +667,72 @@ static void collect_stage_ms(t2b_ctx* c)
 
 namespace t2b {
 
+// Copies between a caller's device arrays and a staging slot, one launch: part blockIdx.y.
+// Bound by launch latency below about 10 MB (a batch of 64 at box 128 is 3.4 MB), by HBM above
+// (500 particles, 26 MB in: 11 us).  Without it the captured graph held the caller's addresses, and
+// each batch in new buffers was captured and instantiated again: 0.26 ms of host time for a plain
+// E-step, 1.0 ms for a learned one of 2.4 ms, which the GPU waited for.
+constexpr int MAX_PARTS = 20;   // the result arrays
+struct CopyParts {
+    const void* src[MAX_PARTS];
+    void* dst[MAX_PARTS];
+    size_t bytes[MAX_PARTS];   // multiples of 4: every array holds 4- or 8-byte values
+};
+__global__ void __launch_bounds__(256) k_copy_parts(CopyParts c)
+{
+    const void* src = c.src[blockIdx.y];
+    void* dst = c.dst[blockIdx.y];
+    const size_t bytes = c.bytes[blockIdx.y];
+    const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    size_t done = 0;
+    // 16-byte moves where both arrays allow them (any torch or cudaMalloc allocation), the rest by words
+    if ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) {
+        const size_t nv = bytes / 16;
+        for (size_t i = i0; i < nv; i += step) static_cast<uint4*>(dst)[i] = static_cast<const uint4*>(src)[i];
+        done = nv * 4;
+    }
+    for (size_t i = done + i0; i < bytes / 4; i += step)
+        static_cast<uint32_t*>(dst)[i] = static_cast<const uint32_t*>(src)[i];
+}
+
+struct PartList {
+    CopyParts c{};
+    int n = 0;
+    size_t largest = 0;
+    void add(void* dst, const void* src, size_t bytes)
+    {
+        if (!dst || !src || bytes == 0) return;
+        c.src[n] = src;
+        c.dst[n] = dst;
+        c.bytes[n++] = bytes;
+        largest = std::max(largest, bytes);
+    }
+    void launch(cudaStream_t st) const
+    {
+        if (n == 0) return;
+        const int bx = (int)std::min<size_t>(296, std::max<size_t>(1, (largest / 16 + 255) / 256));
+        k_copy_parts<<<dim3(bx, n), 256, 0, st>>>(c);
+        T2B_CUDA(cudaGetLastError());
+    }
+};
+
+// the batch's inputs and results live in staging slot `in`
+static void use_slot(Work& w, const t2b_ctx::InSlot& in, bool nomask)
+{
+    w.fimg = in.fimg;
+    w.fimg_nm = nomask ? in.fimg_nm : in.fimg;   // no separate unmasked image: the masked one serves both
+    w.ctf = in.ctf;
+    w.minv = in.minv;
+    w.scal = in.scal;
+    w.r_min = in.r_min; w.r_sum = in.r_sum; w.r_sig = in.r_sig; w.r_csum = in.r_csum; w.r_csig = in.r_csig;
+    w.r_pmax = in.r_pmax; w.r_nsign = in.r_nsign; w.r_ncsig = in.r_ncsig; w.r_pose = in.r_pose;
+    w.r_norm = in.r_norm; w.r_sumw = in.r_sumw; w.r_sig_off = in.r_sig_off; w.r_sigma2 = in.r_sigma2;
+    w.r_pdf_class = in.r_pdf_class; w.r_pdf_dir = in.r_pdf_dir; w.status = in.status;
+    w.r_learned = in.r_learned; w.r_audit = in.r_audit; w.r_xa = in.r_xa; w.r_aa = in.r_aa;
+}
+
 // Enqueue the batch in `w` on `st` as a CUDA graph: captured once per key
-// (batch shape, buffers, stream, proposal settings) into slot `g`, replayed
+// (batch shape, slot, proposal settings) into slot `g`, replayed
 // afterwards.  Returns the kernel nodes of the graph.
 static int replay_graph(t2b_ctx* c, Work& w, cudaStream_t st, const std::vector<const void*>& key,
                         t2b_ctx::GraphSlot& g)
@@ -722,16 +786,7 @@ static long long submit_host(t2b_ctx* c, const t2b_batch* b, const t2b_result* r
     Work w = c->wk;
     const int n = b->n, P = c->tb.P;
     w.n = n;
-    w.fimg = in.fimg;
-    w.fimg_nm = b->fimg_nomask ? in.fimg_nm : in.fimg;   // no separate unmasked image: the masked one serves both
-    w.ctf = in.ctf;
-    w.minv = in.minv;
-    w.scal = in.scal;
-    w.r_min = in.r_min; w.r_sum = in.r_sum; w.r_sig = in.r_sig; w.r_csum = in.r_csum; w.r_csig = in.r_csig;
-    w.r_pmax = in.r_pmax; w.r_nsign = in.r_nsign; w.r_ncsig = in.r_ncsig; w.r_pose = in.r_pose;
-    w.r_norm = in.r_norm; w.r_sumw = in.r_sumw; w.r_sig_off = in.r_sig_off; w.r_sigma2 = in.r_sigma2;
-    w.r_pdf_class = in.r_pdf_class; w.r_pdf_dir = in.r_pdf_dir; w.status = in.status;
-    w.r_learned = in.r_learned; w.r_audit = in.r_audit; w.r_xa = in.r_xa; w.r_aa = in.r_aa;
+    use_slot(w, in, b->fimg_nomask != nullptr);
     T2B_CUDA(cudaStreamWaitEvent(cs, in.consumed, 0));
     T2B_CUDA(cudaMemcpyAsync(in.fimg, b->fimg, (size_t)n * P * sizeof(float2), cudaMemcpyHostToDevice, cs));
     if (b->fimg_nomask)
@@ -860,32 +915,65 @@ int t2b_estep_batch_device(t2b_ctx* c, const t2b_batch* b, const t2b_result* r, 
         }
         Work w = c->wk;
         w.n = b->n;
-        w.fimg = (const float2*)b->fimg;
-        w.fimg_nm = (const float2*)(b->fimg_nomask ? b->fimg_nomask : b->fimg);
-        w.ctf = b->ctf;
-        w.minv = b->minvsigma2;
-        w.scal = b->scalars;
-        w.r_min = r->min_diff2; w.r_sum = r->sum_weight; w.r_sig = r->sig_weight;
-        w.r_csum = r->coarse_sum_weight; w.r_csig = r->coarse_sig_weight; w.r_pmax = r->pmax;
-        w.r_nsign = r->nr_sign; w.r_ncsig = r->n_coarse_sig; w.r_pose = r->pose;
-        w.r_norm = r->wsum_norm; w.r_sumw = r->sumw; w.r_sig_off = r->wsum_sigma2_offset;
-        w.r_sigma2 = r->wsum_sigma2; w.r_pdf_class = r->wsum_pdf_class; w.r_pdf_dir = r->wsum_pdf_dir;
-        w.status = r->status;
-        w.r_learned = r->learned;
-        w.r_audit = r->audit_mass;
-        w.r_xa = r->wsum_scale_xa;
-        w.r_aa = r->wsum_scale_aa;
         if (c->cfg.use_graph) {
-            const std::vector<const void*> key = {(const void*)(intptr_t)b->n, b->fimg, b->fimg_nomask, b->ctf,
-                                                  b->minvsigma2, b->scalars, r->min_diff2, r->sum_weight, r->sig_weight,
-                                                  r->coarse_sum_weight, r->coarse_sig_weight, r->nr_sign,
-                                                  r->n_coarse_sig, r->pmax, r->pose, r->wsum_norm, r->sumw,
-                                                  r->wsum_sigma2_offset, r->wsum_sigma2, r->wsum_pdf_class,
-                                                  r->wsum_pdf_dir, r->status, r->learned, r->audit_mass,
-                                                  r->wsum_scale_xa, r->wsum_scale_aa, (const void*)st,
+            // staged through the slot the next host batch would take: that slot's last batch has run
+            // (stream order) and its results must have left it; the next host batch's input copies
+            // wait for `consumed`.  The graph holds the slot's addresses, so a batch in other buffers
+            // replays it too.
+            t2b_ctx::InSlot& in = c->in[c->submitted & 1];
+            use_slot(w, in, b->fimg_nomask != nullptr);
+            const size_t n = b->n, P = c->tb.P, K = c->tb.K;
+            T2B_CUDA(cudaStreamWaitEvent(st, in.done, 0));
+            PartList pin;
+            pin.add(in.fimg, b->fimg, n * P * sizeof(float2));
+            pin.add(in.fimg_nm, b->fimg_nomask, n * P * sizeof(float2));
+            pin.add(in.ctf, b->ctf, n * P * sizeof(float));
+            pin.add(in.minv, b->minvsigma2, n * P * sizeof(float));
+            pin.add(in.scal, b->scalars, n * 8 * sizeof(double));
+            pin.launch(st);
+            const std::vector<const void*> key = {(const void*)(intptr_t)n, (const void*)w.fimg_nm,
                                                   (const void*)(intptr_t)(c->net && c->net->enabled ? c->net->kprop : 0)};
-            c->last_kernels = replay_graph(c, w, st, key, c->g_dev);
+            c->last_kernels = replay_graph(c, w, st, key, in.gd);
+            PartList po;
+            po.add(r->min_diff2, in.r_min, n * sizeof(double));
+            po.add(r->sum_weight, in.r_sum, n * sizeof(double));
+            po.add(r->sig_weight, in.r_sig, n * sizeof(double));
+            po.add(r->coarse_sum_weight, in.r_csum, n * sizeof(double));
+            po.add(r->coarse_sig_weight, in.r_csig, n * sizeof(double));
+            po.add(r->nr_sign, in.r_nsign, n * sizeof(long long));
+            po.add(r->n_coarse_sig, in.r_ncsig, n * sizeof(long long));
+            po.add(r->pmax, in.r_pmax, n * sizeof(double));
+            po.add(r->pose, in.r_pose, n * 5 * sizeof(int));
+            po.add(r->wsum_norm, in.r_norm, n * sizeof(double));
+            po.add(r->sumw, in.r_sumw, n * sizeof(double));
+            po.add(r->wsum_sigma2_offset, in.r_sig_off, n * sizeof(double));
+            po.add(r->wsum_sigma2, in.r_sigma2, n * (c->cfg.ori_size / 2 + 1) * sizeof(double));
+            po.add(r->wsum_pdf_class, in.r_pdf_class, n * K * sizeof(double));
+            po.add(r->wsum_pdf_dir, in.r_pdf_dir, n * K * c->tb.n_dir * sizeof(double));
+            po.add(r->status, in.status, n * sizeof(int));
+            po.add(r->learned, in.r_learned, n * sizeof(int));
+            if (c->net && c->net->enabled && c->net->ready)   // written by the audit only
+                po.add(r->audit_mass, in.r_audit, n * sizeof(double));
+            po.add(r->wsum_scale_xa, in.r_xa, n * sizeof(double));
+            po.add(r->wsum_scale_aa, in.r_aa, n * sizeof(double));
+            po.launch(st);
+            T2B_CUDA(cudaEventRecord(in.consumed, st));
         } else {
+            w.fimg = (const float2*)b->fimg;
+            w.fimg_nm = (const float2*)(b->fimg_nomask ? b->fimg_nomask : b->fimg);
+            w.ctf = b->ctf;
+            w.minv = b->minvsigma2;
+            w.scal = b->scalars;
+            w.r_min = r->min_diff2; w.r_sum = r->sum_weight; w.r_sig = r->sig_weight;
+            w.r_csum = r->coarse_sum_weight; w.r_csig = r->coarse_sig_weight; w.r_pmax = r->pmax;
+            w.r_nsign = r->nr_sign; w.r_ncsig = r->n_coarse_sig; w.r_pose = r->pose;
+            w.r_norm = r->wsum_norm; w.r_sumw = r->sumw; w.r_sig_off = r->wsum_sigma2_offset;
+            w.r_sigma2 = r->wsum_sigma2; w.r_pdf_class = r->wsum_pdf_class; w.r_pdf_dir = r->wsum_pdf_dir;
+            w.status = r->status;
+            w.r_learned = r->learned;
+            w.r_audit = r->audit_mass;
+            w.r_xa = r->wsum_scale_xa;
+            w.r_aa = r->wsum_scale_aa;
             enqueue_estep(c, w, st, true, true);
             c->last_kernels = -1;
         }

@@ -316,10 +316,9 @@ struct t2b_ctx {
     int last_n = 0;                           // particles of the last batch
     struct GraphSlot {                        // a captured batch and what it was captured for
         cudaGraphExec_t exec = nullptr;
-        std::vector<const void*> key;         // shape / buffers / stream / proposal settings
+        std::vector<const void*> key;         // shape / stream / proposal settings
         int kernels = -1;                     // its kernel nodes
     };
-    GraphSlot g_dev;                          // device entry point
     // Host entry points: two staging slots, each with the batch inputs and results.  A
     // batch's inputs are copied into its slot on copy_stream while the previous batch
     // computes on `stream`, and its results leave the slot on d2h_stream while the next one
@@ -338,7 +337,8 @@ struct t2b_ctx {
         cudaEvent_t copied = nullptr;         // inputs in the slot (copy_stream)
         cudaEvent_t consumed = nullptr;       // the slot's batch has run (stream)
         cudaEvent_t done = nullptr;           // the slot's results are in host memory (d2h_stream)
-        GraphSlot g;                          // the captured batch of this slot
+        GraphSlot g;                          // the captured batch of this slot (host entry points)
+        GraphSlot gd;                         // ... and of the device entry point, staged through it
     } in[2];
     cudaStream_t copy_stream = nullptr;
     cudaStream_t d2h_stream = nullptr;
@@ -356,7 +356,7 @@ struct t2b_ctx {
     bool stage_timing = false;                // host batches run uncaptured with stage events
     void drop_graphs()
     {
-        for (GraphSlot* g : {&g_dev, &in[0].g, &in[1].g}) {
+        for (GraphSlot* g : {&in[0].g, &in[1].g, &in[0].gd, &in[1].gd}) {
             if (g->exec) cudaGraphExecDestroy(g->exec);
             g->exec = nullptr;
             g->key.clear();
