@@ -130,7 +130,7 @@ void t2b_destroy(t2b_ctx* c)
         for (auto p : c->mdl) cudaFree(p);
         for (auto p : c->gdata) cudaFree(p);
         for (auto p : c->gweight) cudaFree(p);
-        cudaFree(c->sym_scratch);
+        cudaFree(c->ms_scratch);
         for (auto& ev : c->ev) cudaEventDestroy(ev);
         for (auto& ev : c->handoff) cudaEventDestroy(ev);
         for (auto& s : c->in)
@@ -159,6 +159,7 @@ int t2b_projector_set(t2b_ctx* c, int iclass, int ref_dim, int xdim, int ydim, i
         v.inity = inity; v.initz = initz; v.r_max = r_max; v.pad = pad;
         if (c->mdl[iclass] && c->mvol[iclass].nvox() != v.nvox()) { cudaFree(c->mdl[iclass]); c->mdl[iclass] = nullptr; }
         if (!c->mdl[iclass]) {
+            c->release_scratch();
             void* p = nullptr;
             if (cudaMalloc(&p, v.nvox() * sizeof(float2)) != cudaSuccess) {
                 cudaGetLastError();
@@ -194,6 +195,7 @@ int t2b_backprojector_init(t2b_ctx* c, int iclass, int ref_dim, int xdim, int yd
             c->gdata[iclass] = nullptr; c->gweight[iclass] = nullptr;
         }
         if (!c->gdata[iclass]) {
+            c->release_scratch();
             void *p = nullptr, *q = nullptr;
             if (cudaMalloc(&p, v.nvox() * sizeof(float2)) != cudaSuccess || cudaMalloc(&q, v.nvox() * sizeof(float)) != cudaSuccess) {
                 cudaGetLastError();
@@ -286,6 +288,7 @@ int t2b_configure(t2b_ctx* c, const t2b_config* cfg)
         DeviceGuard g(c->device);
         c->quiesce();
         free_allocs(c);
+        c->release_scratch();
         proposal_invalidate(c);
         estep_init_attributes();
         if (f.diff2_mode == T2B_DIFF2_SPLIT_BF16) tc_init_attributes();
@@ -1276,17 +1279,17 @@ int t2b_reconstruct_divide(t2b_ctx* c, int iclass, double* fconv)
         const int ps = v.ydim, fx = ps / 2 + 1;
         const size_t total = (size_t)ps * ps * fx;
         double2* fc = nullptr;
-        double *fw = nullptr, *rad = nullptr;
+        double* rad = nullptr;
         cudaStream_t st = c->stream;
-        auto cleanup = [&] { cudaFree(fc); cudaFree(fw); cudaFree(rad); };
-        if (cudaMalloc(&fc, total * sizeof(double2)) != cudaSuccess || cudaMalloc(&fw, total * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&rad, 2 * (size_t)v.r_max * sizeof(double)) != cudaSuccess) {
+        auto cleanup = [&] { cudaFree(fc); cudaFree(rad); };
+        if (cudaMalloc(&fc, total * sizeof(double2)) != cudaSuccess ||
+            cudaMalloc(&rad, 3 * (size_t)v.r_max * sizeof(double)) != cudaSuccess) {
             cudaGetLastError();
             cleanup();
             throw Error{T2B_ERR_NOMEM, "reconstruction buffers"};
         }
         try {
-            launch_reconstruct(v, c->gdata[iclass], c->gweight[iclass], fc, fw, rad, rad + v.r_max, st);
+            launch_reconstruct(v, c->gdata[iclass], c->gweight[iclass], fc, rad, rad + v.r_max, st);
             T2B_CUDA(cudaMemcpyAsync(fconv, fc, total * sizeof(double2), cudaMemcpyDeviceToHost, st));
             T2B_CUDA(cudaStreamSynchronize(st));
         } catch (...) {

@@ -18,6 +18,7 @@
 //             prior sums, then trilinear backprojection with float2 atomics
 //             (src/ml_optimiser.cpp:8153-8700, src/backprojector.cpp:55-230)
 #include "t2b_internal.cuh"
+#include "shells.cuh"
 #include "project_pixel.cuh"
 #include <map>
 #include <algorithm>
@@ -1741,52 +1742,33 @@ __global__ void k_results(Tables tb, Work w)
 }
 
 // --------------------------------------------------- reconstruction (FP64)
-__global__ void k_decenter(Volume g, const float2* __restrict__ data, const float* __restrict__ weight,
-                           double2* __restrict__ fconv, double* __restrict__ fw, double* rad, double* cnt,
-                           const double* __restrict__ tau2, double tscale, int minres_map)
+// per shell (floor of r / pad, r < r_max pad): sum of the weights and count, into acc[2 shell]
+__global__ void __launch_bounds__(256) k_radial(Volume g, const float* __restrict__ weight, double* __restrict__ acc,
+                                                const double* __restrict__ inv_tau2, int minres_map)
 {
-    const int ps = g.ydim, fx = ps / 2 + 1, nz = g.ref_dim == 3 ? ps : 1;   // 2D grids: one plane
-    const long long total = (long long)nz * ps * fx;
-    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= total) return;
-    const int j = (int)(n % fx);
-    const int i = (int)((n / fx) % ps);
-    const int k = (int)(n / ((long long)fx * ps));
-    const int kp = k < fx ? k : k - ps, ip = i < fx ? i : i - ps, jp = j;
+    extern __shared__ double sb[];
     const int rp = g.r_max * g.pad;
-    const int r2 = kp * kp + ip * ip + jp * jp;
-    double2 v = make_double2(0., 0.);
-    double wv = 0.;
-    if (r2 <= rp * rp) {
-        const size_t src = ((size_t)(kp - g.initz) * g.ydim + (ip - g.inity)) * g.xdim + jp;
-        const float2 d = data[src];
-        v = make_double2(d.x, d.y);
-        wv = weight[src];
-    }
-    // MAP term: the inverse tau2 spectrum added to the weight (src/backprojector.cpp:1412-1455)
-    if (tau2 && r2 < rp * rp) {
-        const double rr = sqrt((double)r2) / g.pad;
-        const int im = rr > 0 ? (int)(rr + 0.5) : (int)(rr - 0.5);
-        const double t = tau2[im];
-        const double invtau2 = t > 0. ? 1. / (tscale * t) : (wv > 1e-20 ? 1. / (0.001 * wv) : 0.);
-        if (im >= minres_map) wv += invtau2;
-    }
-    fconv[n] = v;
-    fw[n] = wv;
-    if (r2 < rp * rp) {
-        const int ires = (int)floor(sqrt((double)r2) / g.pad);
-        atomicAdd(&rad[ires], wv);
-        atomicAdd(&cnt[ires], 1.);
-    }
+    shell_sums<2>(g, rp * rp, g.r_max, sb, acc, [&](int r2) { return shell_floor(r2, g.pad); },
+                  [&](long long n, int r2, int, double* x) {
+                      const double w = weight[n];
+                      x[0] = inv_tau2 ? map_weight(w, r2, g.pad, inv_tau2, minres_map) : w;
+                      x[1] = 1.;
+                  });
 }
 
-__global__ void k_radnorm(int r_max, double* rad, const double* cnt)
+// sum, count -> average / 1000 (rad[shell])
+__global__ void k_radnorm(int r_max, double* rad, const double* acc)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < r_max && (cnt[i] > 0. || rad[i] > 0.)) rad[i] /= 1000. * cnt[i];
+    if (i >= r_max) return;
+    const double s = acc[2 * i], n = acc[2 * i + 1];
+    rad[i] = n > 0. || s > 0. ? s / (1000. * n) : s;
 }
 
-__global__ void k_divide(Volume g, double2* __restrict__ fconv, const double* __restrict__ fw, const double* rad)
+// the pad_size transform in FFTW layout, divided by max(weight, radial average / 1000); zero
+// outside ROUND(r_max pad)
+__global__ void k_divide(Volume g, const float2* __restrict__ data, const float* __restrict__ weight,
+                         double2* __restrict__ fconv, const double* __restrict__ rad)
 {
     const int ps = g.ydim, fx = ps / 2 + 1, nz = g.ref_dim == 3 ? ps : 1;
     const long long total = (long long)nz * ps * fx;
@@ -1796,15 +1778,15 @@ __global__ void k_divide(Volume g, double2* __restrict__ fconv, const double* __
     const int i = (int)((n / fx) % ps);
     const int k = (int)(n / ((long long)fx * ps));
     const int kp = k < fx ? k : k - ps, ip = i < fx ? i : i - ps;
-    const int r2 = kp * kp + ip * ip + j * j;
-    const int ires = (int)floor(sqrt((double)r2) / g.pad);
-    const double wv = fmax(fw[n], rad[ires < g.r_max ? ires : g.r_max - 1]);
-    if (wv != 0.) {
-        double2 v = fconv[n];
-        v.x /= wv;
-        v.y /= wv;
-        fconv[n] = v;
+    const int rp = g.r_max * g.pad, r2 = kp * kp + ip * ip + j * j;
+    double2 v = make_double2(0., 0.);
+    if (r2 <= rp * rp) {
+        const size_t src = ((size_t)(kp - g.initz) * g.ydim + (ip - g.inity)) * g.xdim + j;
+        const float2 d = data[src];
+        const double wv = fmax((double)weight[src], rad[min(shell_floor(r2, g.pad), g.r_max - 1)]);
+        v = wv != 0. ? make_double2(d.x / wv, d.y / wv) : make_double2(d.x, d.y);
     }
+    fconv[n] = v;
 }
 
 int sm_count()
@@ -2034,30 +2016,25 @@ void launch_wsum_bp(const Tables& tb, const Work& w, const Volume& g, float2* co
     T2B_CUDA(cudaGetLastError());
 }
 
-void launch_reconstruct(const Volume& g, const float2* data, const float* weight, double2* fconv,
-                        double* fw, double* rad, double* cnt, cudaStream_t st, const double* tau2, double tscale,
-                        int minres_map)
+// rad[r_max]: the radial averages / 1000 of the weights (with the MAP term when inv_tau2 is given); acc: 2 r_max
+void launch_radial(const Volume& g, const float* weight, double* rad, double* acc, cudaStream_t st,
+                   const double* inv_tau2, int minres_map)
 {
-    const int ps = g.ydim, fx = ps / 2 + 1, nz = g.ref_dim == 3 ? ps : 1;
-    const long long total = (long long)nz * ps * fx;
-    T2B_CUDA(cudaMemsetAsync(rad, 0, sizeof(double) * g.r_max, st));
-    T2B_CUDA(cudaMemsetAsync(cnt, 0, sizeof(double) * g.r_max, st));
-    const int nb = (int)((total + 255) / 256);
-    k_decenter<<<nb, 256, 0, st>>>(g, data, weight, fconv, fw, rad, cnt, tau2, tscale, minres_map);
-    k_radnorm<<<(g.r_max + 255) / 256, 256, 0, st>>>(g.r_max, rad, cnt);
-    k_divide<<<nb, 256, 0, st>>>(g, fconv, fw, rad);
+    T2B_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double) * g.r_max, st));
+    const long long items = (long long)g.zdim * g.ydim * ((g.xdim + RUN - 1) / RUN);
+    const int nb = (int)std::min<long long>((items + 255) / 256, 8LL * sm_count());
+    k_radial<<<nb, 256, 2 * g.r_max * sizeof(double), st>>>(g, weight, acc, inv_tau2, minres_map);
+    k_radnorm<<<(g.r_max + 255) / 256, 256, 0, st>>>(g.r_max, rad, acc);
     T2B_CUDA(cudaGetLastError());
 }
 
-void launch_decenter(const Volume& g, const float2* data, const float* weight, double2* fconv, double* fw,
-                     double* rad, double* cnt, cudaStream_t st, const double* tau2, double tscale, int minres_map)
+void launch_reconstruct(const Volume& g, const float2* data, const float* weight, double2* fconv, double* rad,
+                        double* acc, cudaStream_t st)
 {
     const int ps = g.ydim, fx = ps / 2 + 1, nz = g.ref_dim == 3 ? ps : 1;
     const long long total = (long long)nz * ps * fx;
-    T2B_CUDA(cudaMemsetAsync(rad, 0, sizeof(double) * g.r_max, st));
-    T2B_CUDA(cudaMemsetAsync(cnt, 0, sizeof(double) * g.r_max, st));
-    k_decenter<<<(int)((total + 255) / 256), 256, 0, st>>>(g, data, weight, fconv, fw, rad, cnt, tau2, tscale,
-                                                          minres_map);
+    launch_radial(g, weight, rad, acc, st);
+    k_divide<<<(int)((total + 255) / 256), 256, 0, st>>>(g, data, weight, fconv, rad);
     T2B_CUDA(cudaGetLastError());
 }
 

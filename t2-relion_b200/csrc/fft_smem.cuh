@@ -65,6 +65,25 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 
+// A sequence of N points lies padded in shared memory: point i at px(i), sequences fft_ld(N) apart.
+// A power-of-two radix writes its first stage's outputs R apart, which without the padding lands on
+// the same banks (16 ways for radix 16), and fft_ld is odd, so copies that walk the sequences
+// fastest do not collide either.
+// The odd boxes of the gridding iterations (plans with any prime) have odd radices only and lie
+// unpadded, N apart (PAD = false).
+__host__ __device__ constexpr int px(int i) { return i + (i >> 4); }
+__host__ __device__ constexpr int fft_ld(int N) { return (N + (N >> 4)) | 1; }
+template <bool PAD> __device__ __forceinline__ int pxp(int i) { return PAD ? px(i) : i; }
+template <bool PAD> __device__ __forceinline__ int ldp(int N) { return PAD ? fft_ld(N) : N; }
+
+// e / d for 0 <= e < 65536 by one multiplication (the sizes here are run-time values; an integer
+// division is some 20 instructions, and a butterfly needs three)
+struct FastDiv {
+    unsigned d, m;
+    __device__ __forceinline__ explicit FastDiv(int x) : d((unsigned)x), m(x > 1 ? 0xffffffffu / (unsigned)x + 1u : 0u) {}
+    __device__ __forceinline__ int div(int e) const { return d == 1 ? e : (int)__umulhi((unsigned)e, m); }
+};
+
 template <bool INV>
 __device__ __forceinline__ float2 twid(const float2* tw, int t)
 {
@@ -72,16 +91,26 @@ __device__ __forceinline__ float2 twid(const float2* tw, int t)
     return INV ? make_float2(w.x, -w.y) : w;
 }
 
-// DFT of R points in registers: out[q] = sum_r v[r] W^{q r}, W = e^{-+2 pi i / R}
-// (tw[t] = e^{-2 pi i t / N}, NR = N / R).
-template <int R, bool INV>
-__device__ __forceinline__ void dft_small(float2* v, const float2* tw, int NR)
+// e^{-+2 pi i k / 16} (k a constant once unrolled)
+template <bool INV>
+__device__ __forceinline__ float2 root16(int k)
 {
-    if (R == 2) {
+    constexpr float C[5] = {1.f, 0.92387953251128675613f, 0.70710678118654752440f, 0.38268343236508977173f, 0.f};
+    const int q = k & 15, a = q & 7, m = a <= 4 ? a : 8 - a;       // cos(pi a / 8) up to its sign
+    float c = a <= 4 ? C[m] : -C[m], s = a <= 4 ? C[4 - m] : C[4 - m];   // a in 0..7: sin >= 0
+    if (q >= 8) { c = -c; s = -s; }
+    return make_float2(c, INV ? s : -s);
+}
+
+// DFT of R points in registers: out[q] = sum_r v[r] W^{q r}, W = e^{-+2 pi i / R}.
+template <int R, bool INV>
+__device__ __forceinline__ void dft_small(float2* v)
+{
+    if constexpr (R == 2) {
         const float2 a = v[0], b = v[1];
         v[0] = cadd(a, b);
         v[1] = csub(a, b);
-    } else if (R == 4) {
+    } else if constexpr (R == 4) {
         const float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]);
         const float2 c = cadd(v[1], v[3]), d = csub(v[1], v[3]);
         // forward: X1 = b - i d, X3 = b + i d; inverse swaps them
@@ -90,24 +119,24 @@ __device__ __forceinline__ void dft_small(float2* v, const float2* tw, int NR)
         v[2] = csub(a, c);
         v[1] = cadd(b, mid);
         v[3] = csub(b, mid);
-    } else if (R == 8) {
+    } else if constexpr (R == 8) {
         // 8 = 2 x 4: DFT4 of the even and odd points, X[k] = E[k] + W8^k O[k], X[k+4] = E[k] - W8^k O[k]
         float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-        dft_small<4, INV>(e, tw, NR);
-        dft_small<4, INV>(o, tw, NR);
+        dft_small<4, INV>(e);
+        dft_small<4, INV>(o);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float2 t = k == 0 ? o[0] : cmul(o[k], twid<INV>(tw, k * NR));
+            const float2 t = k == 0 ? o[0] : cmul(o[k], root16<INV>(2 * k));
             v[k] = cadd(e[k], t);
             v[k + 4] = csub(e[k], t);
         }
-    } else if (R == 16) {
+    } else if constexpr (R == 16) {
         // 16 = 4 x 4: Y_l = DFT4 over m of v[4m + l]; X[k1 + 4 k2] = DFT4 over l of W16^{l k1} Y_l[k1]
         float2 y[4][4];
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
             float2 t[4] = {v[l], v[4 + l], v[8 + l], v[12 + l]};
-            dft_small<4, INV>(t, tw, NR);
+            dft_small<4, INV>(t);
 #pragma unroll
             for (int k1 = 0; k1 < 4; ++k1) y[l][k1] = t[k1];
         }
@@ -115,19 +144,49 @@ __device__ __forceinline__ void dft_small(float2* v, const float2* tw, int NR)
         for (int k1 = 0; k1 < 4; ++k1) {
             float2 z[4];
 #pragma unroll
-            for (int l = 0; l < 4; ++l) z[l] = (l * k1 == 0) ? y[l][k1] : cmul(y[l][k1], twid<INV>(tw, l * k1 * NR));
-            dft_small<4, INV>(z, tw, NR);
+            for (int l = 0; l < 4; ++l) z[l] = (l * k1 == 0) ? y[l][k1] : cmul(y[l][k1], root16<INV>(l * k1));
+            dft_small<4, INV>(z);
 #pragma unroll
             for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = z[k2];
         }
     } else {
-        float2 o[R];
+        // odd R in conjugate output pairs: with S_r = v_r + v_{R-r}, D_r = v_r - v_{R-r},
+        // X_u, X_{R-u} = v_0 + sum_r cos(2 pi u r / R) S_r -+ i sum_r sin(2 pi u r / R) D_r
+        // (upper signs forward): (R - 1)^2 multiply-adds and no table reads, where R (R - 1)
+        // complex products with a twiddle load each stood before
+        static_assert(R == 3 || R == 5 || R == 7, "register DFT size");
+        constexpr int H = (R - 1) / 2;
+        constexpr float C3[1] = {-0.5f}, S3[1] = {0.86602540378443864676f};
+        constexpr float C5[2] = {0.30901699437494742410f, -0.80901699437494742410f};
+        constexpr float S5[2] = {0.95105651629515357212f, 0.58778525229247312917f};
+        constexpr float C7[3] = {0.62348980185873353053f, -0.22252093395631440429f, -0.90096886790241912624f};
+        constexpr float S7[3] = {0.78183148246802980871f, 0.97492791218182360702f, 0.43388373911755812048f};
+        float2 S[H], D[H], o[R];
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-            float2 acc = v[0];
+        for (int r = 0; r < H; ++r) {
+            S[r] = cadd(v[r + 1], v[R - 1 - r]);
+            D[r] = csub(v[r + 1], v[R - 1 - r]);
+        }
+        o[0] = v[0];
 #pragma unroll
-            for (int r = 1; r < R; ++r) acc = cadd(acc, cmul(v[r], twid<INV>(tw, ((q * r) % R) * NR)));
-            o[q] = acc;
+        for (int r = 0; r < H; ++r) o[0] = cadd(o[0], S[r]);
+#pragma unroll
+        for (int u = 1; u <= H; ++u) {
+            float2 A = v[0], B = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int r = 1; r <= H; ++r) {
+                const int t = (u * r) % R, k = t <= H ? t : R - t;   // cos even, sin odd about R / 2
+                const float c = R == 3 ? C3[k - 1] : R == 5 ? C5[R == 5 ? k - 1 : 0] : C7[R == 7 ? k - 1 : 0];
+                const float s0 = R == 3 ? S3[k - 1] : R == 5 ? S5[R == 5 ? k - 1 : 0] : S7[R == 7 ? k - 1 : 0];
+                const float sn = t <= H ? s0 : -s0;
+                A.x = fmaf(c, S[r - 1].x, A.x);
+                A.y = fmaf(c, S[r - 1].y, A.y);
+                B.x = fmaf(sn, D[r - 1].x, B.x);
+                B.y = fmaf(sn, D[r - 1].y, B.y);
+            }
+            const float2 mib = make_float2(B.y, -B.x);   // -i B
+            o[u] = INV ? csub(A, mib) : cadd(A, mib);
+            o[R - u] = INV ? cadd(A, mib) : csub(A, mib);
         }
 #pragma unroll
         for (int q = 0; q < R; ++q) v[q] = o[q];
@@ -135,115 +194,181 @@ __device__ __forceinline__ void dft_small(float2* v, const float2* tw, int NR)
 }
 
 // One Stockham stage over nfft sequences of length N: a -> b.
-template <int R, bool INV>
+template <int R, bool INV, bool PAD>
 __device__ __forceinline__ void fft_stage(const float2* a, float2* b, int nfft, int N, int Ns, const float2* tw)
 {
-    const int NR = N / R;
+    const int NR = N / R, LD = ldp<PAD>(N);
     const int tstride = N / (Ns * R);
+    const FastDiv dnr(NR), dns(Ns);
     for (int e = threadIdx.x; e < nfft * NR; e += blockDim.x) {
-        const int f = e / NR, j = e - f * NR;
-        const float2* in = a + f * N;
-        float2* out = b + f * N;
-        const int k = j % Ns;
+        const int f = dnr.div(e), j = e - f * NR;
+        const float2* in = a + f * LD;
+        float2* out = b + f * LD;
+        const int jq = dns.div(j), k = j - jq * Ns;
         float2 v[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = in[j + r * NR];
+        for (int r = 0; r < R; ++r) v[r] = in[pxp<PAD>(j + r * NR)];
+        if (Ns > 1) {
 #pragma unroll
-        for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twid<INV>(tw, k * r * tstride));
-        dft_small<R, INV>(v, tw, NR);
-        const int base = (j / Ns) * Ns * R + k;
+            for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twid<INV>(tw, k * r * tstride));
+        }
+        dft_small<R, INV>(v);
+        const int base = jq * Ns * R + k;
 #pragma unroll
-        for (int r = 0; r < R; ++r) out[base + r * Ns] = v[r];
+        for (int r = 0; r < R; ++r) out[pxp<PAD>(base + r * Ns)] = v[r];
     }
 }
 
 // The same stage for a radix R known only at run time (a prime >= 7): one thread per output,
 // X[m Ns R + q Ns + k] = sum_r in[m Ns + k + r N/R] e^{-+2 pi i (k r N/(Ns R) + (q r mod R) N/R) / N},
 // the Stockham twiddle and the length-R DFT's root folded into one table entry.
-template <bool INV>
+template <bool INV, bool PAD>
 __device__ __forceinline__ void fft_stage_gen(const float2* a, float2* b, int nfft, int N, int Ns, int R,
                                               const float2* tw)
 {
-    const int NR = N / R;
+    const int NR = N / R, LD = ldp<PAD>(N);
     const int tstride = N / (Ns * R);
     for (int e = threadIdx.x; e < nfft * N; e += blockDim.x) {
         const int f = e / N, o = e - f * N;
         const int k = o % Ns, q = (o / Ns) % R, m = o / (Ns * R);
-        const float2* in = a + f * N + m * Ns + k;
+        const float2* in = a + f * LD;
+        const int i0 = m * Ns + k;
         float2 acc = make_float2(0.f, 0.f);
         int qr = 0;   // (q r) mod R
         for (int r = 0; r < R; ++r) {
             int t = k * r * tstride + qr * NR;
             if (t >= N) t -= N;
-            acc = cadd(acc, cmul(in[r * NR], twid<INV>(tw, t)));
+            acc = cadd(acc, cmul(in[pxp<PAD>(i0 + r * NR)], twid<INV>(tw, t)));
             qr += q;
             if (qr >= R) qr -= R;
         }
-        b[f * N + o] = acc;
+        b[f * LD + pxp<PAD>(o)] = acc;
     }
 }
 
-// The first stage (Ns = 1: no input twiddles) for an odd prime radix R >= 7: one thread per
-// (sequence, group m, pair u), X[u] and X[R - u] from the same sums over r = 1 .. (R - 1) / 2 of
-// S_r = x_r + x_{R-r} and D_r = x_r - x_{R-r}: X[u] = x_0 + A -+ i B, X[R - u] = x_0 + A +- i B
-// with A = sum_r cos(2 pi u r / R) S_r, B = sum_r sin(2 pi u r / R) D_r (upper signs forward);
-// u = 0 gives X[0] = x_0 + sum_r S_r.  About a quarter of the generic stage's loads and products.
-template <bool INV>
+// The first stage (Ns = 1: no input twiddles) for an odd prime radix R > 7: X[u] and X[R - u]
+// from the same sums over r = 1 .. h = (R - 1) / 2 of S_r = x_r + x_{R-r} and D_r = x_r - x_{R-r}:
+// X[u] = x_0 + A -+ i B, X[R - u] = x_0 + A +- i B with A = sum_r cos(2 pi u r / R) S_r,
+// B = sum_r sin(2 pi u r / R) D_r (upper signs forward); X[0] = x_0 + sum_r S_r.
+// Bound by shared-memory reads.  One thread takes PF_U consecutive u of two sequences (f and
+// f + nfft / 2; nfft even), so the two loads of an r serve PF_U pairs and each (cos, sin) entry two
+// sequences; u is the slowest index, so the lanes of a warp share their u and the entries come as
+// broadcast 16-byte reads: from `tab`, [r - 1][u - 1], when it is full (R <= PF_TAB_MAX), else entry
+// (u r mod R) of R entries.  The sums are FP64 (the FP64 units are otherwise idle, and an FP64 pair is
+// the width of the reads already): the half-box transforms of the gridding iterations lose the
+// averaging over both halves that the full box had, and this stage is the one with long sums.
+constexpr int PF_U = 5;
+constexpr int PF_TAB_MAX = 43;
+
+template <bool INV, bool TAB>
 __device__ __forceinline__ void fft_stage_prime_first(const float2* a, float2* b, int nfft, int N, int R,
-                                                      const float2* tw)
+                                                      const double2* tab)
 {
-    const int NR = N / R, h = (R - 1) / 2, per = NR * (h + 1);
-    for (int e = threadIdx.x; e < nfft * per; e += blockDim.x) {
-        const int f = e / per, rem = e - f * per;
-        const int m = rem / (h + 1), u = rem - m * (h + 1);
-        const float2* in = a + f * N + m;
-        float2* out = b + f * N + m * R;
-        const float2 x0 = in[0];
-        float2 A = make_float2(0.f, 0.f), Bs = make_float2(0.f, 0.f);
-        int ur = 0;   // (u r) mod R
+    const int NR = N / R, h = (R - 1) / 2, nub = (h + PF_U - 1) / PF_U, half = nfft / 2, per = half * NR;
+    const FastDiv dper(per), dnr(NR);
+    for (int e = threadIdx.x; e < per * nub; e += blockDim.x) {
+        const int ub = dper.div(e), rem = e - ub * per;
+        const int f = dnr.div(rem), m = rem - f * NR;
+        const int u0 = 1 + ub * PF_U, nu = min(PF_U, h - ub * PF_U);
+        const float2* in0 = a + f * N + m;
+        const float2* in1 = in0 + half * N;
+        double2 A0[PF_U], B0[PF_U], A1[PF_U], B1[PF_U];
+        double2 s0 = make_double2(0., 0.), s1 = s0;
+        int ur[PF_U];
+#pragma unroll
+        for (int i = 0; i < PF_U; ++i) {
+            A0[i] = B0[i] = A1[i] = B1[i] = make_double2(0., 0.);
+            ur[i] = 0;
+        }
         for (int r = 1; r <= h; ++r) {
-            ur += u;
-            if (ur >= R) ur -= R;
-            const float2 xr = in[r * NR], xm = in[(R - r) * NR];
-            const float2 S = cadd(xr, xm), D = csub(xr, xm);
-            const float2 w = tw[ur * NR];   // (cos, -sin) of 2 pi u r / R
-            A.x = fmaf(w.x, S.x, A.x);
-            A.y = fmaf(w.x, S.y, A.y);
-            Bs.x = fmaf(-w.y, D.x, Bs.x);
-            Bs.y = fmaf(-w.y, D.y, Bs.y);
+            const float2 p0 = in0[r * NR], q0 = in0[(R - r) * NR], p1 = in1[r * NR], q1 = in1[(R - r) * NR];
+            const double px0 = p0.x, py0 = p0.y, qx0 = q0.x, qy0 = q0.y, px1 = p1.x, py1 = p1.y, qx1 = q1.x, qy1 = q1.y;
+            const double2 S0 = make_double2(px0 + qx0, py0 + qy0), D0 = make_double2(px0 - qx0, py0 - qy0);
+            const double2 S1 = make_double2(px1 + qx1, py1 + qy1), D1 = make_double2(px1 - qx1, py1 - qy1);
+            s0.x += S0.x; s0.y += S0.y;
+            s1.x += S1.x; s1.y += S1.y;
+#pragma unroll
+            for (int i = 0; i < PF_U; ++i) {
+                if (i >= nu) break;
+                int k;
+                if (TAB) {
+                    k = (r - 1) * h + u0 - 1 + i;
+                } else {
+                    ur[i] += u0 + i;
+                    if (ur[i] >= R) ur[i] -= R;
+                    k = ur[i];
+                }
+                const double2 w = tab[k];   // (cos, sin) of 2 pi u r / R
+                A0[i].x = fma(w.x, S0.x, A0[i].x);
+                A0[i].y = fma(w.x, S0.y, A0[i].y);
+                B0[i].x = fma(w.y, D0.x, B0[i].x);
+                B0[i].y = fma(w.y, D0.y, B0[i].y);
+                A1[i].x = fma(w.x, S1.x, A1[i].x);
+                A1[i].y = fma(w.x, S1.y, A1[i].y);
+                B1[i].x = fma(w.y, D1.x, B1[i].x);
+                B1[i].y = fma(w.y, D1.y, B1[i].y);
+            }
         }
-        const float2 c0 = cadd(x0, A);
-        if (u == 0) {
-            out[0] = c0;
-        } else {
-            const float2 mib = make_float2(Bs.y, -Bs.x);   // -i B
-            out[u] = INV ? csub(c0, mib) : cadd(c0, mib);
-            out[R - u] = INV ? cadd(c0, mib) : csub(c0, mib);
-        }
+        const auto emit = [&](const float2* in, float2* out, const double2* A, const double2* B, double2 sum) {
+            const double x = in[0].x, y = in[0].y;
+            if (ub == 0) out[0] = make_float2((float)(x + sum.x), (float)(y + sum.y));
+            const double sg = INV ? -1. : 1.;
+#pragma unroll
+            for (int i = 0; i < PF_U; ++i) {
+                if (i >= nu) break;
+                const double cx = x + A[i].x, cy = y + A[i].y, bx = sg * B[i].y, by = -sg * B[i].x;   // -+ i B
+                out[u0 + i] = make_float2((float)(cx + bx), (float)(cy + by));
+                out[R - u0 - i] = make_float2((float)(cx - bx), (float)(cy - by));
+            }
+        };
+        emit(in0, b + f * N + m * R, A0, B0, s0);
+        emit(in1, b + (f + half) * N + m * R, A1, B1, s1);
     }
+}
+
+// The table of fft_stage_prime_first for the plan's first radix: entries of 2 pi k / R,
+// by the CTA into shared memory (before the barrier that precedes the transform)
+__device__ __forceinline__ void fft_prime_table(double2* tab, const FftPlan& pl)
+{
+    const int R = pl.rad[0], h = (R - 1) / 2;
+    if (R <= 7) return;
+    const bool full = R <= PF_TAB_MAX;
+    for (int e = threadIdx.x; e < (full ? h * h : R); e += blockDim.x) {
+        const int k = full ? ((e / h + 1) * (e % h + 1)) % R : e;
+        double sn, cs;
+        sincospi(2. * k / R, &sn, &cs);
+        tab[e] = make_double2(cs, sn);
+    }
+}
+inline int fft_prime_table_entries(const FftPlan& pl)
+{
+    const int R = pl.nst ? pl.rad[0] : 0, h = (R - 1) / 2;
+    return R <= 7 ? 0 : R <= PF_TAB_MAX ? h * h : R;
 }
 
 // All stages; returns the buffer holding the transform (natural order).  PRIMES (the plans of
 // fft_plan(N, true)): the radix-7 register stage and the first-stage pairs for larger primes,
 // compiled only into the kernels that take such plans (they cost the others registers).
 template <bool INV, bool PRIMES = false>
-__device__ float2* fft_smem(float2* a, float2* b, int nfft, const FftPlan& pl, const float2* tw)
+__device__ float2* fft_smem(float2* a, float2* b, int nfft, const FftPlan& pl, const float2* tw,
+                            const double2* ptab = nullptr)
 {
     int Ns = 1;
     for (int st = 0; st < pl.nst; ++st) {
         const int R = pl.rad[st];
         switch (R) {
-        case 4: fft_stage<4, INV>(a, b, nfft, pl.n, Ns, tw); break;
-        case 2: fft_stage<2, INV>(a, b, nfft, pl.n, Ns, tw); break;
-        case 3: fft_stage<3, INV>(a, b, nfft, pl.n, Ns, tw); break;
-        case 5: fft_stage<5, INV>(a, b, nfft, pl.n, Ns, tw); break;
+        case 4: fft_stage<4, INV, !PRIMES>(a, b, nfft, pl.n, Ns, tw); break;
+        case 2: fft_stage<2, INV, !PRIMES>(a, b, nfft, pl.n, Ns, tw); break;
+        case 3: fft_stage<3, INV, !PRIMES>(a, b, nfft, pl.n, Ns, tw); break;
+        case 5: fft_stage<5, INV, !PRIMES>(a, b, nfft, pl.n, Ns, tw); break;
         default:
             if constexpr (PRIMES) {
-                if (R == 7) fft_stage<7, INV>(a, b, nfft, pl.n, Ns, tw);
-                else if (Ns == 1) fft_stage_prime_first<INV>(a, b, nfft, pl.n, R, tw);
-                else fft_stage_gen<INV>(a, b, nfft, pl.n, Ns, R, tw);
+                if (R == 7) fft_stage<7, INV, false>(a, b, nfft, pl.n, Ns, tw);
+                else if (Ns == 1 && R <= PF_TAB_MAX) fft_stage_prime_first<INV, true>(a, b, nfft, pl.n, R, ptab);
+                else if (Ns == 1) fft_stage_prime_first<INV, false>(a, b, nfft, pl.n, R, ptab);
+                else fft_stage_gen<INV, false>(a, b, nfft, pl.n, Ns, R, tw);
             } else {
-                fft_stage_gen<INV>(a, b, nfft, pl.n, Ns, R, tw);
+                fft_stage_gen<INV, true>(a, b, nfft, pl.n, Ns, R, tw);
             }
             break;
         }
@@ -281,24 +406,66 @@ constexpr int ct_ns(int N, int st)
 template <int R, bool INV, int N, int Ns>
 __device__ __forceinline__ void fft_stage_ct(const float2* a, float2* b, int nfft, const float2* tw)
 {
-    constexpr int NR = N / R;
+    constexpr int NR = N / R, LD = fft_ld(N);
     constexpr int tstride = N / (Ns * R);
     for (int e = threadIdx.x; e < nfft * NR; e += blockDim.x) {
         const int f = e / NR, j = e - f * NR;
-        const float2* in = a + f * N;
-        float2* out = b + f * N;
+        const float2* in = a + f * LD;
+        float2* out = b + f * LD;
         const int k = j % Ns;
         float2 v[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = in[j + r * NR];
+        for (int r = 0; r < R; ++r) v[r] = in[px(j + r * NR)];
         if (Ns > 1) {
 #pragma unroll
             for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twid<INV>(tw, k * r * tstride));
         }
-        dft_small<R, INV>(v, tw, NR);
+        dft_small<R, INV>(v);
         const int base = (j / Ns) * Ns * R + k;
 #pragma unroll
-        for (int r = 0; r < R; ++r) out[base + r * Ns] = v[r];
+        for (int r = 0; r < R; ++r) out[px(base + r * Ns)] = v[r];
+    }
+}
+
+// The transforms of one warp's NF sequences in place, the size known at compile time: every lane
+// loads all its butterflies of a stage before any is stored, so one buffer and __syncwarp do
+template <int R, bool INV, int N, int Ns, int NF>
+__device__ __forceinline__ void fft_stage_warp(float2* a, const float2* tw, int lane)
+{
+    constexpr int NR = N / R, LD = fft_ld(N), TOT = NF * NR, K = (TOT + 31) / 32;
+    constexpr int tstride = N / (Ns * R);
+    float2 v[K][R];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int e = lane + 32 * k;
+        if (TOT % 32 && e >= TOT) break;
+        const int f = e / NR, j = e - f * NR;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[k][r] = a[f * LD + px(j + r * NR)];
+        if (Ns > 1) {
+#pragma unroll
+            for (int r = 1; r < R; ++r) v[k][r] = cmul(v[k][r], twid<INV>(tw, (j % Ns) * r * tstride));
+        }
+        dft_small<R, INV>(v[k]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int e = lane + 32 * k;
+        if (TOT % 32 && e >= TOT) break;
+        const int f = e / NR, j = e - f * NR;
+        const int base = (j / Ns) * Ns * R + j % Ns;
+#pragma unroll
+        for (int r = 0; r < R; ++r) a[f * LD + px(base + r * Ns)] = v[k][r];
+    }
+    __syncwarp();
+}
+template <int N, bool INV, int NF, int ST = 0>
+__device__ __forceinline__ void fft_warp(float2* a, const float2* tw, int lane)
+{
+    if constexpr (ct_radix(N, ST) != 0) {
+        fft_stage_warp<ct_radix(N, ST), INV, N, ct_ns(N, ST), NF>(a, tw, lane);
+        fft_warp<N, INV, NF, ST + 1>(a, tw, lane);
     }
 }
 

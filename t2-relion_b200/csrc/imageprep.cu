@@ -16,8 +16,8 @@
 //   (CTF::getFftwImage without padding), Minvsigma2.
 //
 // Layout: one 2D transform = a row pass and a column pass, each a batch of 1D
-// FFTs held in shared memory (mixed-radix Stockham, radices 4, 2, 3, 5; any
-// even N = 2^a 3^b 5^c up to 512).  The row pass transforms the masked and the
+// FFTs held in shared memory (mixed-radix Stockham, radices 16 to 2, 3 and 5;
+// any even N = 2^a 3^b 5^c up to 512, each with its own compiled kernels).  The row pass transforms the masked and the
 // unmasked row together as one complex sequence (masked + i * unmasked) and
 // separates the two half spectra; the column pass only transforms the N/2 + 1
 // columns of the half spectrum.  The intermediate half spectra stay in L2.
@@ -43,9 +43,7 @@ constexpr int PREP_THREADS = 256;
 struct ImagePrep {
     t2b_prep_config cfg{};
     int N = 0, h = 0, s = 0, hs = 0, P = 0, max_batch = 0;
-    int rpb = 0, cpb = 0, ncol_blocks = 0;
-    bool fused = false;            // one CTA per particle (k_noise_fused, k_prep_fused)
-    FftPlan plan{};
+    bool fused = false;            // one CTA per particle (k_prep_fused)
     double minv_dc = 0.;
     float2* tw = nullptr;          // N twiddles e^{-2 pi i t / N}
     double* noise_sig = nullptr;   // h: sqrt(sigma2_fudge * remapped sigma2_noise)
@@ -55,7 +53,6 @@ struct ImagePrep {
     float2* gm = nullptr;          // max_batch x N x h  masked half spectra (rows transformed)
     float2* gu = nullptr;          // max_batch x N x h  unmasked
     float2* gn = nullptr;          // max_batch x N x h  noise (columns transformed)
-    float* noise = nullptr;        // max_batch x N x N  noise images
     float* pw = nullptr;           // max_batch x N x h  |F|^2 of the masked transform
     double* bg = nullptr;          // max_batch          average background
     // host batch staging
@@ -104,8 +101,7 @@ __device__ __forceinline__ float2 noise_value(unsigned long long key, unsigned l
 }
 
 struct PrepArgs {
-    FftPlan plan;
-    int N, h, s, hs, P, rpb, cpb;
+    int N, h, s, hs, P;
     int zero_mask, do_ctf;
     int premult, do_abs, flip, intact;
     long long seed;
@@ -125,7 +121,6 @@ struct PrepArgs {
     float2* gm;
     float2* gu;
     float2* gn;
-    float* noise;
     float* pw;
     double* bg;
     float* fimg;
@@ -141,70 +136,6 @@ constexpr int NPAR = T2B_PREP_NPARAM;
 __device__ __forceinline__ void load_tw(float2* s_tw, const float2* tw, int N)
 {
     for (int t = threadIdx.x; t < N; t += blockDim.x) s_tw[t] = tw[t];
-}
-
-// ------------------------------------------------------------ noise image
-// columns: spectrum of the noise (rows i, columns kx), inverse FFT over y
-__global__ void __launch_bounds__(PREP_THREADS) k_noise_cols(PrepArgs a)
-{
-    extern __shared__ float2 sm[];
-    const int N = a.N, h = a.h, C = a.cpb;
-    float2* s_tw = sm;
-    float2* b0 = sm + N;
-    float2* b1 = b0 + C * N;
-    const int p = blockIdx.x, j0 = blockIdx.y * C;
-    load_tw(s_tw, a.tw, N);
-    const unsigned long long key = splitmix64((unsigned long long)(a.seed + a.pid[p]));
-    for (int e = threadIdx.x; e < C * N; e += blockDim.x) {
-        const int c = e % C, i = e / C, j = j0 + c;
-        float2 v = make_float2(0.f, 0.f);
-        if (j < h) {
-            const int ky = i < h ? i : i - N;
-            const int ires = ring_of(ky, j);
-            if (ires < h) v = noise_value(key, (unsigned long long)i * h + j, (float)a.noise_sig[ires]);
-        }
-        b0[c * N + i] = v;
-    }
-    __syncthreads();
-    const float2* r = fft_smem<true>(b0, b1, C, a.plan, s_tw);
-    float2* out = a.gn + (size_t)p * N * h;
-    for (int e = threadIdx.x; e < C * N; e += blockDim.x) {
-        const int c = e % C, i = e / C, j = j0 + c;
-        if (j < h) out[(size_t)i * h + j] = r[c * N + i];
-    }
-}
-
-// rows: Hermitian extension (imaginary parts of kx = 0 and N/2 dropped), inverse FFT over x
-__global__ void __launch_bounds__(PREP_THREADS) k_noise_rows(PrepArgs a)
-{
-    extern __shared__ float2 sm[];
-    const int N = a.N, h = a.h, R = a.rpb;
-    float2* s_tw = sm;
-    float2* b0 = sm + N;
-    float2* b1 = b0 + R * N;
-    const int p = blockIdx.x, y0 = blockIdx.y * R;
-    load_tw(s_tw, a.tw, N);
-    const float2* g = a.gn + (size_t)p * N * h;
-    for (int e = threadIdx.x; e < R * N; e += blockDim.x) {
-        const int rr = e / N, k = e - rr * N, y = y0 + rr;
-        float2 v = make_float2(0.f, 0.f);
-        if (y < N) {
-            if (k == 0 || k == N / 2) v = make_float2(g[(size_t)y * h + k].x, 0.f);
-            else if (k < N / 2) v = g[(size_t)y * h + k];
-            else {
-                const float2 w = g[(size_t)y * h + (N - k)];
-                v = make_float2(w.x, -w.y);
-            }
-        }
-        b0[e] = v;
-    }
-    __syncthreads();
-    const float2* r = fft_smem<true>(b0, b1, R, a.plan, s_tw);
-    float* out = a.noise + (size_t)p * N * N;
-    for (int e = threadIdx.x; e < R * N; e += blockDim.x) {
-        const int rr = e / N, x = e - rr * N, y = y0 + rr;
-        if (y < N) out[(size_t)y * N + x] = r[e].x;
-    }
 }
 
 // ------------------------------------------------------------ pixel helpers
@@ -242,9 +173,17 @@ __device__ __forceinline__ float mask_weight(const PrepArgs& a, int x, int y)
     return 0.5f + 0.5f * cospif((rp - r) / a.width);
 }
 
-// average background of the zero-mask path (softMaskOutsideMap without a noise
-// image): sum of the weights and weighted pixels outside the radius; fixed-order
-// reduction in FP64
+// ------------------------------------------------------------ two-pass path (boxes above 128)
+// The half spectra go through memory (L2): columns of the noise spectrum, rows, columns, ring sums.
+// A warp transforms its sequences in place (fft_warp); a column block stages COLS columns, so that
+// memory sees 128-byte rows of them.  With run-time radix-4 stages for the whole block, and the noise
+// image and its rows in kernels of their own, 160 particles of box 256 took 604 us; 246 now.
+constexpr int COLS = 16;                                                    // columns of a block
+constexpr int BG_PARTS = 8;                                                 // blocks of a particle's background sums
+constexpr int warp_seqs(int N) { return N <= 256 ? 2 : 1; }                 // sequences of a warp at a time
+
+// partial sums (weights, weighted pixels) of the average background outside the mask
+// (softMaskOutsideMap without a noise image): rows y = part, part + BG_PARTS, ..., fixed-order FP64
 __global__ void __launch_bounds__(PREP_THREADS) k_background(PrepArgs a)
 {
     __shared__ double s_w[PREP_THREADS], s_v[PREP_THREADS];
@@ -252,13 +191,13 @@ __global__ void __launch_bounds__(PREP_THREADS) k_background(PrepArgs a)
     const PixelCtx c = pixel_ctx(a, p);
     const float* img = a.img + (size_t)p * N * N;
     double sw = 0., sv = 0.;
-    for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
-        const int y = e / N, x = e - y * N;
-        const float w = mask_weight(a, x, y);
-        if (w < 0.f) continue;
-        sw += w;
-        sv += (double)w * shifted_pixel(a, img, c, x, y);
-    }
+    for (int y = blockIdx.y; y < N; y += BG_PARTS)
+        for (int x = threadIdx.x; x < N; x += PREP_THREADS) {
+            const float w = mask_weight(a, x, y);
+            if (w < 0.f) continue;
+            sw += w;
+            sv += (double)w * shifted_pixel(a, img, c, x, y);
+        }
     s_w[threadIdx.x] = sw;
     s_v[threadIdx.x] = sv;
     __syncthreads();
@@ -269,51 +208,131 @@ __global__ void __launch_bounds__(PREP_THREADS) k_background(PrepArgs a)
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) a.bg[p] = s_w[0] > 0. ? s_v[0] / s_w[0] : 0.;
+    if (threadIdx.x == 0) {
+        a.bg[2 * (p * BG_PARTS + blockIdx.y)] = s_w[0];
+        a.bg[2 * (p * BG_PARTS + blockIdx.y) + 1] = s_v[0];
+    }
 }
 
-// ------------------------------------------------------------ row pass
-// z = masked + i * unmasked, forward FFT over x, split into the two half spectra
-__global__ void __launch_bounds__(PREP_THREADS) k_rows(PrepArgs a)
+// the block's COLS sequences in W, transformed by its warps
+template <int N, bool INV>
+__device__ __forceinline__ void fft_columns(float2* W, const float2* s_tw)
 {
+    constexpr int NF = warp_seqs(N), LD = fft_ld(N);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int c = warp * NF; c < COLS; c += PREP_THREADS / 32 * NF) fft_warp<N, INV, NF>(W + c * LD, s_tw, lane);
+}
+
+// noise: spectrum (rows i, columns kx), inverse FFT over y
+template <int N>
+__global__ void __launch_bounds__(PREP_THREADS) k_noise_cols(PrepArgs a)
+{
+    constexpr int h = N / 2 + 1, LD = fft_ld(N);
     extern __shared__ float2 sm[];
-    const int N = a.N, h = a.h, R = a.rpb;
     float2* s_tw = sm;
-    float2* b0 = sm + N;
-    float2* b1 = b0 + R * N;
-    const int p = blockIdx.x, y0 = blockIdx.y * R;
+    float2* W = sm + N;
+    const int p = blockIdx.x, j0 = blockIdx.y * COLS;
     load_tw(s_tw, a.tw, N);
-    const PixelCtx c = pixel_ctx(a, p);
-    const float* img = a.img + (size_t)p * N * N;
-    const float bgv = a.zero_mask ? (float)a.bg[p] : 0.f;
-    const float* noise = a.zero_mask ? nullptr : a.noise + (size_t)p * N * N;
-    for (int e = threadIdx.x; e < R * N; e += blockDim.x) {
-        const int rr = e / N, x = e - rr * N, y = y0 + rr;
+    const unsigned long long key = splitmix64((unsigned long long)(a.seed + a.pid[p]));
+    for (int e = threadIdx.x; e < COLS * N; e += PREP_THREADS) {
+        const int c = e % COLS, i = e / COLS, j = j0 + c;
+        const int ky = i < h ? i : i - N;
         float2 v = make_float2(0.f, 0.f);
-        if (y < N) {
-            const float u = shifted_pixel(a, img, c, x, y);
-            const float w = mask_weight(a, x, y);
-            float m = u;
-            if (w >= 0.f) {
-                const float fill = a.zero_mask ? bgv : noise[(size_t)y * N + x];
-                m = (w >= 1.f) ? fill : (1.f - w) * u + w * fill;
-            }
-            v = make_float2(m, u);
+        if (j < h) {
+            const int ires = ring_of(ky, j);
+            if (ires < h) v = noise_value(key, (unsigned long long)i * h + j, (float)a.noise_sig[ires]);
         }
-        b0[e] = v;
+        W[c * LD + px(i)] = v;
     }
     __syncthreads();
-    const float2* r = fft_smem<false>(b0, b1, R, a.plan, s_tw);
+    fft_columns<N, true>(W, s_tw);
+    __syncthreads();
+    float2* out = a.gn + (size_t)p * N * h;
+    for (int e = threadIdx.x; e < COLS * N; e += PREP_THREADS) {
+        const int c = e % COLS, i = e / COLS;
+        if (j0 + c < h) out[(size_t)i * h + j0 + c] = W[c * LD + px(i)];
+    }
+}
+
+// rows: z = masked + i * unmasked, forward FFT over x, split into the two half spectra (of the unmasked
+// one only the columns of the window); the noise rows first, two as one inverse transform
+template <int N>
+__global__ void __launch_bounds__(PREP_THREADS) k_rows(PrepArgs a)
+{
+    constexpr int h = N / 2 + 1, LD = fft_ld(N), NF = 2, PER = (NF * N + 31) / 32;
+    extern __shared__ float2 sm[];
+    float2* s_tw = sm;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float2* W = sm + N + (size_t)warp * NF * LD;
+    const int p = blockIdx.x, y0 = (blockIdx.y * (PREP_THREADS / 32) + warp) * NF;
+    load_tw(s_tw, a.tw, N);
+    __syncthreads();
+    if (y0 >= N) return;
+    const PixelCtx c = pixel_ctx(a, p);
+    const float* img = a.img + (size_t)p * N * N;
+    float ru[PER], rn[PER];
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int e = lane + 32 * t, rr = e / N, x = e - rr * N, y = y0 + rr;
+        ru[t] = e < NF * N && y < N ? shifted_pixel(a, img, c, x, y) : 0.f;
+    }
+    if (a.zero_mask) {
+        double sw = 0., sv = 0.;
+#pragma unroll
+        for (int b = 0; b < BG_PARTS; ++b) {
+            sw += a.bg[2 * (p * BG_PARTS + b)];
+            sv += a.bg[2 * (p * BG_PARTS + b) + 1];
+        }
+        const float bgv = (float)(sw > 0. ? sv / sw : 0.);
+#pragma unroll
+        for (int t = 0; t < PER; ++t) rn[t] = bgv;
+    } else {
+        // A + i B of the two rows (imaginary parts of kx = 0 and N/2 dropped)
+        const float2* g = a.gn + (size_t)p * N * h;
+        for (int k = lane; k < h; k += 32) {
+            const float2 g0 = g[(size_t)y0 * h + k];
+            const float2 g1 = y0 + 1 < N ? g[(size_t)(y0 + 1) * h + k] : make_float2(0.f, 0.f);
+            if (k == 0 || k == N / 2) {
+                W[px(k)] = make_float2(g0.x, g1.x);
+            } else {
+                W[px(k)] = make_float2(g0.x - g1.y, g0.y + g1.x);
+                W[px(N - k)] = make_float2(g0.x + g1.y, g1.x - g0.y);
+            }
+        }
+        __syncwarp();
+        fft_warp<N, true, 1>(W, s_tw, lane);
+#pragma unroll
+        for (int t = 0; t < PER; ++t) {
+            const int e = lane + 32 * t, rr = e / N, x = e - rr * N;
+            rn[t] = 0.f;
+            if (e < NF * N) rn[t] = rr ? W[px(x)].y : W[px(x)].x;
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int e = lane + 32 * t, rr = e / N, x = e - rr * N, y = y0 + rr;
+        if (e >= NF * N) continue;
+        const float u = ru[t], w = mask_weight(a, x, y);
+        float m = u;
+        if (w >= 0.f) m = (w >= 1.f) ? rn[t] : (1.f - w) * u + w * rn[t];
+        W[rr * LD + px(x)] = y < N ? make_float2(m, u) : make_float2(0.f, 0.f);
+    }
+    __syncwarp();
+    if (warp_seqs(N) == NF) {
+        fft_warp<N, false, NF>(W, s_tw, lane);
+    } else {
+        for (int q = 0; q < NF; ++q) fft_warp<N, false, 1>(W + q * LD, s_tw, lane);
+    }
     float2* om = a.gm + (size_t)p * N * h;
     float2* ou = a.gu + (size_t)p * N * h;
-    for (int e = threadIdx.x; e < R * h; e += blockDim.x) {
+    for (int e = lane; e < NF * h; e += 32) {
         const int rr = e / h, k = e - rr * h, y = y0 + rr;
         if (y >= N) continue;
-        const float2 zk = r[rr * N + k];
-        const float2 zc = r[rr * N + (N - k) % N];   // Z[N-k], conjugated below
         // masked = (Z[k] + conj Z[N-k]) / 2, unmasked = (Z[k] - conj Z[N-k]) / 2i
+        const float2 zk = W[rr * LD + px(k)], zc = W[rr * LD + px(k ? N - k : 0)];
         om[(size_t)y * h + k] = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y - zc.y));
-        ou[(size_t)y * h + k] = make_float2(0.5f * (zk.y + zc.y), -0.5f * (zk.x - zc.x));
+        if (k < a.hs) ou[(size_t)y * h + k] = make_float2(0.5f * (zk.y + zc.y), -0.5f * (zk.x - zc.x));
     }
 }
 
@@ -336,38 +355,42 @@ __device__ __forceinline__ float ctf_value(const PrepArgs& a, const double* par,
     return (float)v;
 }
 
+// columns, forward FFT over y: blocks of the masked columns (power, window, CTF and Minvsigma2), then of
+// the unmasked columns of the window
+template <int N>
 __global__ void __launch_bounds__(PREP_THREADS) k_cols(PrepArgs a)
 {
+    constexpr int h = N / 2 + 1, LD = fft_ld(N), MT = (h + COLS - 1) / COLS;
     extern __shared__ float2 sm[];
-    const int N = a.N, h = a.h, C = a.cpb, s = a.s, hs = a.hs;
     float2* s_tw = sm;
-    float2* b0 = sm + N;
-    float2* b1 = b0 + 2 * C * N;
-    const int p = blockIdx.x, j0 = blockIdx.y * C;
+    float2* W = sm + N;
+    const int s = a.s, hs = a.hs;
+    const int p = blockIdx.x;
+    const bool masked = blockIdx.y < MT;
+    const int j0 = (masked ? blockIdx.y : blockIdx.y - MT) * COLS, jend = masked ? h : hs;
     load_tw(s_tw, a.tw, N);
-    const float2* gm = a.gm + (size_t)p * N * h;
-    const float2* gu = a.gu + (size_t)p * N * h;
-    // sequences 0 .. C-1: masked columns; C .. 2C-1: unmasked
-    for (int e = threadIdx.x; e < 2 * C * N; e += blockDim.x) {
-        const int half = e / (C * N), q = e - half * C * N;
-        const int c = q % C, i = q / C, j = j0 + c;
-        float2 v = make_float2(0.f, 0.f);
-        if (j < h) v = (half ? gu : gm)[(size_t)i * h + j];
-        b0[(half * C + c) * N + i] = v;
+    const float2* g = (masked ? a.gm : a.gu) + (size_t)p * N * h;
+#pragma unroll 8
+    for (int e = threadIdx.x; e < COLS * N; e += PREP_THREADS) {
+        const int c = e % COLS, i = e / COLS, j = j0 + c;
+        W[c * LD + px(i)] = j < jend ? g[(size_t)i * h + j] : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    const float2* r = fft_smem<false>(b0, b1, 2 * C, a.plan, s_tw);
+    fft_columns<N, false>(W, s_tw);
+    __syncthreads();
     const float inv = 1.f / ((float)N * (float)N);
-    // |F|^2 of the masked transform, for the ring sums
-    float* pw = a.pw + (size_t)p * N * h;
-    for (int e = threadIdx.x; e < C * N; e += blockDim.x) {
-        const int c = e % C, i = e / C, j = j0 + c;
-        if (j >= h) continue;
-        const float2 f = r[c * N + i];
-        const float fr = f.x * inv, fi = f.y * inv;
-        pw[(size_t)i * h + j] = fr * fr + fi * fi;
+    if (masked) {
+        // |F|^2 of the masked transform, for the ring sums
+        float* pw = a.pw + (size_t)p * N * h;
+        for (int e = threadIdx.x; e < COLS * N; e += PREP_THREADS) {
+            const int c = e % COLS, i = e / COLS, j = j0 + c;
+            if (j >= h) continue;
+            const float2 f = W[c * LD + px(i)];
+            const float fr = f.x * inv, fi = f.y * inv;
+            pw[(size_t)i * h + j] = fr * fr + fi * fi;
+        }
     }
-    // window to s, CenterFFTbySign, CTF and Minvsigma2 on the window
+    // window to s, CenterFFTbySign; CTF and Minvsigma2 on the window
     if (j0 >= hs) return;
     const double* par = a.par + (size_t)p * NPAR;
     const double az = par[7] * (PI_D / 180.);
@@ -376,30 +399,32 @@ __global__ void __launch_bounds__(PREP_THREADS) k_cols(PrepArgs a)
     const double Axy = (par[6] - par[5]) * ca * sa;
     const double Ayy = -par[5] * sa * sa - par[6] * ca * ca;
     const size_t o = (size_t)p * a.P;
-    for (int e = threadIdx.x; e < C * s; e += blockDim.x) {
-        const int c = e % C, iw = e / C, j = j0 + c;
+    float2* out = reinterpret_cast<float2*>(masked ? a.fimg : a.fnm);
+    for (int e = threadIdx.x; e < COLS * s; e += PREP_THREADS) {
+        const int c = e % COLS, iw = e / COLS, j = j0 + c;
         if (j >= hs) continue;
         const int ky = iw < hs ? iw : iw - s;
         const int i = ky >= 0 ? ky : ky + N;
         const float sg = ((iw ^ j) & 1) ? -inv : inv;
-        const float2 fm = r[c * N + i], fu = r[(C + c) * N + i];
+        const float2 f = W[c * LD + px(i)];
         const size_t w = o + (size_t)iw * hs + j;
-        reinterpret_cast<float2*>(a.fimg)[w] = make_float2(fm.x * sg, fm.y * sg);
-        reinterpret_cast<float2*>(a.fnm)[w] = make_float2(fu.x * sg, fu.y * sg);
-        a.ctf[w] = a.do_ctf ? ctf_value(a, par, Axx, Axy, Ayy, j, ky) : 1.f;
-        a.minv[w] = a.minv_img[(size_t)iw * hs + j];
+        out[w] = make_float2(f.x * sg, f.y * sg);
+        // the CTF on the blocks of the unmasked columns, which have no power spectrum to write
+        if (masked) a.minv[w] = a.minv_img[(size_t)iw * hs + j];
+        else a.ctf[w] = a.do_ctf ? ctf_value(a, par, Axx, Axy, Ayy, j, ky) : 1.f;
     }
 }
 
 // power spectrum of the masked transform: one warp per ring, lanes over the
 // ring's pixels, fixed-order shuffle reduction (deterministic)
+template <int STRIDE>
 __device__ __forceinline__ void ring_sums(const float* pw, const int* off, const int* pix, int h, double* spec,
                                           double* power)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int r = warp; r < h; r += nw) {
         double acc = 0.;
-        for (int q = off[r] + lane; q < off[r + 1]; q += 32) acc += pw[pix[q]];
+        for (int q = off[r] + lane; q < off[r + 1]; q += 32) acc += pw[(size_t)STRIDE * pix[q]];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) {
@@ -415,7 +440,7 @@ __global__ void __launch_bounds__(PREP_THREADS) k_final(PrepArgs a)
     __shared__ double s_spec[PREP_MAX_N / 2 + 1];
     const int p = blockIdx.x, h = a.h;
     const float* pw = a.pw + (size_t)p * a.N * h;
-    ring_sums(pw, a.ring_off, a.ring_pix, h, s_spec, a.power ? a.power + (size_t)p * h : nullptr);
+    ring_sums<1>(pw, a.ring_off, a.ring_pix, h, s_spec, a.power ? a.power + (size_t)p * h : nullptr);
     __syncthreads();
     if (threadIdx.x != 0) return;
     double xi2 = 0.;
@@ -434,103 +459,45 @@ __global__ void __launch_bounds__(PREP_THREADS) k_final(PrepArgs a)
 }
 
 // ------------------------------------------------------------ fused path: one CTA per particle
-// When the particle's two half spectra fit in shared memory (N <= 136), the row
-// and column passes run in one CTA per particle and the half spectra never
-// leave the SM: rows in chunks of FQ (ping-pong scratch), unpacked into the
-// masked and unmasked half spectra; then columns in chunks of FQ/2 of each.
-constexpr int FQ = 16;
-constexpr int FUSED_THREADS = 512;
+// When the particle's two half spectra fit in shared memory (boxes up to 128), everything
+// runs in one CTA per particle and only the results leave the SM: the noise spectrum and its inverse
+// column transforms, then per row the noise (inverse, two rows as one complex sequence), the mask and
+// the forward transform, then the columns, the power spectrum and the window.
+// Bound by issued instructions.  Each warp transforms FW sequences by itself, in place and with
+// the size known at compile time (fft_warp), so a particle takes four block barriers.  In chunks of 16
+// sequences for the whole block, 128 butterflies for 512 threads and some 80 barriers, with the noise image
+// written to memory by a kernel of its own, 1,024 particles of box 128 took 713 us; 452 now.
+constexpr int FW = 4;   // sequences of a warp
+constexpr int fused_threads(int N) { return N > 80 ? 512 : 256; }
 
+// shared memory: twiddles, masked and unmasked half spectra [N][h], the warps' sequences, ring sums
 size_t fused_prep_smem(int N)
 {
     const size_t h = N / 2 + 1;
-    return sizeof(float2) * (N + 2 * h * N + 2 * (size_t)FQ * N) + sizeof(float) * h * N + sizeof(double) * h;
-}
-size_t fused_noise_smem(int N)
-{
-    const size_t h = N / 2 + 1;
-    return sizeof(float2) * (N + h * N + 2 * (size_t)FQ * N);
+    return sizeof(float2) * (N + 2 * h * N + (size_t)(fused_threads(N) / 32) * FW * fft_ld(N)) + sizeof(double) * (h + 1);
 }
 
-// noise image of one particle: spectrum -> inverse over y (columns) -> c2r over x (rows)
-template <int NC>
-__global__ void __launch_bounds__(FUSED_THREADS) k_noise_fused(PrepArgs a)
+template <int N>
+__global__ void __launch_bounds__(fused_threads(N)) k_prep_fused(PrepArgs a)
 {
+    constexpr int NT = fused_threads(N), NW = NT / 32, h = N / 2 + 1, LD = fft_ld(N);
+    constexpr int PER = (FW * N + 31) / 32;   // pixels of a lane's rows
     extern __shared__ float2 sm[];
-    const int N = NC > 0 ? NC : a.N, h = N / 2 + 1, p = blockIdx.x;
-    float2* s_tw = sm;
-    float2* S = s_tw + N;
-    float2* A = S + (size_t)N * h;
-    float2* B = A + FQ * N;
-    load_tw(s_tw, a.tw, N);
-    const unsigned long long key = splitmix64((unsigned long long)(a.seed + a.pid[p]));
-    for (int e = threadIdx.x; e < N * h; e += blockDim.x) {
-        const int i = e / h, j = e - i * h;
-        const int ky = i < h ? i : i - N;
-        const int ires = ring_of(ky, j);
-        float2 v = make_float2(0.f, 0.f);
-        if (ires < h) v = noise_value(key, (unsigned long long)e, (float)a.noise_sig[ires]);
-        S[e] = v;
-    }
-    __syncthreads();
-    for (int j0 = 0; j0 < h; j0 += FQ) {
-        for (int e = threadIdx.x; e < FQ * N; e += blockDim.x) {
-            const int i = e % N, c = e / N, j = j0 + c;
-            A[e] = j < h ? S[(size_t)i * h + j] : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-        const float2* r = fft_any<NC, true>(A, B, FQ, a.plan, s_tw);
-        for (int e = threadIdx.x; e < FQ * N; e += blockDim.x) {
-            const int i = e % N, c = e / N, j = j0 + c;
-            if (j < h) S[(size_t)i * h + j] = r[e];
-        }
-        __syncthreads();
-    }
-    float* out = a.noise + (size_t)p * N * N;
-    for (int y0 = 0; y0 < N; y0 += FQ) {
-        for (int e = threadIdx.x; e < FQ * N; e += blockDim.x) {
-            const int rr = e / N, k = e - rr * N, y = y0 + rr;
-            float2 v = make_float2(0.f, 0.f);
-            if (y < N) {
-                const float2* g = S + (size_t)y * h;
-                if (k == 0 || k == N / 2) v = make_float2(g[k].x, 0.f);
-                else if (k < N / 2) v = g[k];
-                else v = make_float2(g[N - k].x, -g[N - k].y);
-            }
-            A[e] = v;
-        }
-        __syncthreads();
-        const float2* r = fft_any<NC, true>(A, B, FQ, a.plan, s_tw);
-        for (int e = threadIdx.x; e < FQ * N; e += blockDim.x) {
-            const int rr = e / N, x = e - rr * N, y = y0 + rr;
-            if (y < N) out[(size_t)y * N + x] = r[e].x;
-        }
-        __syncthreads();
-    }
-}
-
-template <int NC>
-__global__ void __launch_bounds__(FUSED_THREADS) k_prep_fused(PrepArgs a)
-{
-    extern __shared__ float2 sm[];
-    __shared__ double s_w[FUSED_THREADS], s_v[FUSED_THREADS];
-    const int N = NC > 0 ? NC : a.N, h = N / 2 + 1, p = blockIdx.x;
-    constexpr int C = FQ / 2;
+    const int p = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int s = a.s, hs = a.hs;
     float2* s_tw = sm;
     float2* SM = s_tw + N;
-    float2* SU = SM + (size_t)N * h;
-    float2* A = SU + (size_t)N * h;
-    float2* B = A + FQ * N;
-    float* PW = reinterpret_cast<float*>(B + FQ * N);
+    float2* SU = SM + (size_t)N * h;   // the noise spectrum until a row's unmasked half replaces it
+    float2* W = SU + (size_t)N * h + (size_t)warp * FW * LD;
     load_tw(s_tw, a.tw, N);
     const PixelCtx pc = pixel_ctx(a, p);
     const float* img = a.img + (size_t)p * N * N;
-    const float* noise = a.zero_mask ? nullptr : a.noise + (size_t)p * N * N;
-    // average background (zero-mask path): fixed-order FP64 reduction
     float bgv = 0.f;
     if (a.zero_mask) {
+        // average background: fixed-order FP64 reduction
+        __shared__ double s_w[NT], s_v[NT];
         double sw = 0., sv = 0.;
-        for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
+        for (int e = threadIdx.x; e < N * N; e += NT) {
             const int y = e / N, x = e - y * N;
             const float w = mask_weight(a, x, y);
             if (w < 0.f) continue;
@@ -540,7 +507,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_prep_fused(PrepArgs a)
         s_w[threadIdx.x] = sw;
         s_v[threadIdx.x] = sv;
         __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+        for (int o = NT / 2; o > 0; o >>= 1) {
             if (threadIdx.x < o) {
                 s_w[threadIdx.x] += s_w[threadIdx.x + o];
                 s_v[threadIdx.x] += s_v[threadIdx.x + o];
@@ -548,102 +515,135 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_prep_fused(PrepArgs a)
             __syncthreads();
         }
         bgv = s_w[0] > 0. ? (float)(s_v[0] / s_w[0]) : 0.f;
-    }
-    // rows: masked + i * unmasked, forward FFT over x, split into the two half spectra.
-    // The pixels (and the noise outside the mask) of the next FQ rows are loaded into
-    // registers before the current rows' FFT, so their latency overlaps it.
-    constexpr int PMAX = (FQ * (NC > 0 ? NC : 136) + FUSED_THREADS - 1) / FUSED_THREADS;
-    float ru[PMAX], rn[PMAX];
-    auto fetch = [&](int y0) {
-#pragma unroll
-        for (int t = 0; t < PMAX; ++t) {
-            const int e = threadIdx.x + t * FUSED_THREADS;
-            const int rr = e / N, x = e - rr * N, y = y0 + rr;
-            ru[t] = 0.f;
-            rn[t] = 0.f;
-            if (e < FQ * N && y < N) {
-                ru[t] = shifted_pixel(a, img, pc, x, y);
-                if (!a.zero_mask && mask_weight(a, x, y) >= 0.f) rn[t] = noise[(size_t)y * N + x];
-            }
-        }
-    };
-    fetch(0);
-    for (int y0 = 0; y0 < N; y0 += FQ) {
-#pragma unroll
-        for (int t = 0; t < PMAX; ++t) {
-            const int e = threadIdx.x + t * FUSED_THREADS;
-            if (e >= FQ * N) continue;
-            const int rr = e / N, x = e - rr * N, y = y0 + rr;
-            const float u = ru[t];
-            const float w = mask_weight(a, x, y);
-            float m = u;
-            if (w >= 0.f) {
-                const float fill = a.zero_mask ? bgv : rn[t];
-                m = (w >= 1.f) ? fill : (1.f - w) * u + w * fill;
-            }
-            A[e] = y < N ? make_float2(m, u) : make_float2(0.f, 0.f);
-        }
+    } else {
+        // noise spectrum, and its columns back to rows of half spectra over kx
+        const unsigned long long key = splitmix64((unsigned long long)(a.seed + a.pid[p]));
         __syncthreads();
-        if (y0 + FQ < N) fetch(y0 + FQ);
-        const float2* r = fft_any<NC, false>(A, B, FQ, a.plan, s_tw);
-        for (int e = threadIdx.x; e < FQ * h; e += blockDim.x) {
+        for (int j0 = warp * FW; j0 < h; j0 += NW * FW) {
+            for (int e = lane; e < FW * N; e += 32) {
+                const int c = e % FW, i = e / FW, j = j0 + c;
+                const int ky = i < h ? i : i - N;
+                float2 v = make_float2(0.f, 0.f);
+                if (j < h) {
+                    const int ires = ring_of(ky, j);
+                    if (ires < h) v = noise_value(key, (unsigned long long)i * h + j, (float)a.noise_sig[ires]);
+                }
+                W[c * LD + px(i)] = v;
+            }
+            __syncwarp();
+            fft_warp<N, true, FW>(W, s_tw, lane);
+            for (int e = lane; e < FW * N; e += 32) {
+                const int c = e % FW, i = e / FW;
+                if (j0 + c < h) SU[(size_t)i * h + j0 + c] = W[c * LD + px(i)];
+            }
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // rows: masked + i * unmasked, forward FFT over x, split into the two half spectra
+    for (int y0 = warp * FW; y0 < N; y0 += NW * FW) {
+        float ru[PER], rn[PER];
+#pragma unroll
+        for (int t = 0; t < PER; ++t) {
+            const int e = lane + 32 * t, rr = e / N, x = e - rr * N, y = y0 + rr;
+            ru[t] = e < FW * N && y < N ? shifted_pixel(a, img, pc, x, y) : 0.f;
+            rn[t] = bgv;
+        }
+        if (!a.zero_mask) {
+            // rows y, y + 1 of the noise from one inverse transform of A + i B (imaginary parts of
+            // kx = 0 and N/2 dropped, as a complex-to-real transform does)
+            for (int e = lane; e < FW / 2 * h; e += 32) {
+                const int c = e / h, k = e - c * h, y = y0 + 2 * c;
+                const float2 g0 = y < N ? SU[(size_t)y * h + k] : make_float2(0.f, 0.f);
+                const float2 g1 = y + 1 < N ? SU[(size_t)(y + 1) * h + k] : make_float2(0.f, 0.f);
+                if (k == 0 || k == N / 2) {
+                    W[c * LD + px(k)] = make_float2(g0.x, g1.x);
+                } else {
+                    W[c * LD + px(k)] = make_float2(g0.x - g1.y, g0.y + g1.x);
+                    W[c * LD + px(N - k)] = make_float2(g0.x + g1.y, g1.x - g0.y);
+                }
+            }
+            __syncwarp();
+            fft_warp<N, true, FW / 2>(W, s_tw, lane);
+#pragma unroll
+            for (int t = 0; t < PER; ++t) {
+                const int e = lane + 32 * t, rr = e / N, x = e - rr * N;
+                if (e < FW * N) {
+                    const float2 v = W[(rr >> 1) * LD + px(x)];
+                    rn[t] = rr & 1 ? v.y : v.x;
+                }
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int t = 0; t < PER; ++t) {
+            const int e = lane + 32 * t, rr = e / N, x = e - rr * N, y = y0 + rr;
+            if (e >= FW * N) continue;
+            const float u = ru[t], w = mask_weight(a, x, y);
+            float m = u;
+            if (w >= 0.f) m = (w >= 1.f) ? rn[t] : (1.f - w) * u + w * rn[t];
+            W[rr * LD + px(x)] = y < N ? make_float2(m, u) : make_float2(0.f, 0.f);
+        }
+        __syncwarp();
+        fft_warp<N, false, FW>(W, s_tw, lane);
+        for (int e = lane; e < FW * h; e += 32) {
             const int rr = e / h, k = e - rr * h, y = y0 + rr;
             if (y >= N) continue;
-            const float2 zk = r[rr * N + k];
-            const float2 zc = r[rr * N + (N - k) % N];
+            const float2 zk = W[rr * LD + px(k)];
+            const float2 zc = W[rr * LD + px(k ? N - k : 0)];
             SM[(size_t)y * h + k] = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y - zc.y));
             SU[(size_t)y * h + k] = make_float2(0.5f * (zk.y + zc.y), -0.5f * (zk.x - zc.x));
         }
-        __syncthreads();
+        __syncwarp();
     }
-    // columns: C of each half spectrum per chunk, forward FFT over y
-    const double* par = a.par + (size_t)p * NPAR;
-    const double az = par[7] * (PI_D / 180.);
-    const double ca = cos(az), sa = sin(az);
-    const double Axx = -par[5] * ca * ca - par[6] * sa * sa;
-    const double Axy = (par[6] - par[5]) * ca * sa;
-    const double Ayy = -par[5] * sa * sa - par[6] * ca * ca;
-    const float inv = 1.f / ((float)N * (float)N);
-    const int s = a.s, hs = a.hs;
-    const size_t o = (size_t)p * a.P;
-    for (int j0 = 0; j0 < h; j0 += C) {
-        for (int e = threadIdx.x; e < 2 * C * N; e += blockDim.x) {
-            const int i = e % N, q = e / N, half = q / C, j = j0 + (q - half * C);
-            A[e] = j < h ? (half ? SU : SM)[(size_t)i * h + j] : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-        const float2* r = fft_any<NC, false>(A, B, 2 * C, a.plan, s_tw);
-        for (int e = threadIdx.x; e < C * N; e += blockDim.x) {
-            const int i = e % N, c = e / N, j = j0 + c;
-            if (j >= h) continue;
-            const float2 f = r[e];
-            const float fr = f.x * inv, fi = f.y * inv;
-            PW[(size_t)i * h + j] = fr * fr + fi * fi;
-        }
-        if (j0 < hs)
-            for (int e = threadIdx.x; e < C * s; e += blockDim.x) {
-                const int c = e % C, iw = e / C, j = j0 + c;
-                if (j >= hs) continue;
-                const int ky = iw < hs ? iw : iw - s;
-                const int i = ky >= 0 ? ky : ky + N;
-                const float sg = ((iw ^ j) & 1) ? -inv : inv;
-                const float2 fm = r[c * N + i], fu = r[(C + c) * N + i];
-                const size_t w = o + (size_t)iw * hs + j;
-                reinterpret_cast<float2*>(a.fimg)[w] = make_float2(fm.x * sg, fm.y * sg);
-                reinterpret_cast<float2*>(a.fnm)[w] = make_float2(fu.x * sg, fu.y * sg);
-                a.ctf[w] = a.do_ctf ? ctf_value(a, par, Axx, Axy, Ayy, j, ky) : 1.f;
-                a.minv[w] = a.minv_img[(size_t)iw * hs + j];
-            }
-        __syncthreads();
-    }
-    // ring sums (fixed order per ring) and the scalars; the ring lists are staged in
-    // the free row scratch (they fit for every N of this kernel)
-    int* s_pix = reinterpret_cast<int*>(A);
-    double* spec = reinterpret_cast<double*>(PW + (size_t)N * h);
-    const int npix = a.ring_off[h];
-    for (int q = threadIdx.x; q < npix; q += blockDim.x) s_pix[q] = a.ring_pix[q];
     __syncthreads();
-    ring_sums(PW, a.ring_off, s_pix, h, spec, a.power ? a.power + (size_t)p * h : nullptr);
+    // columns, forward FFT over y: the masked ones (0 .. h - 1), then the unmasked ones that the window
+    // takes (0 .. hs - 1).  |F|^2 of a masked column replaces it in SM (x component).
+    const float inv = 1.f / ((float)N * (float)N);
+    const size_t o = (size_t)p * a.P;
+    for (int q0 = warp * FW; q0 < h + hs; q0 += NW * FW) {
+        for (int e = lane; e < FW * N; e += 32) {
+            const int c = e % FW, i = e / FW, q = q0 + c;
+            W[c * LD + px(i)] = q < h ? SM[(size_t)i * h + q] : q < h + hs ? SU[(size_t)i * h + q - h] : make_float2(0.f, 0.f);
+        }
+        __syncwarp();
+        fft_warp<N, false, FW>(W, s_tw, lane);
+        for (int e = lane; e < FW * N; e += 32) {
+            const int c = e % FW, i = e / FW, q = q0 + c;
+            if (q >= h) continue;
+            const float2 f = W[c * LD + px(i)];
+            const float fr = f.x * inv, fi = f.y * inv;
+            SM[(size_t)i * h + q].x = fr * fr + fi * fi;
+        }
+        for (int e = lane; e < FW * s; e += 32) {
+            const int c = e % FW, iw = e / FW, q = q0 + c;
+            const int j = q < h ? q : q - h;
+            if (j >= hs || q >= h + hs) continue;
+            const int i = iw < hs ? iw : iw - s + N;
+            const float sg = ((iw ^ j) & 1) ? -inv : inv;
+            const float2 f = W[c * LD + px(i)];
+            reinterpret_cast<float2*>(q < h ? a.fimg : a.fnm)[o + (size_t)iw * hs + j] = make_float2(f.x * sg, f.y * sg);
+        }
+        __syncwarp();
+    }
+    // CTF and Minvsigma2 on the window
+    const double* par = a.par + (size_t)p * NPAR;
+    {
+        const double az = par[7] * (PI_D / 180.);
+        const double ca = cos(az), sa = sin(az);
+        const double Axx = -par[5] * ca * ca - par[6] * sa * sa;
+        const double Axy = (par[6] - par[5]) * ca * sa;
+        const double Ayy = -par[5] * sa * sa - par[6] * ca * ca;
+        for (int e = threadIdx.x; e < s * hs; e += NT) {
+            const int iw = e / hs, j = e - iw * hs;
+            a.ctf[o + e] = a.do_ctf ? ctf_value(a, par, Axx, Axy, Ayy, j, iw < hs ? iw : iw - s) : 1.f;
+            a.minv[o + e] = a.minv_img[e];
+        }
+    }
+    __syncthreads();
+    // ring sums (fixed order per ring) and the scalars
+    double* spec = reinterpret_cast<double*>(SU);
+    ring_sums<2>(&SM[0].x, a.ring_off, a.ring_pix, h, spec, a.power ? a.power + (size_t)p * h : nullptr);
     __syncthreads();
     if (threadIdx.x == 0) {
         double xi2 = 0.;
@@ -663,17 +663,33 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_prep_fused(PrepArgs a)
 
 // ------------------------------------------------------------ host side
 
-// compile-time sizes of the fused kernels (other sizes run the same kernels with the runtime plan)
-#define T2B_PREP_SIZES(X) X(64) X(72) X(80) X(96) X(100) X(120) X(128)
+// every even product of 2, 3 and 5 from 8 to 512: up to 128 the fused kernel, above the two-pass ones
+#define T2B_FUSED_SIZES(X)                                                                                     \
+    X(8) X(10) X(12) X(16) X(18) X(20) X(24) X(30) X(32) X(36) X(40) X(48) X(50) X(54) X(60) X(64) X(72) X(80) \
+        X(90) X(96) X(100) X(108) X(120) X(128)
+#define T2B_TWO_PASS_SIZES(X)                                                                                   \
+    X(144) X(150) X(160) X(162) X(180) X(192) X(200) X(216) X(240) X(250) X(256) X(270) X(288) X(300) X(320)    \
+        X(324) X(360) X(384) X(400) X(432) X(450) X(480) X(486) X(500) X(512)
 
 using PrepKernel = void (*)(PrepArgs);
-PrepKernel fused_kernel(int N, bool noise)
+PrepKernel fused_kernel(int N)   // null: the two-pass kernels
 {
 #define T2B_CASE(n) \
-    if (N == n) return noise ? (PrepKernel)k_noise_fused<n> : (PrepKernel)k_prep_fused<n>;
-    T2B_PREP_SIZES(T2B_CASE)
+    if (N == n) return (PrepKernel)k_prep_fused<n>;
+    T2B_FUSED_SIZES(T2B_CASE)
 #undef T2B_CASE
-    return noise ? (PrepKernel)k_noise_fused<0> : (PrepKernel)k_prep_fused<0>;
+    return nullptr;
+}
+struct TwoPass {
+    PrepKernel noise_cols = nullptr, rows = nullptr, cols = nullptr;
+};
+TwoPass two_pass_kernels(int N)
+{
+#define T2B_CASE(n) \
+    if (N == n) return {(PrepKernel)k_noise_cols<n>, (PrepKernel)k_rows<n>, (PrepKernel)k_cols<n>};
+    T2B_TWO_PASS_SIZES(T2B_CASE)
+#undef T2B_CASE
+    return {};
 }
 
 double host_round(double x) { return x > 0 ? (double)(int)(x + 0.5) : (double)(int)(x - 0.5); }
@@ -695,23 +711,19 @@ void free_prep(ImagePrep* G)
     delete G;
 }
 
-size_t smem_rows(const ImagePrep& G) { return sizeof(float2) * ((size_t)G.N + 2 * (size_t)G.rpb * G.N); }
-size_t smem_noise_cols(const ImagePrep& G) { return sizeof(float2) * ((size_t)G.N + 2 * (size_t)G.cpb * G.N); }
-size_t smem_cols(const ImagePrep& G) { return sizeof(float2) * ((size_t)G.N + 4 * (size_t)G.cpb * G.N); }
+size_t smem_rows(int N) { return sizeof(float2) * ((size_t)N + PREP_THREADS / 32 * 2 * (size_t)fft_ld(N)); }
+size_t smem_cols(int N) { return sizeof(float2) * ((size_t)N + COLS * (size_t)fft_ld(N)); }
 
 PrepArgs make_args(const ImagePrep& G, int n, const float* img, const double* par, const long long* pid,
                    const t2b_prep_out& o)
 {
     const t2b_prep_config& cf = G.cfg;
     PrepArgs a{};
-    a.plan = G.plan;
     a.N = G.N;
     a.h = G.h;
     a.s = G.s;
     a.hs = G.hs;
     a.P = G.P;
-    a.rpb = G.rpb;
-    a.cpb = G.cpb;
     a.zero_mask = cf.zero_mask;
     a.do_ctf = cf.do_ctf_correction;
     a.premult = cf.ctf_premultiplied;
@@ -742,7 +754,6 @@ PrepArgs make_args(const ImagePrep& G, int n, const float* img, const double* pa
     a.gm = G.gm;
     a.gu = G.gu;
     a.gn = G.gn;
-    a.noise = G.noise;
     a.pw = G.pw;
     a.bg = G.bg;
     a.fimg = o.fimg;
@@ -757,31 +768,20 @@ PrepArgs make_args(const ImagePrep& G, int n, const float* img, const double* pa
 
 int enqueue_prep(const ImagePrep& G, const PrepArgs& a, int n, cudaStream_t st)
 {
-    int launches = 0;
     if (G.fused) {
-        if (!G.cfg.zero_mask) {
-            fused_kernel(G.N, true)<<<n, FUSED_THREADS, fused_noise_smem(G.N), st>>>(a);
-            ++launches;
-        }
-        fused_kernel(G.N, false)<<<n, FUSED_THREADS, fused_prep_smem(G.N), st>>>(a);
+        fused_kernel(G.N)<<<n, fused_threads(G.N), fused_prep_smem(G.N), st>>>(a);
         T2B_CUDA(cudaGetLastError());
-        return launches + 1;
+        return 1;
     }
-    const dim3 grow(n, (G.N + G.rpb - 1) / G.rpb), gcol(n, G.ncol_blocks);
-    if (!G.cfg.zero_mask) {
-        k_noise_cols<<<gcol, PREP_THREADS, smem_noise_cols(G), st>>>(a);
-        k_noise_rows<<<grow, PREP_THREADS, smem_rows(G), st>>>(a);
-        launches += 2;
-    } else {
-        k_background<<<n, PREP_THREADS, 0, st>>>(a);
-        launches += 1;
-    }
-    k_rows<<<grow, PREP_THREADS, smem_rows(G), st>>>(a);
-    k_cols<<<gcol, PREP_THREADS, smem_cols(G), st>>>(a);
+    const TwoPass k = two_pass_kernels(G.N);
+    const int rows = PREP_THREADS / 32 * 2, mt = (G.h + COLS - 1) / COLS, ut = (G.hs + COLS - 1) / COLS;
+    if (!G.cfg.zero_mask) k.noise_cols<<<dim3(n, mt), PREP_THREADS, smem_cols(G.N), st>>>(a);
+    else k_background<<<dim3(n, BG_PARTS), PREP_THREADS, 0, st>>>(a);
+    k.rows<<<dim3(n, (G.N + rows - 1) / rows), PREP_THREADS, smem_rows(G.N), st>>>(a);
+    k.cols<<<dim3(n, mt + ut), PREP_THREADS, smem_cols(G.N), st>>>(a);
     k_final<<<n, PREP_THREADS, 0, st>>>(a);
-    launches += 3;
     T2B_CUDA(cudaGetLastError());
-    return launches;
+    return 4;
 }
 
 void check_out(const t2b_prep_out* o)
@@ -810,6 +810,7 @@ int t2b_prep_configure(t2b_ctx* c, const t2b_prep_config* cf)
         T2B_REQUIRE(c && cf, T2B_ERR_ARG, "null argument");
         std::lock_guard<std::mutex> lk(c->mu);
         DeviceGuard dg(c->device);
+        c->release_scratch();
         const int N = cf->image_size, s = cf->current_size;
         T2B_REQUIRE(N >= 8 && N <= PREP_MAX_N && N % 2 == 0, T2B_ERR_UNSUPPORTED, "image_size must be even, 8..512");
         T2B_REQUIRE(s >= 2 && s <= N && s % 2 == 0, T2B_ERR_ARG, "current_size must be even and <= image_size");
@@ -820,7 +821,7 @@ int t2b_prep_configure(t2b_ctx* c, const t2b_prep_config* cf)
         T2B_REQUIRE(cf->q0 >= 0. && cf->q0 < 1. && cf->voltage > 0., T2B_ERR_ARG, "bad optics (voltage, q0)");
         T2B_REQUIRE(!cf->do_norm_correction || cf->avg_norm_correction > 0., T2B_ERR_ARG,
                     "avg_norm_correction must be positive");
-        const FftPlan plan = fft_plan(N);
+        (void)fft_plan(N);   // refuses sizes with other prime factors
         free_prep(c->prep);
         c->prep = nullptr;
         ImagePrep* G = new ImagePrep();
@@ -833,10 +834,6 @@ int t2b_prep_configure(t2b_ctx* c, const t2b_prep_config* cf)
             G->hs = s / 2 + 1;
             G->P = s * G->hs;
             G->max_batch = cf->max_batch;
-            G->plan = plan;
-            G->rpb = std::max(1, std::min(16, 16384 / N));
-            G->cpb = std::max(1, std::min(16, (96 * 1024) / (32 * N)));
-            G->ncol_blocks = (G->h + G->cpb - 1) / G->cpb;
             const int h = G->h, hs = G->hs;
             // twiddles in FP64 on the host
             std::vector<float2> tw(N);
@@ -877,25 +874,22 @@ int t2b_prep_configure(t2b_ctx* c, const t2b_prep_config* cf)
             }
             off[h] = (int)pix.size();
             const size_t B = cf->max_batch, NH = (size_t)N * h;
-            int optin = 0;
-            T2B_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-            // static shared memory of k_prep_fused: the two FP64 reduction arrays
-            // (the fused kernel stages the ring lists in its row scratch: 2 FQ N float2)
-            G->fused = fused_prep_smem(N) + 2 * FUSED_THREADS * sizeof(double) <= (size_t)optin &&
-                       pix.size() <= (size_t)4 * FQ * N;
+            const PrepKernel fused = fused_kernel(N);
+            const TwoPass two = two_pass_kernels(N);
+            T2B_REQUIRE(fused || two.rows, T2B_ERR_STATE, "no transform for this image_size");
+            G->fused = fused != nullptr;
             G->tw = dalloc<float2>(*G, N);
             G->noise_sig = dalloc<double>(*G, h);
             G->minv = dalloc<float>(*G, G->P);
             G->ring_off = dalloc<int>(*G, h + 1);
             G->ring_pix = dalloc<int>(*G, pix.size());
-            G->bg = dalloc<double>(*G, B);
+            G->bg = dalloc<double>(*G, B * 2 * BG_PARTS);
             if (!G->fused) {
                 G->gm = dalloc<float2>(*G, B * NH);
                 G->gu = dalloc<float2>(*G, B * NH);
                 G->pw = dalloc<float>(*G, B * NH);
                 if (!cf->zero_mask) G->gn = dalloc<float2>(*G, B * NH);
             }
-            if (!cf->zero_mask) G->noise = dalloc<float>(*G, B * (size_t)N * N);
             T2B_CUDA(cudaMemcpy(G->tw, tw.data(), N * sizeof(float2), cudaMemcpyHostToDevice));
             T2B_CUDA(cudaMemcpy(G->noise_sig, nsig.data(), h * sizeof(double), cudaMemcpyHostToDevice));
             T2B_CUDA(cudaMemcpy(G->minv, minv.data(), G->P * sizeof(float), cudaMemcpyHostToDevice));
@@ -903,15 +897,13 @@ int t2b_prep_configure(t2b_ctx* c, const t2b_prep_config* cf)
             if (!pix.empty())
                 T2B_CUDA(cudaMemcpy(G->ring_pix, pix.data(), pix.size() * sizeof(int), cudaMemcpyHostToDevice));
             if (G->fused) {
-                T2B_CUDA(cudaFuncSetAttribute((const void*)fused_kernel(N, false),
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_prep_smem(N)));
-                T2B_CUDA(cudaFuncSetAttribute((const void*)fused_kernel(N, true),
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_noise_smem(N)));
+                T2B_CUDA(cudaFuncSetAttribute((const void*)fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)fused_prep_smem(N)));
             } else {
-                const int big = (int)std::max(smem_rows(*G), std::max(smem_cols(*G), smem_noise_cols(*G)));
-                for (const void* k : {(const void*)k_rows, (const void*)k_cols, (const void*)k_noise_cols,
-                                      (const void*)k_noise_rows})
-                    T2B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+                T2B_CUDA(cudaFuncSetAttribute((const void*)two.rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)smem_rows(N)));
+                for (const void* k : {(const void*)two.cols, (const void*)two.noise_cols})
+                    T2B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols(N)));
             }
         } catch (...) {
             free_prep(G);

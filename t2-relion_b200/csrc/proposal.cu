@@ -1853,6 +1853,7 @@ int t2b_proposal_train(t2b_ctx* c, const t2b_proposal_train_config* cfg, t2b_pro
         std::lock_guard<std::mutex> lk(c->mu);
         DeviceGuard dg(c->device);
         c->quiesce();   // training reallocates buffers that host batches in flight still use
+        c->release_scratch();
         cudaStream_t st = c->stream;
         drop_graph(c);
         const Tables& tb = c->tb;
@@ -2066,6 +2067,7 @@ int t2b_proposal_enable(t2b_ctx* c, int topk, int rescore, int audit_every, doub
                     "rescore must be 0 or a multiple of 128 in [topk, min(1024, nr_classes*n_dir*n_psi)]");
         ProposalNet& N = *c->net;
         const int B = c->cfg.max_batch;
+        c->release_scratch();
         // at most ceil(B / every) multiples of `every` in any B consecutive stream positions
         net_setup(c, std::min(B, (B + audit_every - 1) / audit_every));
         T2B_REQUIRE(rescore == 0 || c->tb.T <= RS_TMAX,

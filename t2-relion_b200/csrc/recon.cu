@@ -6,7 +6,7 @@
 // !--dont_skip_gridding, src/ml_optimiser.cpp:525): decenter (r^2 <= ROUND(r_max
 // pad)^2), the MAP term 1 / (pad^3 tau2_fudge tau2) added to the weights
 // (:1412-1455), the FP64 division by max(weight, radial average / 1000)
-// (:1463-1531; the kernels of t2b_reconstruct_divide), then
+// (:1463-1531), then
 // windowToOridimRealSpace (:2486-2620) and Projector::griddingCorrect
 // (src/projector.cpp:489-522):
 //   window the pad_size transform to pad * ori_size (src/fftw.h:736-790),
@@ -21,10 +21,11 @@
 //
 // t2b_fsc_halves: getDownsampledAverage + calculateDownSampledFourierShellCorrelation
 // (src/backprojector.cpp:933-1040).  t2b_update_ssnr: updateSSNRarrays
-// (:1041-1205).  Both reduce the grid on the device (FP64 atomics into shell
-// and down-sampled bins) and finish the per-shell arithmetic on the host.
+// (:1041-1205).  Both reduce the grid to FP64 shell sums on the device and finish the per-shell
+// arithmetic on the host.
 #include "t2b_internal.cuh"
 #include "fft_smem.cuh"
+#include "shells.cuh"
 
 #include <array>
 #include <cctype>
@@ -32,6 +33,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace t2b {
@@ -44,27 +46,55 @@ constexpr int RC_THREADS = 256;
 constexpr int RC_CX = 16;   // columns per CTA in the z and y passes
 constexpr int RC_ROWS = 8;  // rows per CTA in the x pass
 
-__device__ __forceinline__ int rround(double x) { return x > 0 ? (int)(x + 0.5) : (int)(x - 0.5); }
+// How a voxel of the centred grid becomes an element of the transform: divided by
+// max(weight, radial average / 1000) (skip-gridding), or data inv_norm times the gridding weight
+// w_n (fn, FFTW layout of the pad_size box)
+struct Divide {
+    const double* rad;        // r_max radial averages / 1000
+    const double* inv_tau2;   // per shell, null without the MAP term
+    int minres_map;
+    const double* fn;         // gridding weights, null for the division
+    double inv_norm;
+};
 
-// the pad_size transform (FFTW layout, double2) -> the N = pad * ori_size half
-// transform (float2), windowed (shrink: every output element; enlarge: input
-// elements with r^2 <= (ps/2)^2) and centred by sign
-__global__ void k_window(const double2* __restrict__ fc, int ps, int N, int dim, float2* __restrict__ G)
+// the centred grid -> the N = pad * ori_size half transform (float2): decentred (r^2 <= (r_max pad)^2),
+// divided in FP64, windowed (shrink: every output element; enlarge: input elements with
+// r^2 <= (ps/2)^2) and centred by sign.  Bound by reading the grid and writing G once (105 + 68 MB
+// at 259 -> 256: 27 us at the copy bandwidth); an FP64 copy of the transform and of the weights
+// in between cost 210 MB of buffers and two more passes.
+__global__ void k_window(Volume g, const float2* __restrict__ data, const float* __restrict__ weight, Divide dv, int N,
+                         float2* __restrict__ G)
 {
-    const int h = N / 2 + 1, half = ps / 2, fx = ps / 2 + 1;
-    const long long total = (long long)(dim == 3 ? N : 1) * N * h;   // 2D: one plane
+    const int ps = g.ydim, h = N / 2 + 1, half = ps / 2, fx = ps / 2 + 1, rp = g.r_max * g.pad;
+    const long long total = (long long)(g.ref_dim == 3 ? N : 1) * N * h;   // 2D: one plane
     for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
         const int j = (int)(n % h);
         const int i = (int)((n / h) % N);
         const int k = (int)(n / ((long long)h * N));
         const int kp = k < h ? k : k - N, ip = i < h ? i : i - N;
+        const int r2 = kp * kp + ip * ip + j * j;
         float2 v = make_float2(0.f, 0.f);
-        bool ok = kp >= -half && kp <= half && ip >= -half && ip <= half && j <= half;
-        if (ok && N > ps) ok = kp * kp + ip * ip + j * j <= half * half;
+        bool ok = kp >= -half && kp <= half && ip >= -half && ip <= half && j <= half && r2 <= rp * rp;
+        if (ok && N > ps) ok = r2 <= half * half;
         if (ok) {
-            const double2 d = fc[((size_t)(kp < 0 ? kp + ps : kp) * ps + (ip < 0 ? ip + ps : ip)) * fx + j];
+            const size_t src = ((size_t)(kp - g.initz) * g.ydim + (ip - g.inity)) * g.xdim + j;
+            const float2 d = data[src];
+            double re = d.x, im = d.y;
+            if (dv.fn) {
+                const double f = dv.fn[((size_t)(kp < 0 ? kp + ps : kp) * ps + (ip < 0 ? ip + ps : ip)) * fx + j];
+                re = re * dv.inv_norm * f;
+                im = im * dv.inv_norm * f;
+            } else {
+                double w = weight[src];
+                if (dv.inv_tau2 && r2 < rp * rp) w = map_weight(w, r2, g.pad, dv.inv_tau2, dv.minres_map);
+                w = fmax(w, dv.rad[min(shell_floor(r2, g.pad), g.r_max - 1)]);
+                if (w != 0.) {
+                    re /= w;
+                    im /= w;
+                }
+            }
             const float sg = ((k ^ i ^ j) & 1) ? -1.f : 1.f;
-            v = make_float2((float)d.x * sg, (float)d.y * sg);
+            v = make_float2((float)re * sg, (float)im * sg);
         }
         G[n] = v;
     }
@@ -78,9 +108,10 @@ __global__ void __launch_bounds__(RC_THREADS) k_cols3(float2* __restrict__ G, in
 {
     extern __shared__ float2 sm[];
     const int N = NC > 0 ? NC : Nrt, h = N / 2 + 1;
+    const int LD = fft_ld(N);
     float2* s_tw = sm;
     float2* A = sm + N;
-    float2* B = A + RC_CX * N;
+    float2* B = A + RC_CX * LD;
     for (int t = threadIdx.x; t < N; t += blockDim.x) s_tw[t] = tw[t];
     const int x0 = blockIdx.y * RC_CX;
     const size_t line = blockIdx.x;
@@ -90,13 +121,13 @@ __global__ void __launch_bounds__(RC_THREADS) k_cols3(float2* __restrict__ G, in
     };
     for (int e = threadIdx.x; e < RC_CX * N; e += blockDim.x) {
         const int c = e % RC_CX, q = e / RC_CX;
-        A[c * N + q] = x0 + c < h ? G[idx(q, c)] : make_float2(0.f, 0.f);
+        A[c * LD + px(q)] = x0 + c < h ? G[idx(q, c)] : make_float2(0.f, 0.f);
     }
     __syncthreads();
     const float2* r = fft_any<NC, true>(A, B, RC_CX, plan, s_tw);
     for (int e = threadIdx.x; e < RC_CX * N; e += blockDim.x) {
         const int c = e % RC_CX, q = e / RC_CX;
-        if (x0 + c < h) G[idx(q, c)] = r[c * N + q];
+        if (x0 + c < h) G[idx(q, c)] = r[c * LD + px(q)];
     }
 }
 
@@ -110,9 +141,10 @@ __global__ void __launch_bounds__(RC_THREADS) k_rows3(const float2* __restrict__
 {
     extern __shared__ float2 sm[];
     const int N = NC > 0 ? NC : Nrt, h = N / 2 + 1;
+    const int LD = fft_ld(N);
     float2* s_tw = sm;
     float2* A = sm + N;
-    float2* B = A + RC_ROWS * N;
+    float2* B = A + RC_ROWS * LD;
     for (int t = threadIdx.x; t < N; t += blockDim.x) s_tw[t] = tw[t];
     const int row0 = blockIdx.x * RC_ROWS;
     const int nrows = dim == 3 ? ori * ori : ori;
@@ -126,13 +158,13 @@ __global__ void __launch_bounds__(RC_THREADS) k_rows3(const float2* __restrict__
             else if (k < N / 2) v = g[k];
             else v = make_float2(g[N - k].x, -g[N - k].y);
         }
-        A[e] = v;
+        A[rr * LD + px(k)] = v;
     }
     __syncthreads();
     const float2* r = fft_any<NC, true>(A, B, RC_ROWS, plan, s_tw);
     for (int e = threadIdx.x; e < RC_ROWS * ori; e += blockDim.x) {
         const int rr = e / ori, x = e - rr * ori, row = row0 + rr;
-        if (row < nrows) vol[(size_t)row * ori + x] = r[rr * N + z0 + x].x / norm;
+        if (row < nrows) vol[(size_t)row * ori + x] = r[rr * LD + px(z0 + x)].x / norm;
     }
 }
 
@@ -168,20 +200,28 @@ __global__ void __launch_bounds__(RC_THREADS) k_mask_partial(const float* __rest
 }
 
 // soft mask with the background, then the gridding correction (trilinear: sinc^2)
-__global__ void k_mask_grid(const float* __restrict__ vol, int ori, int dim, int pad, double radius, double width,
+__global__ void __launch_bounds__(RC_THREADS) k_mask_grid(const float* __restrict__ vol, int ori, int dim, int pad, double radius, double width,
                             const double2* __restrict__ part, int nparts, double* __restrict__ out)
 {
-    __shared__ double s_bg;
-    if (threadIdx.x == 0) {
-        double w = 0., v = 0.;
-        for (int b = 0; b < nparts; ++b) {
-            w += part[b].x;
-            v += part[b].y;
-        }
-        s_bg = w > 0. ? v / w : 0.;
+    // every block sums the partial sums in one fixed order: strided by thread, then a tree (one
+    // thread walking 2,368 of them took 120 us of the kernel's 186)
+    __shared__ double sw[RC_THREADS], sv[RC_THREADS];
+    double w0 = 0., v0 = 0.;
+    for (int b = threadIdx.x; b < nparts; b += RC_THREADS) {
+        w0 += part[b].x;
+        v0 += part[b].y;
     }
+    sw[threadIdx.x] = w0;
+    sv[threadIdx.x] = v0;
     __syncthreads();
-    const double bg = s_bg;
+    for (int o = RC_THREADS / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) {
+            sw[threadIdx.x] += sw[threadIdx.x + o];
+            sv[threadIdx.x] += sv[threadIdx.x + o];
+        }
+        __syncthreads();
+    }
+    const double bg = sw[0] > 0. ? sv[0] / sw[0] : 0.;
     const long long total = (long long)ori * ori * (dim == 3 ? ori : 1);
     for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
         const int x = (int)(n % ori), y = (int)((n / ori) % ori), z = (int)(n / ((long long)ori * ori));
@@ -206,108 +246,91 @@ __global__ void k_mask_grid(const float* __restrict__ vol, int ori, int dim, int
 }
 
 // ---------------------------------------------------------------- FSC and SSNR
-__global__ void k_downsample(Volume g, const float2* __restrict__ data, const float* __restrict__ weight,
-                             double* __restrict__ acc /* bins x 3 */)
+// the grid coordinates x with ROUND(x / pad) = q are first(q) .. last(q) (half away from zero)
+__device__ __forceinline__ int ds_first(int q, int pad)
 {
-    const int ds = 2 * (g.r_max + 1) + 1, dh = ds / 2;
-    const long long total = (long long)g.zdim * g.ydim * g.xdim;
-    for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(n % g.xdim), i = (int)((n / g.xdim) % g.ydim), k = (int)(n / ((long long)g.xdim * g.ydim));
-        const int kp = g.ref_dim == 3 ? rround((double)(k + g.initz) / g.pad) + dh : 0;   // 2D: one plane
-        const int ip = rround((double)(i + g.inity) / g.pad) + dh;
-        const int jp = rround((double)j / g.pad);
-        if (kp < 0 || kp >= (g.ref_dim == 3 ? ds : 1) || ip < 0 || ip >= ds || jp > dh) continue;   // a grid larger than pad_size
-        const size_t b = (((size_t)kp * ds + ip) * (dh + 1) + jp) * 3;
-        const float2 d = data[n];
-        const float w = weight[n];
-        if (d.x != 0.f) atomicAdd(&acc[b], (double)d.x);
-        if (d.y != 0.f) atomicAdd(&acc[b + 1], (double)d.y);
-        if (w != 0.f) atomicAdd(&acc[b + 2], (double)w);
-    }
+    if (q > 0) return ((2 * q - 1) * pad + 1) / 2;
+    if (q == 0) return -((pad - 1) / 2);
+    return -(((2 * -q + 1) * pad + 1) / 2 - 1);
+}
+__device__ __forceinline__ int ds_last(int q, int pad)
+{
+    return q >= 0 ? ((2 * q + 1) * pad + 1) / 2 - 1 : -(((2 * -q - 1) * pad + 1) / 2);
 }
 
-// shell sums: FP64 shared-memory bins per block, one global atomic per bin and block
-__device__ __forceinline__ void shell_init(double* sb, int n)
-{
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sb[i] = 0.;
-    __syncthreads();
-}
-__device__ __forceinline__ void shell_flush(const double* sb, int n, double* acc)
-{
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        if (sb[i] != 0.) atomicAdd(&acc[i], sb[i]);
-}
-
-__global__ void k_fsc_shells(int r_max, int nb, int dim, const double* __restrict__ a1, const double* __restrict__ a2,
-                             double* __restrict__ sh /* nb x 3 */)
+// Shell sums of the FSC of two grids after down-sampling to the unpadded box: one thread per bin of
+// the down-sampled box gathers the bin's pad^3 voxels of both grids (FP64, in a fixed order), forms the two
+// averages and adds their products to the shell.  Bound by reading the grids once (210 MB at
+// 259 x 259 x 130: 32 us); scattering every voxel by FP64 atomics into bins in memory took
+// 85 us a grid, and the shells another 33.
+__global__ void __launch_bounds__(RC_THREADS) k_fsc(Volume g, int nb, const float2* __restrict__ d1,
+                                                    const float* __restrict__ w1, const float2* __restrict__ d2,
+                                                    const float* __restrict__ w2, double* __restrict__ sh /* nb x 3 */)
 {
     extern __shared__ double sb[];
-    shell_init(sb, 3 * nb);
-    const int ds = 2 * (r_max + 1) + 1, dh = ds / 2;
-    const long long total = (long long)(dim == 3 ? ds : 1) * ds * (dh + 1);
+    for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x) sb[i] = 0.;
+    __syncthreads();
+    const int ds = 2 * (g.r_max + 1) + 1, dh = ds / 2, r2max = g.r_max * g.r_max;
+    const long long total = (long long)(g.ref_dim == 3 ? ds : 1) * ds * (dh + 1);
     for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
         const int j = (int)(n % (dh + 1)), i = (int)((n / (dh + 1)) % ds) - dh;
-        const int k = dim == 3 ? (int)(n / ((long long)(dh + 1) * ds)) - dh : 0;
-        const double R = sqrt((double)(k * k + i * i + j * j));
-        if (R > r_max) continue;
-        const int idx = rround(R);
-        const double w1 = a1[3 * n + 2], w2 = a2[3 * n + 2];
-        const double r1 = w1 > 0. ? a1[3 * n] / w1 : 0., i1 = w1 > 0. ? a1[3 * n + 1] / w1 : 0.;
-        const double r2 = w2 > 0. ? a2[3 * n] / w2 : 0., i2 = w2 > 0. ? a2[3 * n + 1] / w2 : 0.;
-        atomicAdd(&sb[3 * idx], r1 * r2 + i1 * i2);
+        const int k = g.ref_dim == 3 ? (int)(n / ((long long)(dh + 1) * ds)) - dh : 0;
+        const int r2 = k * k + i * i + j * j;
+        if (r2 > r2max) continue;
+        const int za = g.ref_dim == 3 ? max(ds_first(k, g.pad), g.initz) : 0;
+        const int zb = g.ref_dim == 3 ? min(ds_last(k, g.pad), g.initz + g.zdim - 1) : 0;
+        const int ya = max(ds_first(i, g.pad), g.inity), yb = min(ds_last(i, g.pad), g.inity + g.ydim - 1);
+        const int xa = max(ds_first(j, g.pad), 0), xb = min(ds_last(j, g.pad), g.xdim - 1);
+        double s1[3] = {0., 0., 0.}, s2[3] = {0., 0., 0.};
+        for (int z = za; z <= zb; ++z)
+            for (int y = ya; y <= yb; ++y) {
+                const size_t row = ((size_t)(g.ref_dim == 3 ? z - g.initz : 0) * g.ydim + (y - g.inity)) * g.xdim;
+                for (int x = xa; x <= xb; ++x) {
+                    const float2 a = d1[row + x], b = d2[row + x];
+                    s1[0] += a.x; s1[1] += a.y; s1[2] += w1[row + x];
+                    s2[0] += b.x; s2[1] += b.y; s2[2] += w2[row + x];
+                }
+            }
+        const double r1 = s1[2] > 0. ? s1[0] / s1[2] : 0., i1 = s1[2] > 0. ? s1[1] / s1[2] : 0.;
+        const double rr2 = s2[2] > 0. ? s2[0] / s2[2] : 0., i2 = s2[2] > 0. ? s2[1] / s2[2] : 0.;
+        const int idx = shell_round(r2, 1);
+        atomicAdd(&sb[3 * idx], r1 * rr2 + i1 * i2);
         atomicAdd(&sb[3 * idx + 1], r1 * r1 + i1 * i1);
-        atomicAdd(&sb[3 * idx + 2], r2 * r2 + i2 * i2);
+        atomicAdd(&sb[3 * idx + 2], rr2 * rr2 + i2 * i2);
     }
-    shell_flush(sb, 3 * nb, sh);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x)
+        if (sb[i] != 0.) atomicAdd(&sh[i], sb[i]);
 }
 
 // pass 1 of updateSSNRarrays: per shell, sum of pad^3 weight and count (r^2 < max_r2)
-__global__ void k_ssnr_sigma(Volume g, int nb, const float* __restrict__ weight, double oc, double* __restrict__ acc)
+__global__ void __launch_bounds__(RC_THREADS) k_ssnr_sigma(Volume g, int nb, const float* __restrict__ weight, double oc,
+                                                           double* __restrict__ acc)
 {
     extern __shared__ double sb[];
-    shell_init(sb, 2 * nb);
     const int rp = g.r_max * g.pad;
-    const long long total = (long long)g.zdim * g.ydim * g.xdim;
-    for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(n % g.xdim), i = (int)((n / g.xdim) % g.ydim) + g.inity, k = (int)(n / ((long long)g.xdim * g.ydim)) + g.initz;
-        const int r2 = k * k + i * i + j * j;
-        if (r2 >= rp * rp) continue;
-        const int ires = rround(sqrt((double)r2) / g.pad);
-        atomicAdd(&sb[2 * ires], oc * weight[n]);
-        atomicAdd(&sb[2 * ires + 1], 1.);
-    }
-    shell_flush(sb, 2 * nb, acc);
+    shell_sums<2>(g, rp * rp, nb, sb, acc, [&](int r2) { return shell_round(r2, g.pad); },
+                  [&](long long n, int, int, double* x) {
+                      x[0] = oc * weight[n];
+                      x[1] = 1.;
+                  });
 }
 
-// pass 2: per shell, sum of weight / invtau2 (data vs prior), coverage count, count
-__global__ void k_ssnr_prior(Volume g, int nb, const float* __restrict__ weight, double oc, double tau2_fudge,
-                             const double* __restrict__ tau2, const double* __restrict__ avgctf2, int correct_ctf2,
-                             double* __restrict__ acc)
+// pass 2: per shell, sum of weight / invtau2 (data vs prior), coverage count, count; inv_tau2 per
+// shell, negative where tau2 is not positive (then 1 / (0.001 weight))
+__global__ void __launch_bounds__(RC_THREADS) k_ssnr_prior(Volume g, int nb, const float* __restrict__ weight,
+                                                           const double* __restrict__ inv_tau2, double* __restrict__ acc)
 {
     extern __shared__ double sb[];
-    shell_init(sb, 3 * nb);
     const int rp = g.r_max * g.pad;
-    const long long total = (long long)g.zdim * g.ydim * g.xdim;
-    for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(n % g.xdim), i = (int)((n / g.xdim) % g.ydim) + g.inity, k = (int)(n / ((long long)g.xdim * g.ydim)) + g.initz;
-        const int r2 = k * k + i * i + j * j;
-        if (r2 >= rp * rp) continue;
-        const int ires = rround(sqrt((double)r2) / g.pad);
-        const double invw = weight[n];
-        double invtau2;
-        if (tau2[ires] > 0.) {
-            invtau2 = 1. / (oc * tau2_fudge * tau2[ires]);
-            if (correct_ctf2 && avgctf2[ires] > 0.) invtau2 *= 1. / avgctf2[ires];
-        } else {
-            invtau2 = 1. / (0.001 * invw);
-        }
-        const double ratio = invw / invtau2;
-        atomicAdd(&sb[3 * ires], ratio);
-        if (ratio >= 1.) atomicAdd(&sb[3 * ires + 1], 1.);
-        atomicAdd(&sb[3 * ires + 2], 1.);
-    }
-    shell_flush(sb, 3 * nb, acc);
+    shell_sums<3>(g, rp * rp, nb, sb, acc, [&](int r2) { return shell_round(r2, g.pad); },
+                  [&](long long n, int, int sh, double* x) {
+                      const double invw = weight[n], it = inv_tau2[sh];
+                      const double ratio = invw / (it >= 0. ? it : 1. / (0.001 * invw));
+                      x[0] = ratio;
+                      x[1] = ratio >= 1. ? 1. : 0.;
+                      x[2] = 1.;
+                  });
 }
 
 // BackProjector::enforceHermitianSymmetry (src/backprojector.cpp:2104-2121) on the x = 0
@@ -343,118 +366,158 @@ __global__ void k_hermitian(Volume g, float2* __restrict__ data, float* __restri
 // src/backprojector.cpp:1532-1655): weights w_n (FP64, FFTW layout of the pad_size box)
 // start at 1 inside r^2 < max_r2; each iteration convolves w_n * weight with the blob
 // through the Fourier transform of the full box (BackProjector::convoluteBlobRealSpace,
-// :2439-2480) and divides w_n by max(1e-6, |result|) inside max_r2.  The half-complex grids
-// are expanded to the full complex box by Hermitian symmetry (the box is odd: no Nyquist
-// plane), transformed by the shared-memory FFTs along x, y and z, multiplied in real space
-// by the blob's tabulated Fourier transform over its value at 0, and transformed back.
-constexpr int GD_CX = 8;   // lines per CTA of the full-box transforms
+// :2439-2480) and divides w_n by max(1e-6, |result|) inside max_r2.  w_n * weight is real and
+// symmetric, so the box is kept as its half in x (the box is odd: no Nyquist plane): inverse
+// transforms along z and y of the half, then rows in pairs, complex to real, times the blob's
+// tabulated Fourier transform over its value at 0 and back to the half while they are in shared
+// memory, then y and z forward, the last of them updating w_n.
+// At 259 an iteration took 0.64 ms (was 2.05: six passes over the full box and three over the grid
+// between them) and moves 0.84 GB (0.13 ms at the copy bandwidth): bound by the prime-length stage
+// (fft_stage_prime_first), two blocks a SM.
+constexpr int GD_COL = 0, GD_LOAD = 1, GD_UPDATE = 2;   // k_gd_col: V -> V, w_n weight -> V, V -> w_n
 
-// data and weight divided by `normalise`; w_n = 1 inside r^2 < max_r2, else 0
-__global__ void k_gd_init(double2* __restrict__ fc, double* __restrict__ fw, double* __restrict__ fn, int ps, int nz,
-                          int max_r2, double inv_norm)
+// lines (sequences) per CTA: two buffers of them in about 70 KB, and enough work for 256 threads
+int gd_lines(int N) { return N <= 150 ? 32 : N <= 300 ? 16 : 8; }
+
+// the weights of the pad_size box (FFTW layout, MAP term added, times inv_norm); w_n = 1 inside
+// r^2 < max_r2, else 0
+__global__ void k_gd_init(Volume g, const float* __restrict__ weight, double* __restrict__ fw, double* __restrict__ fn,
+                          const double* __restrict__ inv_tau2, int minres_map, double inv_norm)
 {
-    const int fx = ps / 2 + 1;
+    const int ps = g.ydim, fx = ps / 2 + 1, nz = g.ref_dim == 3 ? ps : 1, rp = g.r_max * g.pad;
     const long long total = (long long)nz * ps * fx;
     for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
         const int j = (int)(n % fx), i = (int)((n / fx) % ps), k = (int)(n / ((long long)fx * ps));
         const int kp = k < fx ? k : k - ps, ip = i < fx ? i : i - ps;
-        const double2 d = fc[n];
-        fc[n] = make_double2(d.x * inv_norm, d.y * inv_norm);
-        fw[n] *= inv_norm;
-        fn[n] = kp * kp + ip * ip + j * j < max_r2 ? 1. : 0.;
+        const int r2 = kp * kp + ip * ip + j * j;
+        double w = 0.;
+        if (r2 <= rp * rp) w = weight[((size_t)(kp - g.initz) * g.ydim + (ip - g.inity)) * g.xdim + j];
+        if (inv_tau2 && r2 < rp * rp) w = map_weight(w, r2, g.pad, inv_tau2, minres_map);
+        fw[n] = w * inv_norm;
+        fn[n] = r2 < rp * rp ? 1. : 0.;
     }
 }
 
-// the full box V[z][y][x] (2D: one plane) of w_n * weight (real), from the half by Hermitian
-// symmetry: x > ps/2 reads (-z, -y, ps - x)
-__global__ void k_gd_expand(const double* __restrict__ fn, const double* __restrict__ fw, int ps, int nz,
-                            float2* __restrict__ V)
+// the blob factor of every squared real-space distance: the table's entry floor(r / 5e-5) at
+// r = sqrt(d2) / (ori_size pad), 0 beyond it (TabFtBlob::operator(), src/tabfuncs.cpp:114-121)
+__global__ void k_gd_blob(const double* __restrict__ ratio, int ntab, double ori_pad, int nd2, double* __restrict__ blob)
 {
-    const int fx = ps / 2 + 1;
-    const long long total = (long long)nz * ps * ps;
-    for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(n % ps), y = (int)((n / ps) % ps), z = (int)(n / ((long long)ps * ps));
-        size_t h;
-        if (x < fx) h = ((size_t)z * ps + y) * fx + x;
-        else h = ((size_t)(nz == 1 ? 0 : (ps - z) % ps) * ps + (ps - y) % ps) * fx + (ps - x);
-        V[n] = make_float2((float)(fn[h] * fw[h]), 0.f);
-    }
+    const int d2 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d2 >= nd2) return;
+    const int id = (int)(sqrt((double)d2) / ori_pad / (0.5 / (double)ntab));
+    blob[d2] = id < ntab ? ratio[id] : 0.;
 }
 
-// FFT of GD_CX lines of the full box along one axis: axis 0 = x (rows blockIdx.x * GD_CX + c),
-// axis 1 = y (plane z = blockIdx.x), axis 2 = z (row y = blockIdx.x); x tile blockIdx.y
-template <bool INV>
-__global__ void __launch_bounds__(RC_THREADS) k_gd_fft(float2* __restrict__ V, int N, int nz, int axis,
-                                                       const float2* __restrict__ tw, FftPlan plan)
+// FFT of nl columns of the half box V[z][y][x] along y (axis 1: plane z = blockIdx.x) or z (axis 2:
+// row y = blockIdx.x); x tile blockIdx.y.  IO: GD_LOAD takes (float)(w_n weight) instead of V,
+// GD_UPDATE divides w_n by max(1e-6, |result| inv_n) inside r^2 < max_r2 instead of storing V.
+template <bool INV, int IO, int NL>
+__global__ void __launch_bounds__(RC_THREADS) k_gd_col(float2* __restrict__ V, double* __restrict__ fn,
+                                                       const double* __restrict__ fw, int N, int axis,
+                                                       const float2* __restrict__ tw, FftPlan plan, int ntable,
+                                                       int max_r2, double inv_n)
 {
-    extern __shared__ float2 sm[];
-    float2* s_tw = sm;
-    float2* A = sm + N;
-    float2* B = A + GD_CX * N;
+    extern __shared__ __align__(16) double2 sm4[];
+    double2* s_pt = sm4;
+    float2* s_tw = reinterpret_cast<float2*>(sm4 + ntable);
+    const int fx = N / 2 + 1;
+    float2* A = s_tw + N;
+    float2* B = A + NL * N;
     for (int t = threadIdx.x; t < N; t += blockDim.x) s_tw[t] = tw[t];
-    const long long nrows = (long long)nz * N;
     const size_t o = blockIdx.x;
-    const int x0 = blockIdx.y * GD_CX;
-    auto ok = [&](int c) -> bool { return axis == 0 ? (long long)o * GD_CX + c < nrows : x0 + c < N; };
+    const int x0 = blockIdx.y * NL;
     auto idx = [&](int q, int c) -> size_t {
-        if (axis == 0) return ((size_t)o * GD_CX + c) * N + q;
-        if (axis == 1) return (o * N + q) * N + x0 + c;
-        return ((size_t)q * N + o) * N + x0 + c;
+        return axis == 1 ? (o * N + q) * fx + x0 + c : ((size_t)q * N + o) * fx + x0 + c;
     };
-    for (int e = threadIdx.x; e < GD_CX * N; e += blockDim.x) {
-        // rows: consecutive threads along the row; columns: along x
-        const int c = axis == 0 ? e / N : e % GD_CX, q = axis == 0 ? e % N : e / GD_CX;
-        A[c * N + q] = ok(c) ? V[idx(q, c)] : make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int e = threadIdx.x; e < NL * N; e += RC_THREADS) {
+        const int c = e % NL, q = e / NL;
+        float2 v = make_float2(0.f, 0.f);
+        if (x0 + c < fx) {
+            const size_t i = idx(q, c);
+            if (IO == GD_LOAD) v.x = (float)(fn[i] * fw[i]);
+            else v = V[i];
+        }
+        A[c * N + q] = v;
+    }
+    fft_prime_table(s_pt, plan);
+    __syncthreads();
+    const float2* r = fft_smem<INV, true>(A, B, NL, plan, s_tw, s_pt);
+#pragma unroll 4
+    for (int e = threadIdx.x; e < NL * N; e += RC_THREADS) {
+        const int c = e % NL, q = e / NL;
+        if (x0 + c >= fx) continue;
+        const size_t i = idx(q, c);
+        const float2 v = r[c * N + q];
+        if (IO == GD_UPDATE) {
+            const int qp = q < fx ? q : q - N, op = (int)o < fx ? (int)o : (int)o - N;
+            const int r2 = (x0 + c) * (x0 + c) + qp * qp + (axis == 1 ? 0 : op * op);   // axis 1: the one plane
+            if (r2 < max_r2) {
+                const double a = sqrt((double)v.x * v.x + (double)v.y * v.y) * inv_n;
+                fn[i] /= (a > 1e-6 ? a : 1e-6);
+            }
+        } else {
+            V[i] = v;
+        }
+    }
+}
+
+// The rows of the half box along x, in pairs (row 2 p as the real, row 2 p + 1 as the imaginary
+// part of one complex sequence): inverse transform to real space, times the blob factor
+// (FP64 product, rounded once), forward transform, separated again.  NL pairs per CTA.
+template <int NL>
+__global__ void __launch_bounds__(RC_THREADS) k_gd_rows(float2* __restrict__ V, int N, int nz,
+                                                        const double* __restrict__ blob, const float2* __restrict__ tw,
+                                                        FftPlan plan, int ntable)
+{
+    extern __shared__ __align__(16) double2 sm4[];
+    double2* s_pt = sm4;
+    float2* s_tw = reinterpret_cast<float2*>(sm4 + ntable);
+    const int fx = N / 2 + 1, ph = N / 2;
+    float2* A = s_tw + N;
+    float2* B = A + NL * N;
+    const int nrows = nz * N, r0 = (int)blockIdx.x * NL * 2;
+    const FastDiv dfx(fx), dn(N);
+    for (int t = threadIdx.x; t < N; t += blockDim.x) s_tw[t] = tw[t];
+#pragma unroll 4
+    for (int e = threadIdx.x; e < NL * fx; e += RC_THREADS) {
+        const int c = dfx.div(e), j = e - c * fx;
+        const int row = r0 + 2 * c;
+        const float2 a = row < nrows ? V[(size_t)row * fx + j] : make_float2(0.f, 0.f);
+        const float2 b = row + 1 < nrows ? V[(size_t)(row + 1) * fx + j] : make_float2(0.f, 0.f);
+        if (j == 0) {
+            A[c * N] = make_float2(a.x, b.x);
+        } else {
+            A[c * N + j] = make_float2(a.x - b.y, a.y + b.x);
+            A[c * N + N - j] = make_float2(a.x + b.y, b.x - a.y);
+        }
+    }
+    fft_prime_table(s_pt, plan);
+    __syncthreads();
+    float2* r = fft_smem<true, true>(A, B, NL, plan, s_tw, s_pt);
+    for (int e = threadIdx.x; e < NL * N; e += RC_THREADS) {
+        const int c = dn.div(e), x = e - c * N;
+        const int kx = x < ph ? x : x - N;
+        float2& q = r[c * N + x];
+        float v[2] = {q.x, q.y};
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int row = r0 + 2 * c + t;
+            if (row >= nrows) continue;
+            const int z = row / N, y = row - z * N;
+            const int ky = y < ph ? y : y - N, kz = nz == 1 ? 0 : (z < ph ? z : z - N);
+            v[t] = (float)((double)v[t] * blob[kz * kz + ky * ky + kx * kx]);
+        }
+        q = make_float2(v[0], v[1]);
     }
     __syncthreads();
-    const float2* r = fft_smem<INV, true>(A, B, GD_CX, plan, s_tw);
-    for (int e = threadIdx.x; e < GD_CX * N; e += blockDim.x) {
-        const int c = axis == 0 ? e / N : e % GD_CX, q = axis == 0 ? e % N : e / GD_CX;
-        if (ok(c)) V[idx(q, c)] = r[c * N + q];
-    }
-}
-
-// real space: multiply by the blob's tabulated Fourier transform at
-// r = |(k, i, j)| / (ori_size pad) (coordinates k < ps/2 ? k : k - ps), entry floor(r / 5e-5),
-// 0 beyond the table (TabFtBlob::operator(), src/tabfuncs.cpp:114-121); the imaginary part
-// (rounding of a Hermitian transform) dropped
-__global__ void k_gd_blob(float2* __restrict__ V, int N, int nz, const double* __restrict__ ratio, int ntab,
-                          double ori_pad)
-{
-    const int ph = N / 2;
-    const long long total = (long long)nz * N * N;
-    for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(n % N), y = (int)((n / N) % N), z = (int)(n / ((long long)N * N));
-        const int kz = nz == 1 ? 0 : (z < ph ? z : z - N), ky = y < ph ? y : y - N, kx = x < ph ? x : x - N;
-        const double rval = sqrt((double)(kz * kz + ky * ky + kx * kx)) / ori_pad;
-        const int id = (int)(rval / (0.5 / (double)ntab));
-        const double m = id < ntab ? ratio[id] : 0.;
-        V[n] = make_float2((float)((double)V[n].x * m), 0.f);
-    }
-}
-
-// w_n /= max(1e-6, |V| / N^d) inside r^2 < max_r2 (the forward transform's 1 / N^d here)
-__global__ void k_gd_update(double* __restrict__ fn, const float2* __restrict__ V, int ps, int nz, int max_r2,
-                            double inv_n)
-{
-    const int fx = ps / 2 + 1;
-    const long long total = (long long)nz * ps * fx;
-    for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(n % fx), i = (int)((n / fx) % ps), k = (int)(n / ((long long)fx * ps));
-        const int kp = k < fx ? k : k - ps, ip = i < fx ? i : i - ps;
-        if (kp * kp + ip * ip + j * j >= max_r2) continue;
-        const float2 v = V[((size_t)k * ps + i) * ps + j];
-        const double a = sqrt((double)v.x * v.x + (double)v.y * v.y) * inv_n;
-        fn[n] /= (a > 1e-6 ? a : 1e-6);
-    }
-}
-
-// Fconv = data * w_n
-__global__ void k_gd_apply(double2* __restrict__ fc, const double* __restrict__ fn, long long total)
-{
-    for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
-        const double2 d = fc[n];
-        fc[n] = make_double2(d.x * fn[n], d.y * fn[n]);
+    const float2* f = fft_smem<false, true>(r, r == A ? B : A, NL, plan, s_tw, s_pt);
+    for (int e = threadIdx.x; e < NL * fx; e += RC_THREADS) {
+        const int c = dfx.div(e), j = e - c * fx;
+        const int row = r0 + 2 * c;
+        const float2 p = f[c * N + j], q = f[c * N + (j ? N - j : 0)];
+        if (row < nrows) V[(size_t)row * fx + j] = make_float2(0.5f * (p.x + q.x), 0.5f * (p.y - q.y));
+        if (row + 1 < nrows) V[(size_t)(row + 1) * fx + j] = make_float2(0.5f * (p.y + q.y), 0.5f * (q.x - p.x));
     }
 }
 
@@ -486,83 +549,129 @@ std::vector<double> ftblob_ratio(int ntab)
 // gets the sum, over the group's operators R other than the identity, of the grid read at
 // R (x, y, z) by trilinear interpolation (the conjugate Friedel partner where the rotated x < 0),
 // added to its own value; data and weight alike.  FP64 coordinates and sums, FP32 grids.
-// With zsh (helical symmetry, BackProjector::applyHelicalSymmetry, src/backprojector.cpp:2122-2277),
-// the data read for operator s is also multiplied by e^{2 pi i z zsh[s]} (z the voxel's own z;
-// zsh[s] = hh rise / (-ori_size pad)), formed as the reference forms it: (ac - bd,
+// With z shifts (helical symmetry, BackProjector::applyHelicalSymmetry, src/backprojector.cpp:2122-2277),
+// the data read for operator s is also multiplied by e^{2 pi i z zsh} (z the voxel's own z;
+// zsh = hh rise / (-ori_size pad)), formed as the reference forms it: (ac - bd,
 // (a + b)(c + d) - ac - bd).
-__global__ void k_symmetrise(Volume g, const float2* __restrict__ data, const float* __restrict__ weight,
-                             float2* __restrict__ sdata, float* __restrict__ sweight, const double* __restrict__ R,
-                             const double* __restrict__ zsh, int nsym, int rmax2)
+// Bound by the gathers (L1 lines touched) and FP64 issue.  The grid is packed first, one 16-byte
+// record per voxel, so a corner is one load instead of a data and a weight load, and a warp takes a
+// 4 x 4 x 2 block of voxels, whose rotated image touches fewer lines than that of 32 voxels in a
+// row.  59 operators on 259 x 259 x 130: 4.2 ms (6.4 with separate grids and rows).
+constexpr int SYM_X = 8, SYM_Y = 8, SYM_Z = 4;   // voxels of a block (8 warps of 4 x 4 x 2)
+constexpr int SYM_MAX_SMEM = 48 * 1024;
+
+__global__ void k_pack(const float2* __restrict__ data, const float* __restrict__ weight, float4* __restrict__ out,
+                       long long total)
 {
-    const long long total = (long long)g.zdim * g.ydim * g.xdim;
-    const size_t plane = (size_t)g.ydim * g.xdim;
     for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < total; n += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(n % g.xdim), i = (int)((n / g.xdim) % g.ydim), k = (int)(n / (long long)plane);
-        const int x = j, y = i + g.inity, z = k + g.initz;
-        double sr = data[n].x, si = data[n].y, sw = weight[n];
-        if (x * x + y * y + z * z <= rmax2) {
-            for (int s = 0; s < nsym; ++s) {
-                const double* m = R + 9 * s;
-                // rounded products and sums in the reference's order (no contraction), so
-                // that floor() and the sign test see the reference's coordinates
-                double xp = __dadd_rn(__dadd_rn(__dmul_rn(x, m[0]), __dmul_rn(y, m[1])), __dmul_rn(z, m[2]));
-                double yp = __dadd_rn(__dadd_rn(__dmul_rn(x, m[3]), __dmul_rn(y, m[4])), __dmul_rn(z, m[5]));
-                double zp = __dadd_rn(__dadd_rn(__dmul_rn(x, m[6]), __dmul_rn(y, m[7])), __dmul_rn(z, m[8]));
-                const bool neg = xp < 0;
-                if (neg) { xp = -xp; yp = -yp; zp = -zp; }
-                const int x0 = (int)floor(xp), y0f = (int)floor(yp), z0f = (int)floor(zp);
-                const double fx = xp - x0, fy = yp - y0f, fz = zp - z0f;
-                const int y0 = y0f - g.inity, z0 = z0f - g.initz;
-                if (x0 < 0 || x0 + 1 >= g.xdim || y0 < 0 || y0 + 1 >= g.ydim || z0 < 0 || z0 + 1 >= g.zdim) continue;
-                const size_t b = ((size_t)z0 * g.ydim + y0) * g.xdim + x0;
-                const size_t c[8] = {b, b + 1, b + g.xdim, b + g.xdim + 1,
-                                     b + plane, b + plane + 1, b + plane + g.xdim, b + plane + g.xdim + 1};
-                // (z, y, x) corners: 000 001 010 011 100 101 110 111
-                double dr[8], di[8], dw[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    dr[q] = data[c[q]].x;
-                    di[q] = data[c[q]].y;
-                    dw[q] = weight[c[q]];
-                }
-                const auto tri = [&](const double* d) {
-                    const double x00 = d[0] + (d[1] - d[0]) * fx, x01 = d[4] + (d[5] - d[4]) * fx;
-                    const double x10 = d[2] + (d[3] - d[2]) * fx, x11 = d[6] + (d[7] - d[6]) * fx;
-                    const double y0v = x00 + (x10 - x00) * fy, y1v = x01 + (x11 - x01) * fy;
-                    return y0v + (y1v - y0v) * fz;
-                };
-                double cr = tri(dr), ci = neg ? -tri(di) : tri(di);
-                if (zsh && zsh[s] != 0.) {
-                    double sn, cs;
-                    sincos(2. * PI_R * (z * zsh[s]), &sn, &cs);
-                    const double ac = cs * cr, bd = sn * ci, abcd = (cs + sn) * (cr + ci);
-                    cr = ac - bd;
-                    ci = abcd - ac - bd;
-                }
-                sr += cr;
-                si += ci;
-                sw += tri(dw);
-            }
-        }
-        sdata[n] = make_float2((float)sr, (float)si);
-        sweight[n] = (float)sw;
+        const float2 d = data[n];
+        out[n] = make_float4(d.x, d.y, weight[n], 0.f);
     }
 }
 
-template <typename T>
-struct DevBuf {
-    T* p = nullptr;
-    explicit DevBuf(size_t n)
-    {
-        if (cudaMalloc(&p, (n ? n : 1) * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
-            p = nullptr;
-            throw Error{T2B_ERR_NOMEM, "reconstruction buffers"};
+// in: the packed grid as it was; data, weight: the grid, replaced.  ops: nsym x 10 (R row-major, z shift)
+__global__ void __launch_bounds__(RC_THREADS) k_symmetrise(Volume g, const float4* __restrict__ in,
+                                                           float2* __restrict__ data, float* __restrict__ weight,
+                                                           const double* __restrict__ ops, int nsym, int rmax2)
+{
+    extern __shared__ double s_ops[];
+    const bool staged = (size_t)nsym * 10 * sizeof(double) <= SYM_MAX_SMEM;
+    if (staged)
+        for (int i = threadIdx.x; i < 10 * nsym; i += RC_THREADS) s_ops[i] = ops[i];
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int j = blockIdx.x * SYM_X + (warp & 1) * 4 + (lane & 3);
+    const int i = blockIdx.y * SYM_Y + ((warp >> 1) & 1) * 4 + ((lane >> 2) & 3);
+    const int k = blockIdx.z * SYM_Z + (warp >> 2) * 2 + (lane >> 4);
+    if (j >= g.xdim || i >= g.ydim || k >= g.zdim) return;
+    const int x = j, y = i + g.inity, z = k + g.initz;
+    if (x * x + y * y + z * z > rmax2) return;
+    const size_t plane = (size_t)g.ydim * g.xdim, n = (size_t)k * plane + (size_t)i * g.xdim + j;
+    const float4 own = in[n];
+    double sr = own.x, si = own.y, sw = own.z;
+    for (int s = 0; s < nsym; ++s) {
+        const double* m = (staged ? s_ops : ops) + 10 * s;
+        // rounded products and sums in the reference's order (no contraction), so
+        // that floor() and the sign test see the reference's coordinates
+        double xp = __dadd_rn(__dadd_rn(__dmul_rn(x, m[0]), __dmul_rn(y, m[1])), __dmul_rn(z, m[2]));
+        double yp = __dadd_rn(__dadd_rn(__dmul_rn(x, m[3]), __dmul_rn(y, m[4])), __dmul_rn(z, m[5]));
+        double zp = __dadd_rn(__dadd_rn(__dmul_rn(x, m[6]), __dmul_rn(y, m[7])), __dmul_rn(z, m[8]));
+        const bool neg = xp < 0;
+        if (neg) { xp = -xp; yp = -yp; zp = -zp; }
+        const int x0 = __double2int_rd(xp), y0f = __double2int_rd(yp), z0f = __double2int_rd(zp);
+        const double fx = xp - x0, fy = yp - y0f, fz = zp - z0f;
+        const int y0 = y0f - g.inity, z0 = z0f - g.initz;
+        if (x0 < 0 || x0 + 1 >= g.xdim || y0 < 0 || y0 + 1 >= g.ydim || z0 < 0 || z0 + 1 >= g.zdim) continue;
+        const float4* c = in + ((size_t)z0 * g.ydim + y0) * g.xdim + x0;
+        // (z, y, x) corners: 000 001 010 011 100 101 110 111
+        const float4 d[8] = {c[0], c[1], c[g.xdim], c[g.xdim + 1], c[plane], c[plane + 1], c[plane + g.xdim],
+                             c[plane + g.xdim + 1]};
+        const auto tri = [&](float v0, float v1, float v2, float v3, float v4, float v5, float v6, float v7) {
+            const double d0 = v0, d2 = v2, d4 = v4, d6 = v6;
+            const double x00 = d0 + (v1 - d0) * fx, x01 = d4 + (v5 - d4) * fx;
+            const double x10 = d2 + (v3 - d2) * fx, x11 = d6 + (v7 - d6) * fx;
+            const double y0v = x00 + (x10 - x00) * fy, y1v = x01 + (x11 - x01) * fy;
+            return y0v + (y1v - y0v) * fz;
+        };
+        double cr = tri(d[0].x, d[1].x, d[2].x, d[3].x, d[4].x, d[5].x, d[6].x, d[7].x);
+        double ci = tri(d[0].y, d[1].y, d[2].y, d[3].y, d[4].y, d[5].y, d[6].y, d[7].y);
+        if (neg) ci = -ci;
+        if (m[9] != 0.) {
+            double sn, cs;
+            sincos(2. * PI_R * (z * m[9]), &sn, &cs);
+            const double ac = cs * cr, bd = sn * ci, abcd = (cs + sn) * (cr + ci);
+            cr = ac - bd;
+            ci = abcd - ac - bd;
         }
+        sr += cr;
+        si += ci;
+        sw += tri(d[0].z, d[1].z, d[2].z, d[3].z, d[4].z, d[5].z, d[6].z, d[7].z);
     }
-    ~DevBuf() { cudaFree(p); }
-    DevBuf(const DevBuf&) = delete;
-    DevBuf& operator=(const DevBuf&) = delete;
+    data[n] = make_float2((float)sr, (float)si);
+    weight[n] = (float)sw;
+}
+
+// Device memory of one M-step call, taken in 256-byte steps from the context's scratch.  The
+// scratch stays with the context up to KEEP bytes (an M-step needs it for every class of every
+// iteration, and allocating and freeing 300 MB cost 4.4 ms of a box-128 M-step's 8.4; it takes 3.0 now); beyond that it
+// is given back when the call ends, and always by t2b_configure and whatever else takes memory for
+// good (t2b_ctx::release_scratch).  Calls of one context hold its mutex.
+class Scratch {
+public:
+    static constexpr size_t KEEP = size_t(5) << 28;   // a packed 515 x 515 x 258 grid fits
+    Scratch(t2b_ctx* c, size_t bytes) : c_(c)
+    {
+        if (c->ms_bytes >= bytes) return;
+        c->release_scratch();
+        if (cudaMalloc(&c->ms_scratch, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            c->ms_scratch = nullptr;
+            throw Error{T2B_ERR_NOMEM, "M-step scratch of " + std::to_string(bytes) + " bytes"};
+        }
+        c->ms_bytes = bytes;
+    }
+    ~Scratch()
+    {
+        if (c_->ms_bytes <= KEEP) return;
+        cudaStreamSynchronize(c_->stream);
+        cudaFree(c_->ms_scratch);
+        c_->ms_scratch = nullptr;
+        c_->ms_bytes = 0;
+    }
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    template <typename T> static size_t size(size_t n) { return (n * sizeof(T) + 255) & ~size_t(255); }
+    template <typename T> T* take(size_t n)
+    {
+        T* p = reinterpret_cast<T*>(static_cast<char*>(c_->ms_scratch) + used_);
+        used_ += size<T>(n);
+        T2B_REQUIRE(used_ <= c_->ms_bytes, T2B_ERR_STATE, "M-step scratch exceeded");
+        return p;
+    }
+
+private:
+    t2b_ctx* c_;
+    size_t used_ = 0;
 };
 
 using ColKernel = void (*)(float2*, int, int, int, const float2*, FftPlan);
@@ -580,48 +689,67 @@ int grid_of(long long total)
     return (int)std::min<long long>((total + RC_THREADS - 1) / RC_THREADS, 148LL * 16);
 }
 
-// the gridding iterations on (fc, fw) of the pad_size box, in place: fc becomes data * w_n
-void gridding_weights(const Volume& v, int ori, int pad, int niter, double normalise, double2* fc, double* fw,
-                      cudaStream_t st)
+constexpr int GD_NTAB = 10000;
+size_t gridding_bytes(const Volume& v)
+{
+    const size_t ps = v.ydim, nz = v.ref_dim == 3 ? ps : 1, nh = nz * ps * (ps / 2 + 1), ph = ps / 2 + 1;
+    return 2 * Scratch::size<double>(nh) + Scratch::size<float2>(nh) + Scratch::size<float2>(ps) +
+           Scratch::size<double>(GD_NTAB) + Scratch::size<double>((v.ref_dim == 3 ? 3 : 2) * ph * ph + 1);
+}
+
+// the gridding iterations: returns the weights w_n (FFTW layout of the pad_size box, in `sc`)
+const double* gridding_weights(const Volume& v, const float* weight, int ori, int pad, int niter, double normalise,
+                               const double* inv_tau2, int minres_map, Scratch& sc, cudaStream_t st)
 {
     const int ps = v.ydim, nz = v.ref_dim == 3 ? ps : 1, fx = ps / 2 + 1;
-    const int rp = v.r_max * pad;
-    const int max_r2 = rp * rp;
-    const long long nh = (long long)nz * ps * fx, nf = (long long)nz * ps * ps;
-    const size_t smem = sizeof(float2) * ((size_t)ps + 2 * (size_t)GD_CX * ps);
-    T2B_REQUIRE(smem <= 227 * 1024, T2B_ERR_UNSUPPORTED, "pad_size box too large for the gridding transforms");
+    const int rp = v.r_max * pad, max_r2 = rp * rp;
+    const long long nh = (long long)nz * ps * fx;
     const FftPlan plan = fft_plan(ps, true);
-    constexpr int ntab = 10000;
-    DevBuf<double> fn(nh), ratio(ntab);
-    DevBuf<float2> V(nf), tw(ps);
+    const int nl = gd_lines(ps), ntable = fft_prime_table_entries(plan);
+    const size_t smem = ntable * sizeof(double2) + sizeof(float2) * ((size_t)ps + 2 * (size_t)nl * ps);
+    T2B_REQUIRE(smem <= 227 * 1024, T2B_ERR_UNSUPPORTED, "pad_size box too large for the gridding transforms");
+    double* fn = sc.take<double>(nh);
+    double* fw = sc.take<double>(nh);
+    float2* V = sc.take<float2>(nh);
+    float2* tw = sc.take<float2>(ps);
+    double* ratio = sc.take<double>(GD_NTAB);
+    const int nd2 = (v.ref_dim == 3 ? 3 : 2) * fx * fx + 1;
+    double* blob = sc.take<double>(nd2);
     std::vector<float2> htw(ps);
     for (int t = 0; t < ps; ++t) {
         const double a = -2.0 * PI_R * (double)t / (double)ps;
         htw[t] = make_float2((float)std::cos(a), (float)std::sin(a));
     }
-    const std::vector<double> hr = ftblob_ratio(ntab);
-    T2B_CUDA(cudaMemcpyAsync(tw.p, htw.data(), ps * sizeof(float2), cudaMemcpyHostToDevice, st));
-    T2B_CUDA(cudaMemcpyAsync(ratio.p, hr.data(), ntab * sizeof(double), cudaMemcpyHostToDevice, st));
-    T2B_CUDA(cudaFuncSetAttribute((const void*)k_gd_fft<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    T2B_CUDA(cudaFuncSetAttribute((const void*)k_gd_fft<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int xt = (ps + GD_CX - 1) / GD_CX;
-    const auto fft3 = [&](auto kern) {
-        kern<<<(int)((nz * (long long)ps + GD_CX - 1) / GD_CX), RC_THREADS, smem, st>>>(V.p, ps, nz, 0, tw.p, plan);
-        kern<<<dim3(nz, xt), RC_THREADS, smem, st>>>(V.p, ps, nz, 1, tw.p, plan);
-        if (nz > 1) kern<<<dim3(ps, xt), RC_THREADS, smem, st>>>(V.p, ps, nz, 2, tw.p, plan);
-    };
+    const std::vector<double> hr = ftblob_ratio(GD_NTAB);
+    T2B_CUDA(cudaMemcpyAsync(tw, htw.data(), ps * sizeof(float2), cudaMemcpyHostToDevice, st));
+    T2B_CUDA(cudaMemcpyAsync(ratio, hr.data(), GD_NTAB * sizeof(double), cudaMemcpyHostToDevice, st));
     const double inv_n = 1.0 / ((double)ps * ps * (nz > 1 ? ps : 1));
-    k_gd_init<<<grid_of(nh), RC_THREADS, 0, st>>>(fc, fw, fn.p, ps, nz, max_r2, 1.0 / normalise);
-    for (int it = 0; it < niter; ++it) {
-        k_gd_expand<<<grid_of(nf), RC_THREADS, 0, st>>>(fn.p, fw, ps, nz, V.p);
-        fft3(k_gd_fft<true>);
-        k_gd_blob<<<grid_of(nf), RC_THREADS, 0, st>>>(V.p, ps, nz, ratio.p, ntab, (double)ori * pad);
-        fft3(k_gd_fft<false>);
-        k_gd_update<<<grid_of(nh), RC_THREADS, 0, st>>>(fn.p, V.p, ps, nz, max_r2, inv_n);
-    }
-    k_gd_apply<<<grid_of(nh), RC_THREADS, 0, st>>>(fc, fn.p, nh);
+    k_gd_init<<<grid_of(nh), RC_THREADS, 0, st>>>(v, weight, fw, fn, inv_tau2, minres_map, 1.0 / normalise);
+    k_gd_blob<<<(nd2 + RC_THREADS - 1) / RC_THREADS, RC_THREADS, 0, st>>>(ratio, GD_NTAB, (double)ori * pad, nd2, blob);
+    const auto iterations = [&](auto lines) {
+        constexpr int NL = decltype(lines)::value;
+        const auto load = k_gd_col<true, GD_LOAD, NL>, inv = k_gd_col<true, GD_COL, NL>;
+        const auto fwd = k_gd_col<false, GD_COL, NL>, update = k_gd_col<false, GD_UPDATE, NL>;
+        for (const void* f : {(const void*)load, (const void*)inv, (const void*)fwd, (const void*)update,
+                              (const void*)k_gd_rows<NL>})
+            T2B_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const dim3 gz(ps, (fx + NL - 1) / NL), gy(nz, (fx + NL - 1) / NL);
+        const int gr = (int)(((long long)nz * ps + 2 * NL - 1) / (2 * NL));
+        for (int it = 0; it < niter; ++it) {
+            // the one plane of a 2D grid has its y pass only
+            load<<<nz > 1 ? gz : gy, RC_THREADS, smem, st>>>(V, fn, fw, ps, nz > 1 ? 2 : 1, tw, plan, ntable, 0, 0.);
+            if (nz > 1) inv<<<gy, RC_THREADS, smem, st>>>(V, fn, fw, ps, 1, tw, plan, ntable, 0, 0.);
+            k_gd_rows<NL><<<gr, RC_THREADS, smem, st>>>(V, ps, nz, blob, tw, plan, ntable);
+            if (nz > 1) fwd<<<gy, RC_THREADS, smem, st>>>(V, fn, fw, ps, 1, tw, plan, ntable, 0, 0.);
+            update<<<nz > 1 ? gz : gy, RC_THREADS, smem, st>>>(V, fn, fw, ps, nz > 1 ? 2 : 1, tw, plan, ntable, max_r2, inv_n);
+        }
+    };
+    if (nl == 32) iterations(std::integral_constant<int, 32>{});
+    else if (nl == 16) iterations(std::integral_constant<int, 16>{});
+    else iterations(std::integral_constant<int, 8>{});
     T2B_CUDA(cudaGetLastError());
-    T2B_CUDA(cudaStreamSynchronize(st));   // the buffers above are freed on return
+    T2B_CUDA(cudaStreamSynchronize(st));   // the host tables above are read by the copies
+    return fn;
 }
 
 const Volume& grid_volume(t2b_ctx* c, int ig)
@@ -789,9 +917,8 @@ using namespace t2b;
 
 namespace t2b {
 namespace {
-// the grid of a class summed over operators (and, for helical symmetry, z phase shifts) in place:
-// the sums go to the context's scratch (kept between calls: an M-step symmetrises every class of
-// every iteration), copied back once the kernel has read the whole grid.  C1 (no operator) and
+// the grid of a class summed over operators (and, for helical symmetry, z phase shifts) in place: the
+// sums are read from a packed copy of the grid in the context's scratch.  C1 (no operator) and
 // 2D grids are left as they are, as the reference leaves them.
 void symmetrise_grid(t2b_ctx* c, int iclass, const std::vector<std::array<double, 9>>& ops,
                      const std::vector<double>& zsh)
@@ -801,36 +928,21 @@ void symmetrise_grid(t2b_ctx* c, int iclass, const std::vector<std::array<double
     const int rp = v.r_max * v.pad;
     const size_t nv = v.nvox();
     cudaStream_t st = c->stream;
-    std::vector<double> hr(9 * ops.size());
-    for (size_t i = 0; i < ops.size(); ++i)
-        for (int e = 0; e < 9; ++e) hr[9 * i + e] = ops[i][e];
-    hr.insert(hr.end(), zsh.begin(), zsh.end());
-    // [operators | sums of the data (float2) | sums of the weights], each part 256-byte aligned
-    const size_t r_bytes = (hr.size() * sizeof(double) + 255) & ~size_t(255);
-    const size_t d_bytes = (nv * sizeof(float2) + 255) & ~size_t(255);
-    const size_t need = r_bytes + d_bytes + nv * sizeof(float);
-    if (c->sym_bytes < need) {
-        T2B_CUDA(cudaStreamSynchronize(st));
-        cudaFree(c->sym_scratch);
-        c->sym_scratch = nullptr;
-        c->sym_bytes = 0;
-        if (cudaMalloc(&c->sym_scratch, need) != cudaSuccess) {
-            cudaGetLastError();
-            throw Error{T2B_ERR_NOMEM, "symmetrisation scratch of " + std::to_string(need) + " bytes"};
-        }
-        c->sym_bytes = need;
+    std::vector<double> hr(10 * ops.size(), 0.);
+    for (size_t i = 0; i < ops.size(); ++i) {
+        for (int e = 0; e < 9; ++e) hr[10 * i + e] = ops[i][e];
+        if (!zsh.empty()) hr[10 * i + 9] = zsh[i];
     }
-    char* base = static_cast<char*>(c->sym_scratch);
-    double* R = reinterpret_cast<double*>(base);
-    float2* sd = reinterpret_cast<float2*>(base + r_bytes);
-    float* sw = reinterpret_cast<float*>(base + r_bytes + d_bytes);
+    Scratch sc(c, Scratch::size<double>(hr.size()) + Scratch::size<float4>(nv));
+    double* R = sc.take<double>(hr.size());
+    float4* packed = sc.take<float4>(nv);
     T2B_CUDA(cudaMemcpyAsync(R, hr.data(), hr.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    k_symmetrise<<<grid_of((long long)nv), RC_THREADS, 0, st>>>(v, c->gdata[iclass], c->gweight[iclass], sd, sw, R,
-                                                               zsh.empty() ? nullptr : R + 9 * ops.size(),
-                                                               (int)ops.size(), rp * rp);
+    k_pack<<<grid_of((long long)nv), RC_THREADS, 0, st>>>(c->gdata[iclass], c->gweight[iclass], packed, (long long)nv);
+    const size_t smem = hr.size() * sizeof(double) <= SYM_MAX_SMEM ? hr.size() * sizeof(double) : 0;
+    const dim3 grid((v.xdim + SYM_X - 1) / SYM_X, (v.ydim + SYM_Y - 1) / SYM_Y, (v.zdim + SYM_Z - 1) / SYM_Z);
+    k_symmetrise<<<grid, RC_THREADS, smem, st>>>(v, packed, c->gdata[iclass], c->gweight[iclass], R, (int)ops.size(),
+                                                rp * rp);
     T2B_CUDA(cudaGetLastError());
-    T2B_CUDA(cudaMemcpyAsync(c->gdata[iclass], sd, nv * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-    T2B_CUDA(cudaMemcpyAsync(c->gweight[iclass], sw, nv * sizeof(float), cudaMemcpyDeviceToDevice, st));
     T2B_CUDA(cudaStreamSynchronize(st));   // the host table hr is read by the copy above
 }
 }  // namespace
@@ -854,62 +966,71 @@ int t2b_reconstruct(t2b_ctx* c, int iclass, const t2b_recon_config* cf, double* 
         T2B_REQUIRE(N <= 512, T2B_ERR_UNSUPPORTED, "pad * ori_size must be <= 512");
         const FftPlan plan = fft_plan(N);
         const int dim = v.ref_dim;
-        const int ps = v.ydim, fx = ps / 2 + 1, h = N / 2 + 1;
-        const size_t nps = (size_t)(dim == 3 ? ps : 1) * ps * fx;
+        const int h = N / 2 + 1;
         cudaStream_t st = c->stream;
-        DevBuf<double2> fc(nps);
-        DevBuf<double> fw(nps), rad(2 * (size_t)v.r_max), t2(ori / 2 + 1);
-        if (cf->do_map)
-            T2B_CUDA(cudaMemcpyAsync(t2.p, cf->tau2, (ori / 2 + 1) * sizeof(double), cudaMemcpyHostToDevice, st));
-        const double tscale = (dim == 3 ? (double)pad * pad * pad : (double)pad * pad) * cf->tau2_fudge;
-        if (cf->gridding_iter > 0) {
+        const long long nv = (long long)ori * ori * (dim == 3 ? ori : 1);
+        const size_t ng = (size_t)(dim == 3 ? N : 1) * N * h;
+        const int nb = (int)std::min<long long>((nv + RC_THREADS - 1) / RC_THREADS, 148LL * 4);
+        const bool gridding = cf->gridding_iter > 0;
+        T2B_REQUIRE(!gridding || cf->normalise > 0., T2B_ERR_ARG,
+                    "gridding iterations need normalise > 0 (the class's sum of weights)");
+        using S = Scratch;
+        S sc(c, S::size<double>(3 * (size_t)v.r_max) + S::size<double>(ori / 2 + 1) + S::size<float2>(ng) + S::size<float2>(N) +
+                    S::size<float>(nv) + S::size<double2>(nb) + S::size<double>(nv) + (gridding ? gridding_bytes(v) : 0));
+        double* rad = sc.take<double>(3 * (size_t)v.r_max);
+        double* t2 = sc.take<double>(ori / 2 + 1);
+        // the MAP term's 1 / (pad^3 tau2_fudge tau2) per shell, negative where tau2 is not positive
+        std::vector<double> it2(ori / 2 + 1);
+        if (cf->do_map) {
+            const double tscale = (dim == 3 ? (double)pad * pad * pad : (double)pad * pad) * cf->tau2_fudge;
+            for (int i = 0; i <= ori / 2; ++i) it2[i] = cf->tau2[i] > 0. ? 1. / (tscale * cf->tau2[i]) : -1.;
+            T2B_CUDA(cudaMemcpyAsync(t2, it2.data(), it2.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+        }
+        Divide dv{rad, cf->do_map ? t2 : nullptr, cf->minres_map, nullptr, 1.};
+        if (gridding) {
             // --dont_skip_gridding: the iterative weights in place of the division
-            T2B_REQUIRE(cf->normalise > 0., T2B_ERR_ARG,
-                        "gridding iterations need normalise > 0 (the class's sum of weights)");
-            launch_decenter(v, c->gdata[iclass], c->gweight[iclass], fc.p, fw.p, rad.p, rad.p + v.r_max, st,
-                            cf->do_map ? t2.p : nullptr, tscale, cf->minres_map);
-            gridding_weights(v, ori, pad, cf->gridding_iter, cf->normalise, fc.p, fw.p, st);
+            dv.fn = gridding_weights(v, c->gweight[iclass], ori, pad, cf->gridding_iter, cf->normalise, dv.inv_tau2,
+                                     cf->minres_map, sc, st);
+            dv.inv_norm = 1.0 / cf->normalise;
         } else {
-            launch_reconstruct(v, c->gdata[iclass], c->gweight[iclass], fc.p, fw.p, rad.p, rad.p + v.r_max, st,
-                               cf->do_map ? t2.p : nullptr, tscale, cf->minres_map);
+            launch_radial(v, c->gweight[iclass], rad, rad + v.r_max, st, dv.inv_tau2, cf->minres_map);
         }
         // window + centre by sign, inverse 3D FFT, real-space window
-        DevBuf<float2> G((size_t)(dim == 3 ? N : 1) * N * h), tw(N);
+        float2* G = sc.take<float2>(ng);
+        float2* tw = sc.take<float2>(N);
         std::vector<float2> htw(N);
         for (int t = 0; t < N; ++t) {
             const double a = -2.0 * PI_R * (double)t / (double)N;
             htw[t] = make_float2((float)std::cos(a), (float)std::sin(a));
         }
-        T2B_CUDA(cudaMemcpyAsync(tw.p, htw.data(), N * sizeof(float2), cudaMemcpyHostToDevice, st));
-        k_window<<<grid_of((long long)(dim == 3 ? N : 1) * N * h), RC_THREADS, 0, st>>>(fc.p, ps, N, dim, G.p);
+        T2B_CUDA(cudaMemcpyAsync(tw, htw.data(), N * sizeof(float2), cudaMemcpyHostToDevice, st));
+        k_window<<<grid_of((long long)ng), RC_THREADS, 0, st>>>(v, c->gdata[iclass], c->gweight[iclass], dv, N, G);
         ColKernel col;
         RowKernel row;
         recon_kernels(N, col, row);
-        const size_t smc = sizeof(float2) * ((size_t)N + 2 * (size_t)RC_CX * N);
-        const size_t smr = sizeof(float2) * ((size_t)N + 2 * (size_t)RC_ROWS * N);
+        const size_t smc = sizeof(float2) * ((size_t)N + 2 * (size_t)RC_CX * fft_ld(N));
+        const size_t smr = sizeof(float2) * ((size_t)N + 2 * (size_t)RC_ROWS * fft_ld(N));
         T2B_CUDA(cudaFuncSetAttribute((const void*)col, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smc));
         T2B_CUDA(cudaFuncSetAttribute((const void*)row, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr));
         const int z0 = N / 2 - ori / 2, xt = (h + RC_CX - 1) / RC_CX;
         if (dim == 3) {
-            col<<<dim3(N, xt), RC_THREADS, smc, st>>>(G.p, N, 0, 0, tw.p, plan);          // along z, every (y, x)
-            col<<<dim3(ori, xt), RC_THREADS, smc, st>>>(G.p, N, 1, z0, tw.p, plan);       // along y, window planes
+            col<<<dim3(N, xt), RC_THREADS, smc, st>>>(G, N, 0, 0, tw, plan);          // along z, every (y, x)
+            col<<<dim3(ori, xt), RC_THREADS, smc, st>>>(G, N, 1, z0, tw, plan);       // along y, window planes
         } else {
-            col<<<dim3(1, xt), RC_THREADS, smc, st>>>(G.p, N, 1, 0, tw.p, plan);          // along y, the one plane
+            col<<<dim3(1, xt), RC_THREADS, smc, st>>>(G, N, 1, 0, tw, plan);          // along y, the one plane
         }
-        const long long nv = (long long)ori * ori * (dim == 3 ? ori : 1);
-        DevBuf<float> vol(nv);
+        float* vol = sc.take<float>(nv);
         // normalisation of windowToOridimRealSpace for 2D particles: pad^3 ori (3D maps), pad^2 (2D)
         const float norm = dim == 3 ? (float)((double)pad * pad * pad * ori) : (float)((double)pad * pad);
         const int nrows = dim == 3 ? ori * ori : ori;
-        row<<<(nrows + RC_ROWS - 1) / RC_ROWS, RC_THREADS, smr, st>>>(G.p, N, ori, z0, norm, tw.p, plan, vol.p, dim);
+        row<<<(nrows + RC_ROWS - 1) / RC_ROWS, RC_THREADS, smr, st>>>(G, N, ori, z0, norm, tw, plan, vol, dim);
         // soft mask (radius ori/2, width 3, average background) and gridding correction
-        const int nb = grid_of(nv);
-        DevBuf<double2> part(nb);
-        DevBuf<double> out(nv);
-        k_mask_partial<<<nb, RC_THREADS, 0, st>>>(vol.p, ori, dim, ori / 2.0, 3.0, part.p);
-        k_mask_grid<<<nb, RC_THREADS, 0, st>>>(vol.p, ori, dim, pad, ori / 2.0, 3.0, part.p, nb, out.p);
+        double2* part = sc.take<double2>(nb);
+        double* out = sc.take<double>(nv);
+        k_mask_partial<<<nb, RC_THREADS, 0, st>>>(vol, ori, dim, ori / 2.0, 3.0, part);
+        k_mask_grid<<<nb, RC_THREADS, 0, st>>>(vol, ori, dim, pad, ori / 2.0, 3.0, part, nb, out);
         T2B_CUDA(cudaGetLastError());
-        T2B_CUDA(cudaMemcpyAsync(vol_out, out.p, nv * sizeof(double), cudaMemcpyDeviceToHost, st));
+        T2B_CUDA(cudaMemcpyAsync(vol_out, out, nv * sizeof(double), cudaMemcpyDeviceToHost, st));
         T2B_CUDA(cudaStreamSynchronize(st));
     });
 }
@@ -995,18 +1116,14 @@ int t2b_fsc_halves(t2b_ctx* c, int grid_a, int grid_b, int ori_size, double* fsc
         T2B_REQUIRE(nb <= 1024, T2B_ERR_ARG, "ori_size too large");
         const size_t bins = (size_t)(a.ref_dim == 3 ? ds : 1) * ds * (dh + 1);
         cudaStream_t st = c->stream;
-        DevBuf<double> aa(3 * bins), ab(3 * bins), sh(3 * (size_t)nb);
-        T2B_CUDA(cudaMemsetAsync(aa.p, 0, 3 * bins * sizeof(double), st));
-        T2B_CUDA(cudaMemsetAsync(ab.p, 0, 3 * bins * sizeof(double), st));
-        T2B_CUDA(cudaMemsetAsync(sh.p, 0, 3 * (size_t)nb * sizeof(double), st));
-        const long long nvox = (long long)a.zdim * a.ydim * a.xdim;
-        k_downsample<<<grid_of(nvox), RC_THREADS, 0, st>>>(a, c->gdata[grid_a], c->gweight[grid_a], aa.p);
-        k_downsample<<<grid_of(nvox), RC_THREADS, 0, st>>>(b, c->gdata[grid_b], c->gweight[grid_b], ab.p);
-        k_fsc_shells<<<grid_of((long long)bins), RC_THREADS, 3 * nb * sizeof(double), st>>>(a.r_max, nb, a.ref_dim, aa.p,
-                                                                                             ab.p, sh.p);
+        Scratch sc(c, Scratch::size<double>(3 * (size_t)nb));
+        double* sh = sc.take<double>(3 * (size_t)nb);
+        T2B_CUDA(cudaMemsetAsync(sh, 0, 3 * (size_t)nb * sizeof(double), st));
+        k_fsc<<<grid_of((long long)bins), RC_THREADS, 3 * nb * sizeof(double), st>>>(
+            a, nb, c->gdata[grid_a], c->gweight[grid_a], c->gdata[grid_b], c->gweight[grid_b], sh);
         T2B_CUDA(cudaGetLastError());
         std::vector<double> h(3 * (size_t)nb);
-        T2B_CUDA(cudaMemcpyAsync(h.data(), sh.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+        T2B_CUDA(cudaMemcpyAsync(h.data(), sh, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
         T2B_CUDA(cudaStreamSynchronize(st));
         for (int i = 0; i < nb; ++i) {
             const double d = h[3 * i + 1] * h[3 * i + 2];
@@ -1030,13 +1147,15 @@ int t2b_update_ssnr(t2b_ctx* c, int iclass, const t2b_ssnr_config* cf, double* t
         T2B_REQUIRE(v.r_max < nb && nb <= 1024, T2B_ERR_ARG, "r_max exceeds ori_size / 2 (or ori_size too large)");
         const double oc = v.ref_dim == 3 ? (double)v.pad * v.pad * v.pad : (double)v.pad * v.pad;
         cudaStream_t st = c->stream;
-        DevBuf<double> acc(3 * (size_t)nb), t2d(nb), actf(nb);
-        const long long nvox = (long long)v.zdim * v.ydim * v.xdim;
+        Scratch sc(c, Scratch::size<double>(3 * (size_t)nb) + Scratch::size<double>(nb));
+        double* acc = sc.take<double>(3 * (size_t)nb);
+        double* t2d = sc.take<double>(nb);
+        const long long items = (long long)v.zdim * v.ydim * ((v.xdim + RUN - 1) / RUN);
         // pass 1: sigma2 = count / sum(pad^3 weight) per shell (src/backprojector.cpp:1058-1088)
-        T2B_CUDA(cudaMemsetAsync(acc.p, 0, 3 * (size_t)nb * sizeof(double), st));
-        k_ssnr_sigma<<<grid_of(nvox), RC_THREADS, 2 * nb * sizeof(double), st>>>(v, nb, c->gweight[iclass], oc, acc.p);
+        T2B_CUDA(cudaMemsetAsync(acc, 0, 3 * (size_t)nb * sizeof(double), st));
+        k_ssnr_sigma<<<grid_of(items), RC_THREADS, 2 * nb * sizeof(double), st>>>(v, nb, c->gweight[iclass], oc, acc);
         std::vector<double> h(3 * (size_t)nb);
-        T2B_CUDA(cudaMemcpyAsync(h.data(), acc.p, 2 * (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, st));
+        T2B_CUDA(cudaMemcpyAsync(h.data(), acc, 2 * (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, st));
         T2B_CUDA(cudaStreamSynchronize(st));
         std::vector<double> s2(nb), t(tau2, tau2 + nb), dvp(nb, 0.), cov(nb, 0.);
         for (int i = 0; i < nb; ++i) {
@@ -1054,15 +1173,16 @@ int t2b_update_ssnr(t2b_ctx* c, int iclass, const t2b_ssnr_config* cf, double* t
                 dvp[i] = ssnr;
             }
         // pass 2: data vs prior and Fourier coverage (:1127-1190)
-        T2B_CUDA(cudaMemcpyAsync(t2d.p, t.data(), nb * sizeof(double), cudaMemcpyHostToDevice, st));
-        if (cf->correct_tau2_by_avgctf2)
-            T2B_CUDA(cudaMemcpyAsync(actf.p, cf->avgctf2, nb * sizeof(double), cudaMemcpyHostToDevice, st));
-        T2B_CUDA(cudaMemsetAsync(acc.p, 0, 3 * (size_t)nb * sizeof(double), st));
-        k_ssnr_prior<<<grid_of(nvox), RC_THREADS, 3 * nb * sizeof(double), st>>>(v, nb, c->gweight[iclass], oc,
-                                                                                  cf->tau2_fudge, t2d.p, actf.p,
-                                                                                  cf->correct_tau2_by_avgctf2, acc.p);
+        std::vector<double> it(nb);
+        for (int i = 0; i < nb; ++i) {
+            it[i] = t[i] > 0. ? 1. / (oc * cf->tau2_fudge * t[i]) : -1.;
+            if (t[i] > 0. && cf->correct_tau2_by_avgctf2 && cf->avgctf2[i] > 0.) it[i] *= 1. / cf->avgctf2[i];
+        }
+        T2B_CUDA(cudaMemcpyAsync(t2d, it.data(), nb * sizeof(double), cudaMemcpyHostToDevice, st));
+        T2B_CUDA(cudaMemsetAsync(acc, 0, 3 * (size_t)nb * sizeof(double), st));
+        k_ssnr_prior<<<grid_of(items), RC_THREADS, 3 * nb * sizeof(double), st>>>(v, nb, c->gweight[iclass], t2d, acc);
         T2B_CUDA(cudaGetLastError());
-        T2B_CUDA(cudaMemcpyAsync(h.data(), acc.p, 3 * (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, st));
+        T2B_CUDA(cudaMemcpyAsync(h.data(), acc, 3 * (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, st));
         T2B_CUDA(cudaStreamSynchronize(st));
         for (int i = 0; i < nb; ++i) {
             const double ratio = h[3 * i], ncov = h[3 * i + 1], cn = h[3 * i + 2];

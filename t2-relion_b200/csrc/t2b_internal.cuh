@@ -204,13 +204,10 @@ void launch_fine(const Tables& tb, const Work& w, cudaStream_t st);
 void launch_weights_fine(const Tables& tb, const Work& w, cudaStream_t st);
 void launch_wsum_bp(const Tables& tb, const Work& w, const Volume& g, float2* const* grid_data,
                     float* const* grid_weight, cudaStream_t st);
-void launch_reconstruct(const Volume& g, const float2* data, const float* weight, double2* fconv,
-                        double* fw, double* rad, double* cnt, cudaStream_t st, const double* tau2 = nullptr,
-                        double tscale = 1., int minres_map = 0);
-// Projector::decenter of a grid with the MAP term (the first step of launch_reconstruct,
-// without its division): the gridding iterations' input
-void launch_decenter(const Volume& g, const float2* data, const float* weight, double2* fconv, double* fw,
-                     double* rad, double* cnt, cudaStream_t st, const double* tau2, double tscale, int minres_map);
+void launch_radial(const Volume& g, const float* weight, double* rad, double* acc, cudaStream_t st,
+                   const double* inv_tau2 = nullptr, int minres_map = 0);
+void launch_reconstruct(const Volume& g, const float2* data, const float* weight, double2* fconv, double* rad,
+                        double* acc, cudaStream_t st);
 
 // tcgen05 split-BF16 coarse diff2 (diff2_tc.cu)
 struct TcOperands {
@@ -303,8 +300,8 @@ struct t2b_ctx {
     std::vector<t2b::Volume> gvol;            // per class BP grid geometry
     std::vector<float2*> gdata;               // per class grid data
     std::vector<float*> gweight;              // per class grid weight
-    void* sym_scratch = nullptr;              // symmetrisation sums of one grid (grown on demand)
-    size_t sym_bytes = 0;
+    void* ms_scratch = nullptr;               // M-step scratch, grown on demand (Scratch, recon.cu)
+    size_t ms_bytes = 0;
     bool configured = false;
     t2b_config cfg{};
     t2b::Tables tb{};
@@ -351,6 +348,15 @@ struct t2b_ctx {
     {
         for (cudaStream_t s : {copy_stream, stream, aux_stream, d2h_stream})
             if (s) T2B_CUDA(cudaStreamSynchronize(s));
+    }
+    // Give the M-step scratch back: before anything that takes device memory for good
+    void release_scratch()
+    {
+        if (!ms_scratch) return;
+        T2B_CUDA(cudaStreamSynchronize(stream));
+        cudaFree(ms_scratch);
+        ms_scratch = nullptr;
+        ms_bytes = 0;
     }
     long long submitted = 0;                  // host batches submitted: the next ticket
     bool stage_timing = false;                // host batches run uncaptured with stage events

@@ -302,3 +302,27 @@ def test_gridding_on_odd_boxes_from_a_written_grid(t2b, r_max):
     ref = ro.reconstruct_map(data.astype(np.complex128), w.astype(np.float64), r_max, 2, ori, gridding_iter=2,
                              normalise=3.0)
     _map_close(got, ref)
+
+
+@pytest.mark.parametrize("r_max,ori", [(8, 16), (24, 48), (53, 108), (58, 120)],
+                         ids=["pad35_5x7", "pad99_9x11", "pad215_5x43", "pad235_5x47"])
+def test_gridding_transform_plans(t2b, r_max, ori):
+    """The half-box transforms where their plans change: 35 (radix 7 in registers, no prime table), 99 (the
+    smallest prime first stage, 32 lines a block), 215 and 235 (the last prime with a full table and
+    the first without, 16 lines), on a seeded grid, against the oracle."""
+    import torch
+    import t2relion_b200.parallel as par
+    ps = 2 * (2 * r_max + 1) + 1
+    rng = np.random.default_rng(r_max)
+    shape = (ps, ps, ps // 2 + 1)
+    data = (rng.normal(size=shape) + 1j * rng.normal(size=shape)).astype(np.complex64)
+    w = rng.uniform(0.5, 2.0, size=shape).astype(np.float32)
+    es = t2b.EStep(0)
+    es.init_backprojector(0, 3, ps, r_max, 2)
+    for ptr, src in zip(es.backprojector_device_ptrs(0), (data.view(np.float32), w)):
+        par.device_view(ptr, src.size, 0).copy_(torch.from_numpy(np.ascontiguousarray(src).reshape(-1)))
+    torch.cuda.synchronize()
+    got = es.reconstruct(0, ori, gridding_iter=2, normalise=3.0)
+    es.close()
+    _map_close(got, ro.reconstruct_map(data.astype(np.complex128), w.astype(np.float64), r_max, 2, ori, gridding_iter=2,
+                                       normalise=3.0))
