@@ -254,9 +254,11 @@ __device__ __forceinline__ void fft_stage_gen(const float2* a, float2* b, int nf
 // f + nfft / 2; nfft even), so the two loads of an r serve PF_U pairs and each (cos, sin) entry two
 // sequences; u is the slowest index, so the lanes of a warp share their u and the entries come as
 // broadcast 16-byte reads: from `tab`, [r - 1][u - 1], when it is full (R <= PF_TAB_MAX), else entry
-// (u r mod R) of R entries.  The sums are FP64 (the FP64 units are otherwise idle, and an FP64 pair is
-// the width of the reads already): the half-box transforms of the gridding iterations lose the
-// averaging over both halves that the full box had, and this stage is the one with long sums.
+// (u r mod R) of R entries.  The sums are FP64 (an FP64 pair is the width of the reads already): the
+// half-box transforms of the gridding iterations lose the averaging over both halves that the full
+// box had, and this stage is the one with long sums.  At 259 (7 x 37) a gridding iteration took 0.64 ms
+// with FP32 sums and takes 0.88, for results nearer to 64-bit arithmetic than the full box's (2.5e-7
+// against 5.3e-7).
 constexpr int PF_U = 5;
 constexpr int PF_TAB_MAX = 43;
 

@@ -371,9 +371,10 @@ __global__ void k_hermitian(Volume g, float2* __restrict__ data, float* __restri
 // transforms along z and y of the half, then rows in pairs, complex to real, times the blob's
 // tabulated Fourier transform over its value at 0 and back to the half while they are in shared
 // memory, then y and z forward, the last of them updating w_n.
-// At 259 an iteration took 0.64 ms (was 2.05: six passes over the full box and three over the grid
+// At 259 an iteration takes 0.88 ms (was 2.05: six passes over the full box and three over the grid
 // between them) and moves 0.84 GB (0.13 ms at the copy bandwidth): bound by the prime-length stage
-// (fft_stage_prime_first), two blocks a SM.
+// (fft_stage_prime_first).  Two blocks a SM, by the launch bounds: at the 140 registers that the stage's
+// FP64 sums would take, and one block, an iteration took 1.45 ms.
 constexpr int GD_COL = 0, GD_LOAD = 1, GD_UPDATE = 2;   // k_gd_col: V -> V, w_n weight -> V, V -> w_n
 
 // lines (sequences) per CTA: two buffers of them in about 70 KB, and enough work for 256 threads
@@ -412,7 +413,7 @@ __global__ void k_gd_blob(const double* __restrict__ ratio, int ntab, double ori
 // row y = blockIdx.x); x tile blockIdx.y.  IO: GD_LOAD takes (float)(w_n weight) instead of V,
 // GD_UPDATE divides w_n by max(1e-6, |result| inv_n) inside r^2 < max_r2 instead of storing V.
 template <bool INV, int IO, int NL>
-__global__ void __launch_bounds__(RC_THREADS) k_gd_col(float2* __restrict__ V, double* __restrict__ fn,
+__global__ void __launch_bounds__(RC_THREADS, 2) k_gd_col(float2* __restrict__ V, double* __restrict__ fn,
                                                        const double* __restrict__ fw, int N, int axis,
                                                        const float2* __restrict__ tw, FftPlan plan, int ntable,
                                                        int max_r2, double inv_n)
@@ -466,7 +467,7 @@ __global__ void __launch_bounds__(RC_THREADS) k_gd_col(float2* __restrict__ V, d
 // part of one complex sequence): inverse transform to real space, times the blob factor
 // (FP64 product, rounded once), forward transform, separated again.  NL pairs per CTA.
 template <int NL>
-__global__ void __launch_bounds__(RC_THREADS) k_gd_rows(float2* __restrict__ V, int N, int nz,
+__global__ void __launch_bounds__(RC_THREADS, 2) k_gd_rows(float2* __restrict__ V, int N, int nz,
                                                         const double* __restrict__ blob, const float2* __restrict__ tw,
                                                         FftPlan plan, int ntable)
 {
