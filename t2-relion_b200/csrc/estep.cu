@@ -103,57 +103,81 @@ __global__ void k_prep(Tables tb, Work w)
 }
 
 // ----------------------------------------------------------------- norms
-// N[b][oc] = sum_p w2[b][p] |P_oc[p]|^2 ; tile 128 orientations x 64 particles,
-// 4 x 8 outputs per thread, 16 pixels per shared-memory stage.
+// N[b][oc] = sum_p w2[b][p] |P_oc[p]|^2 ; tile 64 orientations x BN particles, 16 pixels per
+// shared-memory stage, the next stage's values in registers meanwhile.  Bound by the loads of the projection
+// table, once for each BN particles (323 MB for 18,432 orientations of 2,190 pixels: 49 us).  A tile
+// of 128 x 64 without the overlap took 682 us for 37 particles there, this one 270, and for one particle
+// at 9,216 x 797 71 us against 19.
+constexpr int NM_M = 64, NM_KP = 16;
+template <int BN>   // 8: 2 x 1 outputs per thread, 32: 4 x 2, 64: 4 x 4
 __global__ void __launch_bounds__(256) k_norms(Tables tb, Work w, const float2* __restrict__ proj, int nrows,
                                                float* __restrict__ out)
 {
-    __shared__ __align__(16) float Ps[16][132];
-    __shared__ __align__(16) float Ws[16][68];
-    const int o0 = blockIdx.x * 128, b0 = blockIdx.y * 64, P = tb.P;
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;  // 8 particle groups x 32 orientation groups
-    float acc[4][8];
+    constexpr int TR = BN == 8 ? 2 : 4, TC = BN * NM_M / (256 * TR);   // outputs of a thread
+    constexpr int CG = BN / TC;                                         // column groups
+    constexpr int LB = NM_M * NM_KP / 256, LW = (BN * NM_KP + 255) / 256;
+    static_assert(TC >= 1 && (NM_M / TR) * CG == 256, "256 threads");
+    __shared__ __align__(16) float Ps[2][NM_KP][NM_M + 4];
+    __shared__ __align__(16) float Ws[2][NM_KP][BN + 4];
+    const int o0 = blockIdx.x * NM_M, b0 = blockIdx.y * BN, P = tb.P, nk = tb.nk;
+    const int tx = threadIdx.x % CG, ty = threadIdx.x / CG;
+    const int lp = threadIdx.x % NM_KP, lr = threadIdx.x / NM_KP;
+    float2 rp[LB];
+    float rw[LW];
+    const auto load = [&](int p0) {
+        const bool in = p0 + lp < nk;
+        const int p = in ? tb.kpix[p0 + lp] : 0;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-    const int nk = tb.nk;
-    for (int p0 = 0; p0 < nk; p0 += 16) {
-        for (int idx = threadIdx.x; idx < 128 * 16; idx += 256) {
-            const int oo = idx >> 4, pp = idx & 15;
-            float v = 0.f;
-            if (o0 + oo < nrows && p0 + pp < nk) {
-                const float2 z = proj[(size_t)(o0 + oo) * P + tb.kpix[p0 + pp]];
-                v = z.x * z.x + z.y * z.y;
-            }
-            Ps[pp][oo] = v;
+        for (int i = 0; i < LB; i++) {
+            const int o = o0 + lr + 16 * i;
+            rp[i] = in && o < nrows ? proj[(size_t)o * P + p] : make_float2(0.f, 0.f);
         }
-        for (int idx = threadIdx.x; idx < 64 * 16; idx += 256) {
-            const int bb = idx >> 4, pp = idx & 15;
-            Ws[pp][bb] = (b0 + bb < w.n && p0 + pp < nk) ? w.w2[(size_t)(b0 + bb) * P + tb.kpix[p0 + pp]] : 0.f;
+#pragma unroll
+        for (int i = 0; i < LW; i++) {
+            const int b = lr + 16 * i;
+            rw[i] = in && b < BN && b0 + b < w.n ? w.w2[(size_t)(b0 + b) * P + p] : 0.f;
         }
-        __syncthreads();
+    };
+    const auto store = [&](int buf) {
 #pragma unroll
-        for (int pp = 0; pp < 16; pp++) {
-            const float4 pv = *reinterpret_cast<const float4*>(&Ps[pp][ty * 4]);
-            const float4 w0 = *reinterpret_cast<const float4*>(&Ws[pp][tx * 8]);
-            const float4 w1 = *reinterpret_cast<const float4*>(&Ws[pp][tx * 8 + 4]);
-            const float a[4] = {pv.x, pv.y, pv.z, pv.w};
-            const float c[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        for (int i = 0; i < LB; i++) Ps[buf][lp][lr + 16 * i] = rp[i].x * rp[i].x + rp[i].y * rp[i].y;
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+        for (int i = 0; i < LW; i++)
+            if (lr + 16 * i < BN) Ws[buf][lp][lr + 16 * i] = rw[i];
+    };
+    float acc[TR][TC] = {};
+    load(0);
+    store(0);
+    __syncthreads();
+    int buf = 0;
+    for (int p0 = 0; p0 < nk; p0 += NM_KP) {
+        const bool more = p0 + NM_KP < nk;
+        if (more) load(p0 + NM_KP);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i], c[j], acc[i][j]);
+        for (int k = 0; k < NM_KP; k++) {
+            float a[TR], c[TC];
+#pragma unroll
+            for (int i = 0; i < TR; i++) a[i] = Ps[buf][k][ty * TR + i];
+#pragma unroll
+            for (int j = 0; j < TC; j++) c[j] = Ws[buf][k][tx * TC + j];
+#pragma unroll
+            for (int i = 0; i < TR; i++)
+#pragma unroll
+                for (int j = 0; j < TC; j++) acc[i][j] = fmaf(a[i], c[j], acc[i][j]);
         }
-        __syncthreads();
+        if (more) {
+            store(buf ^ 1);
+            __syncthreads();
+            buf ^= 1;
+        }
     }
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int bb = b0 + tx * 8 + j;
+    for (int j = 0; j < TC; j++) {
+        const int bb = b0 + tx * TC + j;
         if (bb >= w.n) continue;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int o = o0 + ty * 4 + i;
+        for (int i = 0; i < TR; i++) {
+            const int o = o0 + ty * TR + i;
             if (o < nrows) out[(size_t)bb * nrows + o] = acc[i][j];
         }
     }
@@ -162,38 +186,49 @@ __global__ void __launch_bounds__(256) k_norms(Tables tb, Work w, const float2* 
 // --------------------------------------------------- plain FP32 diff2 GEMM
 // C[oc][col] = sum_k Bm[oc][k] A[col][k], k over interleaved (re, im) of the P
 // pixels, col = b*T + t.  A is built on the fly from cvec and the phase table.
-// 128 x 128 tile, 256 threads, 8x8 register micro-tile, double-buffered smem.
-constexpr int SB_M = 128, SB_N = 128, SB_KP = 8, SB_K = 16, SB_LD = 132;
-
-__global__ void __launch_bounds__(256, 2) k_diff2_simt(Tables tb, Work w)
+// BM x BN tile, TR x TC outputs per thread, double-buffered shared memory.  Bound by FP32 issue: the
+// multiply-adds are packed in pairs of columns (fma.rn.f32x2, each half rounded as a scalar one), which
+// this chip needs for its FP32 rate.  18,432 orientations x 1,813 columns x K = 4,380 took 8.73 ms with
+// scalar ones (36 TFLOP/s), 7.05 with these (42), the same sums in the same order.
+template <int BM, int BN, int KP, int TR, int TC>
+__global__ void __launch_bounds__((BM / TR) * (BN / TC), TR == 8 ? 2 : 4) k_diff2_simt(Tables tb, Work w)
 {
-    __shared__ __align__(16) float Bs[2][SB_K][SB_LD];
-    __shared__ __align__(16) float As[2][SB_K][SB_LD];
-    __shared__ unsigned smin[SB_N + 2];
+    constexpr int NT = (BM / TR) * (BN / TC), K = 2 * KP, ROWS = NT / KP;   // rows of one loader pass
+    constexpr int LB = BM / ROWS, LA = BN / ROWS;
+    constexpr int RH = TR / 4, CH = TC / 4;      // groups of four rows / columns of a thread, BM / RH and BN / CH apart
+    __shared__ __align__(16) float Bs[2][K][BM + 4];
+    __shared__ __align__(16) float As[2][K][BN + 4];
+    __shared__ unsigned smin[BN + 2];
     const int P = tb.P, T = tb.T, KO = tb.K * tb.O;
-    const int m0 = blockIdx.x * SB_M, n0 = blockIdx.y * SB_N;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
     const int ncols = w.n * T;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // a warp covers 4 x 8 threads, so that its reads of either operand touch one line each
+    constexpr int WC = BN / TC / 8;   // warps along the columns
+    const int tx = (warp % WC) * 8 + (lane & 7), ty = (warp / WC) * 4 + (lane >> 3);
     const int bfirst = n0 / T;
 
-    // loader coordinates: thread loads rows/cols (tid>>3) + 32*j, pixel (tid & 7)
-    const int lrow = tid >> 3, lp = tid & 7;
-    int la_b[4], la_t[4];
+    // loader coordinates: rows/cols (tid / KP) + ROWS * j, pixel tid % KP
+    const int lrow = tid / KP, lp = tid % KP;
+    int la_b[LA], la_t[LA];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int col = n0 + lrow + 32 * j;
+    for (int j = 0; j < LA; j++) {
+        const int col = n0 + lrow + ROWS * j;
         la_b[j] = col < ncols ? col / T : -1;
         la_t[j] = col < ncols ? col - (col / T) * T : 0;
     }
-    float2 rb[4], ra[4];
+    float2 rb[LB], ra[LA];
     const int nk = tb.nk;
     auto gload = [&](int p0) {
         const bool in = p0 + lp < nk;
         const int p = in ? tb.kpix[p0 + lp] : 0;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int row = m0 + lrow + 32 * j;
+        for (int j = 0; j < LB; j++) {
+            const int row = m0 + lrow + ROWS * j;
             rb[j] = (row < KO && in) ? tb.proj_c[(size_t)row * P + p] : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int j = 0; j < LA; j++) {
             if (la_b[j] >= 0 && in) {
                 const float2 c = w.cvec[(size_t)la_b[j] * P + p];
                 const float2 ab = tb.ab_c[(size_t)la_t[j] * P + p];
@@ -205,39 +240,46 @@ __global__ void __launch_bounds__(256, 2) k_diff2_simt(Tables tb, Work w)
     };
     auto sstore = [&](int buf) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            Bs[buf][2 * lp][lrow + 32 * j] = rb[j].x;
-            Bs[buf][2 * lp + 1][lrow + 32 * j] = rb[j].y;
-            As[buf][2 * lp][lrow + 32 * j] = ra[j].x;
-            As[buf][2 * lp + 1][lrow + 32 * j] = ra[j].y;
+        for (int j = 0; j < LB; j++) {
+            Bs[buf][2 * lp][lrow + ROWS * j] = rb[j].x;
+            Bs[buf][2 * lp + 1][lrow + ROWS * j] = rb[j].y;
+        }
+#pragma unroll
+        for (int j = 0; j < LA; j++) {
+            As[buf][2 * lp][lrow + ROWS * j] = ra[j].x;
+            As[buf][2 * lp + 1][lrow + ROWS * j] = ra[j].y;
         }
     };
-    float acc[8][8];
+    float2 acc[TR][TC / 2];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < TR; i++)
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-    for (int i = tid; i < SB_N + 2; i += 256) smin[i] = 0xffffffffu;
+        for (int j = 0; j < TC / 2; j++) acc[i][j] = make_float2(0.f, 0.f);
+    for (int i = tid; i < BN + 2; i += NT) smin[i] = 0xffffffffu;
 
     gload(0);
     sstore(0);
     __syncthreads();
     int buf = 0;
-    for (int p0 = 0; p0 < nk; p0 += SB_KP) {
-        const bool more = p0 + SB_KP < nk;
-        if (more) gload(p0 + SB_KP);
+    for (int p0 = 0; p0 < nk; p0 += KP) {
+        const bool more = p0 + KP < nk;
+        if (more) gload(p0 + KP);
 #pragma unroll
-        for (int k = 0; k < SB_K; k++) {
-            const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][k][ty * 4]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][k][64 + ty * 4]);
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][k][tx * 4]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][k][64 + tx * 4]);
-            const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        for (int k = 0; k < K; k++) {
+            float bv[TR];
+            float2 av[TC / 2];
 #pragma unroll
-            for (int i = 0; i < 8; i++)
+            for (int h = 0; h < RH; h++)
+                *reinterpret_cast<float4*>(&bv[4 * h]) = *reinterpret_cast<const float4*>(&Bs[buf][k][h * (BM / RH) + ty * 4]);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(bv[i], av[j], acc[i][j]);
+            for (int h = 0; h < CH; h++)
+                *reinterpret_cast<float4*>(&av[2 * h]) = *reinterpret_cast<const float4*>(&As[buf][k][h * (BN / CH) + tx * 4]);
+#pragma unroll
+            for (int i = 0; i < TR; i++) {
+                const float2 bb = make_float2(bv[i], bv[i]);
+#pragma unroll
+                for (int j = 0; j < TC / 2; j++) acc[i][j] = __ffma2_rn(bb, av[j], acc[i][j]);
+            }
         }
         if (more) {
             sstore(buf ^ 1);
@@ -247,28 +289,28 @@ __global__ void __launch_bounds__(256, 2) k_diff2_simt(Tables tb, Work w)
     }
     // epilogue
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int oc = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
+    for (int i = 0; i < TR; i++) {
+        const int oc = m0 + (i >> 2) * (BM / RH) + ty * 4 + (i & 3);
         if (oc >= KO) continue;
         const bool skip = tb.skip[oc] != 0;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int col = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
+        for (int j = 0; j < TC; j++) {
+            const int col = n0 + (j >> 2) * (BN / CH) + tx * 4 + (j & 3);
             if (col >= ncols) continue;
             const int b = col / T, t = col - b * T;
             float d;
             if (skip) {
                 d = -999.f;
             } else {
-                d = w.c0[b] + w.norms[(size_t)b * KO + oc] - acc[i][j];
+                d = w.c0[b] + w.norms[(size_t)b * KO + oc] - (j & 1 ? acc[i][j >> 1].y : acc[i][j >> 1].x);
                 atomicMin(&smin[b - bfirst], f2key(d));
             }
             w.d2c[((size_t)b * KO + oc) * T + t] = d;
         }
     }
     __syncthreads();
-    const int nb = min(SB_N / T + 2, SB_N + 2);
-    for (int i = tid; i < nb; i += 256) {
+    const int nb = min(BN / T + 2, BN + 2);
+    for (int i = tid; i < nb; i += NT) {
         const int b = bfirst + i;
         if (b < w.n && smin[i] != 0xffffffffu) atomicMin(&w.minkey_c[b], smin[i]);
     }
@@ -1908,17 +1950,22 @@ void launch_prep(const Tables& tb, const Work& w, cudaStream_t st)
 
 void launch_norms(const Tables& tb, const Work& w, cudaStream_t st)
 {
-    const int KO = tb.K * tb.O;
-    dim3 grid((KO + 127) / 128, (w.n + 63) / 64);
-    k_norms<<<grid, 256, 0, st>>>(tb, w, tb.proj_c, KO, w.norms);
+    const int KO = tb.K * tb.O, mt = (KO + NM_M - 1) / NM_M;
+    // the widest tile that the batch fills: the table is read once for each of its particles
+    if (w.n <= 8) k_norms<8><<<dim3(mt, 1), 256, 0, st>>>(tb, w, tb.proj_c, KO, w.norms);
+    else if (w.n <= 32) k_norms<32><<<dim3(mt, 1), 256, 0, st>>>(tb, w, tb.proj_c, KO, w.norms);
+    else k_norms<64><<<dim3(mt, (w.n + 63) / 64), 256, 0, st>>>(tb, w, tb.proj_c, KO, w.norms);
     T2B_CUDA(cudaGetLastError());
 }
 
 void launch_diff2_simt(const Tables& tb, const Work& w, cudaStream_t st)
 {
-    const int KO = tb.K * tb.O;
-    dim3 grid((KO + SB_M - 1) / SB_M, (w.n * tb.T + SB_N - 1) / SB_N);
-    k_diff2_simt<<<grid, 256, 0, st>>>(tb, w);
+    const int KO = tb.K * tb.O, cols = w.n * tb.T;
+    const dim3 big((KO + 127) / 128, (cols + 127) / 128);
+    // two 128 x 128 tiles run on an SM; where they would leave SMs idle (one particle of 29 shifts against
+    // 9,216 orientations: 72 tiles, a quarter of their columns used, 136 us), tiles of 64 x 32 (49 us)
+    if ((long long)big.x * big.y >= 2LL * sm_count()) k_diff2_simt<128, 128, 8, 8, 8><<<big, 256, 0, st>>>(tb, w);
+    else k_diff2_simt<64, 32, 16, 4, 4><<<dim3((KO + 63) / 64, (cols + 31) / 32), 128, 0, st>>>(tb, w);
     T2B_CUDA(cudaGetLastError());
 }
 

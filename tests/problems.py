@@ -24,10 +24,12 @@ def build(name, n_particles=16, seed=7, nr_classes=1, diff2_mode=0, max_batch=No
         "learn_o2_lowsnr": dict(N=64, angpix=2.0, order=2, psi=7.5, rng=3, r=16, snr=0.03, ovs=1),
         # 2D classification: 2D references, psi 6 deg, oversampling 1
         "class2d": dict(N=48, angpix=2.0, order=0, psi=6.0, rng=3, r=12, snr=0.2, ovs=1),
+        # 997 in-plane angles x 29 shifts: hypotheses in no multiple of 4, orientations of no tile
+        "class2d_odd": dict(N=48, angpix=2.0, order=0, psi=360. / 997, rng=3, r=12, snr=0.05, ovs=0),
     }
     p = presets[name]
     N, r, s = p["N"], p["r"], 2 * p["r"]
-    ref_dim = 2 if name == "class2d" else 3
+    ref_dim = 2 if name.startswith("class2d") else 3
     maps = []
     for k in range(nr_classes):
         vol = sy.blob_volume(N, 40 if ref_dim == 3 else 12, seed=seed + 101 * k, ndim=ref_dim)
