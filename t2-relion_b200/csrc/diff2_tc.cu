@@ -22,9 +22,8 @@
 // T2B_ERR_TIMEOUT in a device flag, waits (bounded) for its own copies and
 // MMAs, frees TMEM and returns.
 #include "t2b_internal.cuh"
+#include "tc_ptx.cuh"
 #include "project_pixel.cuh"
-#include <cuda.h>
-#include <cuda_bf16.h>
 #include <algorithm>
 #include <cstring>
 
@@ -45,122 +44,11 @@ constexpr int NTHREADS = 192;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr int EPI_LD = 33;
 constexpr size_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 4 * 32 * EPI_LD * 4 + 4 * (TN + 2) * 4;
-constexpr unsigned long long WAIT_NS = 2000000000ull;
 
 // instruction descriptor: D f32, A/B bf16, both K-major, M = 128; N (bits 17-22, N/8)
 // is set per launch (256, or 96 for one particle's translations)
 constexpr uint32_t IDESC_BASE = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
 __host__ __device__ constexpr uint32_t idesc_for(int n) { return IDESC_BASE | ((uint32_t)(n >> 3) << 17); }
-
-__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ unsigned long long gtimer()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t n)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(b)), "r"(n));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* b)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(su32(b)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait for the phase of parity `parity`; false on timeout / abort.
-__device__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag)
-{
-    const unsigned long long t0 = gtimer();
-    for (uint32_t i = 1;; i++) {
-        if (mbar_try(b, parity)) return true;
-        if ((i & 255u) == 0) {
-            if (*abort_flag) return false;
-            if (gtimer() - t0 > WAIT_NS) return false;
-        }
-    }
-}
-
-__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-            su32(dst)),
-        "l"(map), "r"(su32(bar)), "r"(x), "r"(y)
-        : "memory");
-}
-
-// Bring one box of a tensor map into L2 ahead of its load (no shared memory, no barrier).
-__device__ __forceinline__ void tma_prefetch_l2(const CUtensorMap* map, int x, int y)
-{
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y)
-                 : "memory");
-}
-
-// One contiguous block global -> shared (untiled bulk copy): the operand is stored
-// pre-swizzled, so the block lands in the layout the UMMA descriptor reads
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     su32(dst)),
-                 "l"(src), "r"(bytes), "r"(su32(bar))
-                 : "memory");
-}
-
-// UMMA shared-memory descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)1 << 16;             // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;   // stride byte offset
-    d |= (uint64_t)1 << 46;             // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;             // SWIZZLE_128B
-    return d;
-}
-
-__device__ __forceinline__ void umma(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum)
-{
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-            dtmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(accum));
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r)
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 __device__ __forceinline__ unsigned f2key(float f)
 {
@@ -718,38 +606,6 @@ __global__ void k_split_w2(const float* __restrict__ w2, int n, int P, const int
         const float v = (r < n && kk < nk) ? w2[r * P + kpix[kk]] : 0.f;
         split_bf16(v, hi[i], lo[i]);
     }
-}
-
-using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeFn encoder()
-{
-    static EncodeFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess || !p)
-            throw Error{T2B_ERR_CUDA, "cuTensorMapEncodeTiled unavailable"};
-        fn = reinterpret_cast<EncodeFn>(p);
-    }
-    return fn;
-}
-
-CUtensorMap make_map(void* ptr, int rows, int kdim, int box_rows)
-{
-    CUtensorMap m;
-    const cuuint64_t dims[2] = {(cuuint64_t)kdim, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)kdim * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)TK, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, dims, strides, box, estr,
-                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) throw Error{T2B_ERR_CUDA, "cuTensorMapEncodeTiled failed"};
-    return m;
 }
 
 int sms()

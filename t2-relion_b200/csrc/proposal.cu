@@ -18,13 +18,14 @@
 //   fc1, fc2  2048 -> 1024 -> 1024, ReLU
 //   fc3       1024 -> K*O logits
 // Inference runs fc1..fc3 on the tcgen05 kernel (one BF16 product); training
-// runs every layer through the SIMT kernels below, forward and backward, with
-// Adam, on particles generated here from the current references (projection,
+// runs them on the tensor cores too, with FP32 activations and gradients split into
+// BF16 parts (train_gemm.cu) and Adam in the gradients' epilogue, the convolutions in FP32 below, on particles generated here from the current references (projection,
 // CTF, shift, noise) and labelled with their true orientation and with the
 // posterior of the plain E-step run on them.
 #include "t2b_internal.cuh"
 #include "project_pixel.cuh"
 #include "proposal.cuh"
+#include "train_gemm.cuh"
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cmath>
@@ -67,25 +68,6 @@ __device__ T bsum(T v, T* sh /* >= 32 */)
     if (threadIdx.x == 0) sh[0] = v;
     __syncthreads();
     const T r = sh[0];
-    __syncthreads();
-    return r;
-}
-
-__device__ __forceinline__ float bmax(float v, float* sh)
-{
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    const int nw = (blockDim.x + 31) >> 5;
-    v = (threadIdx.x < nw) ? sh[threadIdx.x] : -INFINITY;
-    if (wid == 0)
-        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __syncthreads();
-    if (threadIdx.x == 0) sh[0] = v;
-    __syncthreads();
-    const float r = sh[0];
     __syncthreads();
     return r;
 }
@@ -1001,236 +983,450 @@ __global__ void __launch_bounds__(256) k_capture(const double* __restrict__ marg
 }
 
 // ----------------------------------------------------------- training
-// C[m][n] (+)= sum_k A(m,k) B(k,n), A(m,k) = AT ? A[k*lda+m] : A[m*lda+k],
-// B(k,n) = BT ? B[n*ldb+k] : B[k*ldb+n]; 64 x 64 tiles, 4 x 4 per thread.
-// gridDim.z > 1 splits K (chunks of kchunk) and accumulates with atomics into
-// a zeroed C.
-template <bool AT, bool BT, typename TA, typename TB>
-__global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const TA* __restrict__ A, int lda,
-                                               const TB* __restrict__ B, int ldb, float* __restrict__ C, int ldc,
-                                               int kchunk)
-{
-    __shared__ __align__(16) float As[16][68];
-    __shared__ __align__(16) float Bs[16][68];
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    for (int k0 = kbeg; k0 < kend; k0 += 16) {
-        for (int e = 0; e < 4; e++) {
-            const int idx = threadIdx.x * 4 + e;
-            int mm, kk;
-            if (AT) { mm = idx & 63; kk = idx >> 6; } else { kk = idx & 15; mm = idx >> 4; }
-            const int m = m0 + mm, k = k0 + kk;
-            float v = 0.f;
-            if (m < M && k < kend) v = (float)(AT ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k]);
-            As[kk][mm] = v;
-            int nn, kb;
-            if (BT) { kb = idx & 15; nn = idx >> 4; } else { nn = idx & 63; kb = idx >> 6; }
-            const int n = n0 + nn, k2 = k0 + kb;
-            float u = 0.f;
-            if (n < N && k2 < kend) u = (float)(BT ? B[(size_t)n * ldb + k2] : B[(size_t)k2 * ldb + n]);
-            Bs[kb][nn] = u;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            const float4 a = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-            const float4 c = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-            const float av[4] = {a.x, a.y, a.z, a.w}, cv[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], cv[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) {
-            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m >= M || n >= N) continue;
-            if (gridDim.z > 1) atomicAdd(&C[(size_t)m * ldc + n], acc[i][j]);
-            else C[(size_t)m * ldc + n] = acc[i][j];
-        }
-}
-
 // Geometric target of a training particle: q(oc) proportional to
 // exp(-angle(A_oc, A)^2 / (2 sigma^2)) over the orientations of its class
 // (angle of the rotation between the coarse orientation and the true pose).
-__device__ __forceinline__ float geo_q(const double* __restrict__ eul_c, int O, const float* geo, int cls, int oc,
-                                       float inv2s2)
+__device__ __forceinline__ float geo_q(const float* E, const float* geo, float inv2s2)
 {
-    if (oc / O != cls) return 0.f;
-    const double* E = eul_c + 9 * (size_t)(oc - cls * O);
     float tr = 0.f;
-    for (int j = 0; j < 9; j++) tr += (float)E[j] * geo[j];
+#pragma unroll
+    for (int j = 0; j < 9; j++) tr += E[j] * geo[j];
     const float ang = acosf(fminf(1.f, fmaxf(-1.f, 0.5f * (tr - 1.f))));
     return expf(-ang * ang * inv2s2);
 }
 
-// Softmax cross-entropy against soft targets q = geo weight x normalised
-// geometric target (geo: per row A[9] and its weight; null = none) + sparse
-// (orientation, weight) pairs (NET_NTGT per row); the weights of a row sum to
-// 1.  Logits (+ bias) are replaced by dL/dlogit = (softmax - q)/nb.
-// Orientations with a zero prior are outside the softmax (gradient 0).
-__global__ void __launch_bounds__(1024) k_softmax_ce(float* __restrict__ y, const bf16* __restrict__ bias,
-                                                     const unsigned char* __restrict__ skip, int KO,
-                                                     const int* __restrict__ tgt_oc, const float* __restrict__ tgt_w,
-                                                     const float* __restrict__ geo, const int* __restrict__ gcls,
-                                                     const double* __restrict__ eul_c, int O, float inv2s2, int nb,
-                                                     double* loss)
+// the coarse Euler matrices in FP32, element-major (9 x O): neighbouring threads read neighbouring orientations
+__global__ void k_geo_table(const double* __restrict__ eul, int O, float* __restrict__ out)
 {
-    __shared__ float red[32];
-    __shared__ double redd[32];
-    const int b = blockIdx.x;
-    float* row = y + (size_t)b * KO;
-    const float* gb = geo ? geo + (size_t)b * 10 : nullptr;
-    const float gw = gb ? gb[9] : 0.f;
-    const int gc = geo ? gcls[b] : 0;
-    float mx = -INFINITY;
-    for (int i = threadIdx.x; i < KO; i += blockDim.x)
-        if (!skip[i]) mx = fmaxf(mx, row[i] + __bfloat162float(bias[i]));
-    mx = bmax(mx, red);
-    double se = 0.;
-    for (int i = threadIdx.x; i < KO; i += blockDim.x)
-        if (!skip[i]) se += exp((double)(row[i] + __bfloat162float(bias[i]) - mx));
-    se = bsum(se, redd);
-    const double lse = log(se);
-    double lq = 0.;
-    for (int j = threadIdx.x; j < NET_NTGT; j += blockDim.x) {
-        const int oc = tgt_oc[(size_t)b * NET_NTGT + j];
-        const float q = tgt_w[(size_t)b * NET_NTGT + j];
-        if (oc >= 0 && q > 0.f && !skip[oc]) lq += q * (lse - (double)(row[oc] + __bfloat162float(bias[oc]) - mx));
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 9 * O) out[(size_t)(i % 9) * O + i / 9] = (float)eul[i];
+}
+
+// Softmax cross-entropy against soft targets q = geo weight x normalised geometric target (geo: per row
+// A[9] and its weight; null = none) + sparse (orientation, weight) pairs (NET_NTGT per row); the
+// weights of a row sum to 1.  Orientations with a zero prior are outside the softmax (gradient 0).
+// Three kernels: sums of SM_ROWS rows over a chunk of columns, so an orientation's matrix and target
+// serve all of them; the rows' statistics and the loss; the gradient, written as the split operands of
+// the backward products (k_softmax_split).  Bound by FP64 exponentials; one block per row, which read
+// every orientation's FP64 matrix twice for each row, took 258 us a minibatch of 256 at 36,864.
+constexpr int SM_ROWS = 4, SM_COLS = 8, SM_THREADS = 256;
+constexpr int SM_CHUNK = SM_COLS * SM_THREADS;
+constexpr double GEO_LOSS = 1024.;
+struct SmPart {          // of one row and chunk
+    double se, gz, gy;   // sum exp(y - mx), sum q, sum q y
+    float mx;
+};
+struct SmRow {           // of one row
+    double lse;          // log of the sum of exp(y - mx)
+    float mx, gs;        // gs: geo weight / sum q (0: no geometric target)
+};
+
+__global__ void __launch_bounds__(SM_THREADS) k_softmax_stats(const float* __restrict__ y, const bf16* __restrict__ bias,
+                                                              const unsigned char* __restrict__ skip, int KO, int nb,
+                                                              const float* __restrict__ geo, const int* __restrict__ gcls,
+                                                              const float* __restrict__ eulf, int O, float inv2s2,
+                                                              SmPart* __restrict__ part)
+{
+    __shared__ float s_geo[SM_ROWS][10];
+    __shared__ int s_cls[SM_ROWS];
+    __shared__ float s_mx[SM_THREADS / 32][SM_ROWS];
+    __shared__ double s_sum[SM_THREADS / 32][SM_ROWS][3];
+    const int r0 = blockIdx.y * SM_ROWS, c0 = blockIdx.x * SM_CHUNK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < SM_ROWS * 10; i += SM_THREADS)
+        s_geo[i / 10][i % 10] = geo && r0 + i / 10 < nb ? geo[(size_t)(r0 + i / 10) * 10 + i % 10] : 0.f;
+    if (threadIdx.x < SM_ROWS) s_cls[threadIdx.x] = geo && r0 + threadIdx.x < nb ? gcls[r0 + threadIdx.x] : -1;
+    float v[SM_COLS][SM_ROWS];
+    bool on[SM_COLS];
+#pragma unroll
+    for (int i = 0; i < SM_COLS; i++) {
+        const int c = c0 + i * SM_THREADS + threadIdx.x;
+        on[i] = c < KO && !skip[c];
+        const float b = on[i] ? __bfloat162float(bias[c]) : 0.f;
+#pragma unroll
+        for (int r = 0; r < SM_ROWS; r++) v[i][r] = on[i] && r0 + r < nb ? y[(size_t)(r0 + r) * KO + c] + b : -INFINITY;
     }
-    double gz = 0., gl = 0.;
-    if (gw > 0.f) {
-        for (int i = threadIdx.x; i < KO; i += blockDim.x)
-            if (!skip[i]) {
-                const float q = geo_q(eul_c, O, gb, gc, i, inv2s2);
-                gz += q;
-                gl += q * (lse - (double)(row[i] + __bfloat162float(bias[i]) - mx));
+#pragma unroll
+    for (int r = 0; r < SM_ROWS; r++) {
+        float m = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < SM_COLS; i++) m = fmaxf(m, v[i][r]);
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) s_mx[warp][r] = m;
+    }
+    __syncthreads();
+    double se[SM_ROWS], gz[SM_ROWS], gy[SM_ROWS];
+    float mx[SM_ROWS];
+#pragma unroll
+    for (int r = 0; r < SM_ROWS; r++) {
+        se[r] = gz[r] = gy[r] = 0.;
+        float m = s_mx[0][r];
+        for (int w = 1; w < SM_THREADS / 32; w++) m = fmaxf(m, s_mx[w][r]);
+        mx[r] = m;
+    }
+#pragma unroll
+    for (int i = 0; i < SM_COLS; i++) {
+        if (!on[i]) continue;
+        const int c = c0 + i * SM_THREADS + threadIdx.x;
+        float E[9];
+        if (geo) {
+#pragma unroll
+            for (int j = 0; j < 9; j++) E[j] = eulf[(size_t)j * O + c % O];
+        }
+#pragma unroll
+        for (int r = 0; r < SM_ROWS; r++) {
+            if (r0 + r >= nb) break;
+            se[r] += exp((double)(v[i][r] - mx[r]));
+            if (geo && s_geo[r][9] > 0.f && c / O == s_cls[r]) {
+                const float q = geo_q(E, s_geo[r], inv2s2);
+                gz[r] += q;
+                gy[r] += q * (double)v[i][r];
             }
-        gz = bsum(gz, redd);
-        gl = bsum(gl, redd);
-        if (gz > 0.) lq += gw * gl / gz;
+        }
     }
-    lq = bsum(lq, redd);
-    if (threadIdx.x == 0) atomicAdd(loss, lq);
-    __syncthreads();
-    const float inv = 1.f / nb;
-    const float gs = (gw > 0.f && gz > 0.) ? (float)(gw / gz) : 0.f;
-    for (int i = threadIdx.x; i < KO; i += blockDim.x) {
-        float v = skip[i] ? 0.f : (float)exp((double)(row[i] + __bfloat162float(bias[i]) - mx) - lse);
-        if (gs > 0.f && !skip[i]) v -= gs * geo_q(eul_c, O, gb, gc, i, inv2s2);
-        row[i] = v * inv;
+#pragma unroll
+    for (int r = 0; r < SM_ROWS; r++) {
+        double a = se[r], b = gz[r], c = gy[r];
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+            c += __shfl_xor_sync(0xffffffffu, c, o);
+        }
+        if (lane == 0) {
+            s_sum[warp][r][0] = a;
+            s_sum[warp][r][1] = b;
+            s_sum[warp][r][2] = c;
+        }
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < NET_NTGT; j += blockDim.x) {
-        const int oc = tgt_oc[(size_t)b * NET_NTGT + j];
-        const float q = tgt_w[(size_t)b * NET_NTGT + j];
-        if (oc >= 0 && q > 0.f && !skip[oc]) atomicAdd(&row[oc], -q * inv);
+    if (threadIdx.x < SM_ROWS && r0 + threadIdx.x < nb) {
+        const int r = threadIdx.x;
+        SmPart p{};
+        float m = s_mx[0][r];
+        for (int w = 0; w < SM_THREADS / 32; w++) {
+            p.se += s_sum[w][r][0];
+            p.gz += s_sum[w][r][1];
+            p.gy += s_sum[w][r][2];
+            m = fmaxf(m, s_mx[w][r]);
+        }
+        p.mx = m;
+        part[(size_t)(r0 + r) * gridDim.x + blockIdx.x] = p;
     }
 }
 
-// d (rows x cols) *= (h > 0) when relu; db[c] += sum_r d[r][c]
-__global__ void k_relu_back_bias(float* __restrict__ d, const float* __restrict__ h, int rows, int cols, int relu,
-                                 float* __restrict__ db)
+// one warp per row: the chunks' sums joined, the loss, the geometric weight
+__global__ void __launch_bounds__(32) k_softmax_rows(const SmPart* __restrict__ part, int nchunk, const float* __restrict__ y,
+                                                     const bf16* __restrict__ bias, const unsigned char* __restrict__ skip,
+                                                     int KO, const int* __restrict__ tgt_oc, const float* __restrict__ tgt_w,
+                                                     const float* __restrict__ geo, SmRow* __restrict__ row, double* loss)
+{
+    const int b = blockIdx.x, lane = threadIdx.x;
+    const SmPart* p = part + (size_t)b * nchunk;
+    float mx = -INFINITY;
+    for (int i = lane; i < nchunk; i += 32) mx = fmaxf(mx, p[i].mx);
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    double se = 0., gz = 0., gy = 0.;
+    for (int i = lane; i < nchunk; i += 32) {
+        if (p[i].mx == -INFINITY) continue;   // a chunk without an orientation of the softmax
+        se += p[i].se * exp((double)p[i].mx - (double)mx);
+        gz += p[i].gz;
+        gy += p[i].gy;
+    }
+    const double lse_all = [&] {
+        for (int o = 16; o > 0; o >>= 1) {
+            se += __shfl_xor_sync(0xffffffffu, se, o);
+            gz += __shfl_xor_sync(0xffffffffu, gz, o);
+            gy += __shfl_xor_sync(0xffffffffu, gy, o);
+        }
+        return log(se);
+    }();
+    double lq = 0.;
+    for (int j = lane; j < NET_NTGT; j += 32) {
+        const int oc = tgt_oc[(size_t)b * NET_NTGT + j];
+        const float q = tgt_w[(size_t)b * NET_NTGT + j];
+        if (oc >= 0 && q > 0.f && !skip[oc])
+            lq += q * (lse_all - (double)(y[(size_t)b * KO + oc] + __bfloat162float(bias[oc]) - mx));
+    }
+    for (int o = 16; o > 0; o >>= 1) lq += __shfl_xor_sync(0xffffffffu, lq, o);
+    if (lane == 0) {
+        const float gw = geo ? geo[(size_t)b * 10 + 9] : 0.f;
+        const bool on = gw > 0.f && gz > 0.;
+        // the reported loss counts the geometric term GEO_LOSS times (it did from the start, once per thread of a
+        // block, and reports are compared with each other); the gradient is that of the plain sum
+        if (on) lq += GEO_LOSS * gw * ((lse_all + mx) * gz - gy) / gz;
+        row[b] = SmRow{lse_all, mx, on ? (float)(gw / gz) : 0.f};
+        atomicAdd(loss, lq);
+    }
+}
+
+// x = p0 + p1 + p2 in BF16
+__device__ __forceinline__ void split3(float x, bf16* p)
+{
+    p[0] = __float2bfloat16_rn(x);
+    const float r = x - __bfloat162float(p[0]);
+    p[1] = __float2bfloat16_rn(r);
+    p[2] = __float2bfloat16_rn(r - __bfloat162float(p[1]));
+}
+
+// The split forms of a rows x C matrix whose values come from `value(r, c)`, after `touch(r0, tile)`
+// has been through each tile of 32 rows: row-major parts rp [3][rows][ldr] and transposed parts
+// tp [3][C][ldt] (either may be null), and the sums over the block's rows into colsum (may be null).  A block
+// takes 32 columns and the row tiles blockIdx.y, blockIdx.y + gridDim.y, ....
+template <class Value, class Touch>
+__device__ __forceinline__ void split_tiles(int rows, int C, bf16* rp, int ldr, bf16* tp, int ldt, float* colsum,
+                                            Value value, Touch touch)
+{
+    __shared__ float tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 8 warps: rows ty, ty + 8, ...
+    const int c = blockIdx.x * 32 + tx;
+    float sum = 0.f;
+    for (int r0 = blockIdx.y * 32; r0 < rows; r0 += 32 * gridDim.y) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = r0 + ty + 8 * i;
+            tile[ty + 8 * i][tx] = r < rows && c < C ? value(r, c) : 0.f;
+        }
+        __syncthreads();
+        if (touch(r0, tile)) __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = r0 + ty + 8 * i;
+            const float v = tile[ty + 8 * i][tx];
+            sum += v;
+            if (rp && r < rows && c < C) {
+                bf16 p[3];
+                split3(v, p);
+#pragma unroll
+                for (int k = 0; k < 3; k++) rp[((size_t)k * rows + r) * ldr + c] = p[k];
+            }
+        }
+        if (tp) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int cc = blockIdx.x * 32 + ty + 8 * i, r = r0 + tx;
+                if (cc < C && r < rows) {
+                    bf16 p[3];
+                    split3(tile[tx][ty + 8 * i], p);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) tp[((size_t)k * C + cc) * ldt + r] = p[k];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (colsum) {
+        tile[ty][tx] = sum;
+        __syncthreads();
+        if (ty == 0 && c < C) {
+            float s = 0.f;
+            for (int i = 0; i < 8; i++) s += tile[i][tx];
+            colsum[c] = s;
+        }
+    }
+}
+
+// dL/dlogit = (softmax - q) / nb of the rows, and its sums over them (the bias gradient)
+__global__ void __launch_bounds__(256) k_softmax_split(const float* __restrict__ y, const bf16* __restrict__ bias,
+                                                       const unsigned char* __restrict__ skip, int KO, int nb,
+                                                       const int* __restrict__ tgt_oc, const float* __restrict__ tgt_w,
+                                                       const float* __restrict__ geo, const int* __restrict__ gcls,
+                                                       const float* __restrict__ eulf, int O, float inv2s2,
+                                                       const SmRow* __restrict__ row, bf16* rp, int ldr, bf16* tp, int ldt,
+                                                       float* colsum)
+{
+    const int c0 = blockIdx.x * 32, c = c0 + (threadIdx.x & 31);
+    const bool on = c < KO && !skip[c];
+    const float b3 = on ? __bfloat162float(bias[c]) : 0.f, inv = 1.f / nb;
+    float E[9];
+    if (geo && c < KO)
+#pragma unroll
+        for (int j = 0; j < 9; j++) E[j] = eulf[(size_t)j * O + c % O];
+    const int cls = c / O;
+    split_tiles(
+        nb, KO, rp, ldr, tp, ldt, colsum,
+        [&](int r, int cc) {
+            if (!on) return 0.f;
+            const SmRow st = row[r];
+            float v = (float)exp((double)(y[(size_t)r * KO + cc] + b3 - st.mx) - st.lse);
+            if (st.gs > 0.f && cls == gcls[r]) v -= st.gs * geo_q(E, geo + (size_t)r * 10, inv2s2);
+            return v * inv;
+        },
+        [&](int r0, float (*tile)[33]) {
+            // the sparse targets of the tile's rows, one thread per row
+            const int r = r0 + threadIdx.x;
+            if (threadIdx.x < 32 && r < nb)
+                for (int j = 0; j < NET_NTGT; j++) {
+                    const int oc = tgt_oc[(size_t)r * NET_NTGT + j];
+                    const float q = tgt_w[(size_t)r * NET_NTGT + j];
+                    if (oc >= c0 && oc < c0 + 32 && q > 0.f && !skip[oc]) tile[threadIdx.x][oc - c0] += -q * inv;
+                }
+            return true;
+        });
+}
+
+// x = act(sum_s in_s + bias) (K slices rows x C apart, in slice order), masked where `mask` is not positive;
+// as FP32 (out), split operands and sums over the rows (gridDim.y x C, joined by k_colsum)
+__global__ void __launch_bounds__(256) k_split_parts(const float* __restrict__ in, int slices, int rows, int C,
+                                                     const bf16* __restrict__ bias, int relu, const float* __restrict__ mask,
+                                                     float* out, bf16* rp, bf16* tp, int ldt, float* colpart)
+{
+    const size_t step = (size_t)rows * C;
+    split_tiles(
+        rows, C, rp, C, tp, ldt, colpart ? colpart + (size_t)blockIdx.y * C : nullptr,
+        [&](int r, int c) {
+            const float* p = in + (size_t)r * C + c;
+            float v = p[0];
+            int s = 1;
+            for (; s + 3 < slices; s += 4) {   // four loads in flight, summed in slice order
+                const float a0 = p[s * step], a1 = p[(s + 1) * step], a2 = p[(s + 2) * step], a3 = p[(s + 3) * step];
+                v += a0;
+                v += a1;
+                v += a2;
+                v += a3;
+            }
+            for (; s < slices; s++) v += p[s * step];
+            if (bias) v += __bfloat162float(bias[c]);
+            if (relu) v = fmaxf(v, 0.f);
+            if (mask && !(mask[(size_t)r * C + c] > 0.f)) v = 0.f;
+            if (out) out[(size_t)r * C + c] = v;
+            return v;
+        },
+        [](int, float (*)[33]) { return false; });
+}
+
+__global__ void k_colsum(const float* __restrict__ part, int n, int C, float* __restrict__ out)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float acc = 0.f;
-    for (int r = 0; r < rows; r++) {
-        float v = d[(size_t)r * cols + c];
-        if (relu && !(h[(size_t)r * cols + c] > 0.f)) { v = 0.f; d[(size_t)r * cols + c] = 0.f; }
-        acc += v;
+    if (c >= C) return;
+    float s = 0.f;
+    for (int i = 0; i < n; i++) s += part[(size_t)i * C + c];
+    out[c] = s;
+}
+
+// W [R][C] -> WT [C][ldt]
+__global__ void __launch_bounds__(256) k_transpose_bf16(const bf16* __restrict__ in, int R, int C, bf16* __restrict__ out,
+                                                        int ldt)
+{
+    __shared__ bf16 tile[32][34];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int i = ty; i < 32; i += 8) {
+        const int r = blockIdx.y * 32 + i, c = blockIdx.x * 32 + tx;
+        if (r < R && c < C) tile[i][tx] = in[(size_t)r * C + c];
     }
-    db[c] += acc;
+    __syncthreads();
+    for (int i = ty; i < 32; i += 8) {
+        const int c = blockIdx.x * 32 + i, r = blockIdx.y * 32 + tx;
+        if (r < R && c < C) out[(size_t)c * ldt + r] = tile[tx][i];
+    }
 }
 
 // conv2 / conv1 backward of one particle per CTA: dx0 (2048, before the
-// ReLU mask) -> conv weight and bias gradients (atomics into g)
+// ReLU mask) -> conv weight and bias gradients (atomics into g).  Bound by shared-memory reads: dx0 lies
+// as [position][channel] and the conv2 weights as [tap][c1][c2], so that four channels come with one read
+// (one weight and one position at a time, the weights from memory, took 119 us for 256 particles).
+struct ConvBwdSmem {
+    float im[18][18];
+    float a1[NET_C1][18][18];
+    float d2[64][NET_C2 + 4];   // rows 144 bytes apart: lanes of different positions on different banks
+    float da1[NET_C1][16][16];
+    float w2[9][NET_C1][NET_C2];
+};
 __global__ void __launch_bounds__(256) k_conv_bwd(const float* __restrict__ img, const float* __restrict__ a1g,
                                                   const float* __restrict__ x0, const float* __restrict__ dx0,
                                                   const bf16* __restrict__ th, NetLayout L, float* __restrict__ g)
 {
-    __shared__ float im[18][18];
-    __shared__ float a1[NET_C1][18][18];
-    __shared__ float d2[NET_H0];
-    __shared__ float da1[NET_C1][16][16];
+    extern __shared__ __align__(16) unsigned char cb_raw[];
+    ConvBwdSmem& S = *reinterpret_cast<ConvBwdSmem*>(cb_raw);
     const int b = blockIdx.x;
-    for (int i = threadIdx.x; i < 18 * 18; i += blockDim.x) (&im[0][0])[i] = 0.f;
-    for (int i = threadIdx.x; i < NET_C1 * 18 * 18; i += blockDim.x) (&a1[0][0][0])[i] = 0.f;
+    for (int i = threadIdx.x; i < 18 * 18; i += blockDim.x) (&S.im[0][0])[i] = 0.f;
+    for (int i = threadIdx.x; i < NET_C1 * 18 * 18; i += blockDim.x) (&S.a1[0][0][0])[i] = 0.f;
+    for (int i = threadIdx.x; i < NET_C2 * NET_C1 * 9; i += blockDim.x) {
+        const int c2 = i / (NET_C1 * 9), r = i - c2 * (NET_C1 * 9), c1 = r / 9;   // global layout [c2][c1][dy][dx]
+        S.w2[r - c1 * 9][c1][c2] = ldw(th, L.wc2 + i);
+    }
+    for (int o = threadIdx.x; o < NET_H0; o += blockDim.x)
+        S.d2[o & 63][o >> 6] = x0[(size_t)b * NET_H0 + o] > 0.f ? dx0[(size_t)b * NET_H0 + o] : 0.f;
     __syncthreads();
     {
         const int y = threadIdx.x >> 4, x = threadIdx.x & 15;
-        im[y + 1][x + 1] = img[(size_t)b * NET_NPIX + threadIdx.x];
-        for (int c = 0; c < NET_C1; c++) a1[c][y + 1][x + 1] = a1g[(size_t)b * NET_C1 * NET_NPIX + c * NET_NPIX + threadIdx.x];
+        S.im[y + 1][x + 1] = img[(size_t)b * NET_NPIX + threadIdx.x];
+        for (int c = 0; c < NET_C1; c++) S.a1[c][y + 1][x + 1] = a1g[(size_t)b * NET_C1 * NET_NPIX + c * NET_NPIX + threadIdx.x];
     }
-    for (int o = threadIdx.x; o < NET_H0; o += blockDim.x)
-        d2[o] = x0[(size_t)b * NET_H0 + o] > 0.f ? dx0[(size_t)b * NET_H0 + o] : 0.f;
     __syncthreads();
-    // conv2 weights: dW[c2][c1][dy][dx] = sum_{Y,X} d2[c2][Y][X] a1[c1][2Y+dy][2X+dx] (padded coordinates)
-    for (int wi = threadIdx.x; wi < NET_C2 * NET_C1 * 9; wi += blockDim.x) {
-        const int c2 = wi / (NET_C1 * 9), r = wi - c2 * NET_C1 * 9, c1 = r / 9, dy = (r % 9) / 3, dx = r % 3;
-        float acc = 0.f;
+    // conv2 weights: dW[c2][c1][dy][dx] = sum_{Y,X} d2[c2][Y][X] a1[c1][2Y+dy][2X+dx] (padded coordinates);
+    // eight c2 of one (c1, tap) per item
+    for (int e = threadIdx.x; e < NET_C1 * 9 * (NET_C2 / 8); e += blockDim.x) {
+        const int cg = e / (NET_C1 * 9) * 8, r = e % (NET_C1 * 9), c1 = r / 9, tap = r - c1 * 9, dy = tap / 3, dx = tap % 3;
+        float acc[8] = {};
         for (int Y = 0; Y < 8; Y++)
-            for (int X = 0; X < 8; X++) acc += d2[c2 * 64 + Y * 8 + X] * a1[c1][2 * Y + dy][2 * X + dx];
-        atomicAdd(&g[L.wc2 + wi], acc);
+#pragma unroll
+            for (int X = 0; X < 8; X++) {
+                const float a = S.a1[c1][2 * Y + dy][2 * X + dx];
+                const float4 d0 = *reinterpret_cast<const float4*>(&S.d2[Y * 8 + X][cg]);
+                const float4 d1 = *reinterpret_cast<const float4*>(&S.d2[Y * 8 + X][cg + 4]);
+                acc[0] += d0.x * a; acc[1] += d0.y * a; acc[2] += d0.z * a; acc[3] += d0.w * a;
+                acc[4] += d1.x * a; acc[5] += d1.y * a; acc[6] += d1.z * a; acc[7] += d1.w * a;
+            }
+#pragma unroll
+        for (int k = 0; k < 8; k++) atomicAdd(&g[L.wc2 + (size_t)(cg + k) * NET_C1 * 9 + r], acc[k]);
     }
     if (threadIdx.x < NET_C2) {
         float acc = 0.f;
-        for (int q = 0; q < 64; q++) acc += d2[threadIdx.x * 64 + q];
+        for (int q = 0; q < 64; q++) acc += S.d2[q][threadIdx.x];
         atomicAdd(&g[L.bc2 + threadIdx.x], acc);
     }
-    // da1[c1][y][x]: every conv2 output reading padded position (y+1, x+1), masked by a1 > 0
+    // da1[c1][y][x]: every conv2 output reading padded position (y+1, x+1), masked by a1 > 0.  The stride-2
+    // taps that do depend on the parities of y and x, so two warps share one pair of parities
     {
-        const int y = threadIdx.x >> 4, x = threadIdx.x & 15;
+        const int cls = threadIdx.x >> 6, q = threadIdx.x & 63;
+        const int y = 2 * (q >> 3) + (cls >> 1), x = 2 * (q & 7) + (cls & 1);
         for (int c1 = 0; c1 < NET_C1; c1++) {
             float acc = 0.f;
-            for (int dy = 0; dy < 3; dy++) {
-                const int yy = y + 1 - dy;
-                if (yy < 0 || (yy & 1)) continue;
-                const int Y = yy >> 1;
+            for (int dy = (y & 1) ? 0 : 1; dy < 3; dy += 2) {
+                const int Y = (y + 1 - dy) >> 1;
                 if (Y >= 8) continue;
-                for (int dx = 0; dx < 3; dx++) {
-                    const int xx = x + 1 - dx;
-                    if (xx < 0 || (xx & 1)) continue;
-                    const int X = xx >> 1;
+                for (int dx = (x & 1) ? 0 : 1; dx < 3; dx += 2) {
+                    const int X = (x + 1 - dx) >> 1;
                     if (X >= 8) continue;
-                    for (int c2 = 0; c2 < NET_C2; c2++)
-                        acc += d2[c2 * 64 + Y * 8 + X] * ldw(th, L.wc2 + ((size_t)c2 * NET_C1 + c1) * 9 + dy * 3 + dx);
+                    const float4* d = reinterpret_cast<const float4*>(S.d2[Y * 8 + X]);
+                    const float4* w = reinterpret_cast<const float4*>(S.w2[dy * 3 + dx][c1]);
+#pragma unroll
+                    for (int k = 0; k < NET_C2 / 4; k++) {
+                        const float4 dv = d[k], wv = w[k];
+                        acc += dv.x * wv.x;
+                        acc += dv.y * wv.y;
+                        acc += dv.z * wv.z;
+                        acc += dv.w * wv.w;
+                    }
                 }
             }
-            da1[c1][y][x] = a1[c1][y + 1][x + 1] > 0.f ? acc : 0.f;
+            S.da1[c1][y][x] = S.a1[c1][y + 1][x + 1] > 0.f ? acc : 0.f;
         }
     }
     __syncthreads();
-    // conv1 weights and bias
-    for (int wi = threadIdx.x; wi < NET_C1 * 9; wi += blockDim.x) {
-        const int c1 = wi / 9, dy = (wi % 9) / 3, dx = wi % 3;
+    // conv1 weights and bias: a warp per (c1, tap) or c1, lanes over the pixels
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int wi = warp; wi < NET_C1 * 10; wi += 8) {
+        const int c1 = wi % NET_C1, tap = wi / NET_C1, dy = tap / 3, dx = tap % 3;   // tap 9: the bias
         float acc = 0.f;
-        for (int y = 0; y < 16; y++)
-            for (int x = 0; x < 16; x++) acc += da1[c1][y][x] * im[y + dy][x + dx];
-        atomicAdd(&g[L.wc1 + wi], acc);
-    }
-    if (threadIdx.x < NET_C1) {
-        float acc = 0.f;
-        for (int q = 0; q < 256; q++) acc += (&da1[threadIdx.x][0][0])[q];
-        atomicAdd(&g[L.bc1 + threadIdx.x], acc);
+#pragma unroll
+        for (int q = lane; q < 256; q += 32) {
+            const int y = q >> 4, x = q & 15;
+            acc += S.da1[c1][y][x] * (tap == 9 ? 1.f : S.im[y + dy][x + dx]);
+        }
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) atomicAdd(&g[tap == 9 ? L.bc1 + c1 : L.wc1 + c1 * 9 + tap], acc);
     }
 }
 
-// Adam (bias-corrected), then the BF16 copy every forward pass reads
+// Adam, then the BF16 copy every forward pass reads
 __global__ void k_adam(float* __restrict__ th, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       bf16* __restrict__ thb, size_t n, float lr, float c1, float c2)
+                       bf16* __restrict__ thb, size_t n, AdamStep step)
 {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = 0.9f * m[i] + 0.1f * gi;
-        const float vi = 0.999f * v[i] + 0.001f * gi * gi;
+        float t = th[i], mi = m[i], vi = v[i];
+        adam_update(t, mi, vi, g[i], step);
         m[i] = mi;
         v[i] = vi;
-        const float t = th[i] - lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
         th[i] = t;
         thb[i] = __float2bfloat16_rn(t);
     }
@@ -1364,7 +1560,7 @@ void free_list(std::vector<void*>& v)
 // as the matched filter of the feature image against the templates T_oc.
 void init_params_host(const NetLayout& L, unsigned long long seed, std::vector<float>& h)
 {
-    h.assign(L.alloc, 0.f);
+    h.assign(L.w3, 0.f);   // fc3 is filled on the device (k_init_w3)
     std::mt19937_64 rng(seed ^ 0x5eed5eedull);
     auto fill = [&](size_t off, size_t cnt, int fan_in) {
         const float bnd = 0.01f / std::sqrt((float)fan_in);
@@ -1435,7 +1631,8 @@ ProposalNet& net_params(t2b_ctx* c, int KO)
     N.thb = net_dalloc(N.owned, n * sizeof(bf16));
     std::vector<float> h;
     init_params_host(N.L, 1, h);
-    T2B_CUDA(cudaMemcpy(N.th, h.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+    T2B_CUDA(cudaMemcpy(N.th, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+    T2B_CUDA(cudaMemset(N.th + h.size(), 0, (n - h.size()) * sizeof(float)));
     T2B_CUDA(cudaMemset(N.g, 0, n * sizeof(float)));
     T2B_CUDA(cudaMemset(N.m, 0, n * sizeof(float)));
     T2B_CUDA(cudaMemset(N.v, 0, n * sizeof(float)));
@@ -1611,80 +1808,191 @@ void infer_dense(ProposalNet& N, int n, int* err, cudaStream_t st)
     T2B_CUDA(cudaGetLastError());
 }
 
-template <bool AT, bool BT, typename TA, typename TB>
-void sgemm(int M, int N, int K, const TA* A, int lda, const TB* B, int ldb, float* C, int ldc, int splitk,
-           cudaStream_t st)
-{
-    const int kchunk = ((K + splitk - 1) / splitk + 15) / 16 * 16;
-    const int z = (K + kchunk - 1) / kchunk;
-    if (z > 1) T2B_CUDA(cudaMemsetAsync(C, 0, sizeof(float) * (size_t)M * ldc, st));
-    dim3 grid((N + 63) / 64, (M + 63) / 64, z);
-    k_sgemm<AT, BT, TA, TB><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, kchunk);
-    T2B_CUDA(cudaGetLastError());
-}
+int round64(int x) { return (x + 63) / 64 * 64; }
 
-// buffers of one training minibatch of nb particles
-struct TrainBufs {
-    std::vector<void*> mem;
-    int nb = 0;
-    float *bimg, *a1, *x0, *h1, *h2, *y, *dh2, *dh1, *dx0, *tgt_w, *geo;
-    int *tgt_oc, *gcls;
-    double* loss;
-    TrainBufs(int nb_, int KO) : nb(nb_)
+// FP32 activations or gradients (rows x C) as operands of the tensor-core products: split row-major
+// (contracted over C) and transposed (contracted over the rows, padded to ldt)
+struct SplitMat {
+    bf16 *rp = nullptr, *tp = nullptr;
+    TgOperand cols, t;   // row-major, transposed
+    template <class Take>
+    void alloc(Take take, int rows, int C, int ldr, int ldt)
     {
-        auto f = [&](size_t n) { return (float*)net_dalloc(mem, n * sizeof(float)); };
-        bimg = f((size_t)nb * NET_NPIX);
-        a1 = f((size_t)nb * NET_C1 * NET_NPIX);
-        x0 = f((size_t)nb * NET_H0);
-        h1 = f((size_t)nb * NET_H1);
-        h2 = f((size_t)nb * NET_H2);
-        y = f((size_t)nb * KO);
-        dh2 = f((size_t)nb * NET_H2);
-        dh1 = f((size_t)nb * NET_H1);
-        dx0 = f((size_t)nb * NET_H0);
-        tgt_w = f((size_t)nb * NET_NTGT);
-        geo = f((size_t)nb * 10);
-        tgt_oc = (int*)net_dalloc(mem, (size_t)nb * NET_NTGT * sizeof(int));
-        gcls = (int*)net_dalloc(mem, (size_t)nb * sizeof(int));
-        loss = (double*)net_dalloc(mem, sizeof(double));
+        rp = (bf16*)take((size_t)3 * rows * ldr * sizeof(bf16));
+        tp = (bf16*)take((size_t)3 * C * ldt * sizeof(bf16));
     }
-    ~TrainBufs() { free_list(mem); }
+    void maps(int rows, int C, int ldr, int ldt)
+    {
+        cols = tg_operand(rp, 3, rows, C, ldr);
+        t = tg_operand(tp, 3, C, rows, ldt);
+    }
 };
 
-// forward + backward of one minibatch (bimg and targets filled): gradient in
-// N.g, summed loss added to *t.loss; use_geo: the rows' geometric targets count
+// buffers and operands of one training minibatch of nb particles
+struct TrainBufs {
+    std::vector<void*> mem;
+    int nb = 0, ldt = 0, kol = 0, nchunk = 0;
+    float *bimg, *a1, *x0, *h1, *h2, *y, *dx0, *tgt_w, *geo, *slices, *eulf, *colpart;
+    int *tgt_oc, *gcls, *err;
+    double* loss;
+    SmPart* part;
+    SmRow* row;
+    SplitMat X0, H1m, H2m, DY, D2, D1;
+    bf16 *w1t, *w2t, *w3t;
+    TgOperand W1, W2, W3, W1T, W2T, W3T;
+    TrainBufs(int nb_, const ProposalNet& N, const Tables& tb) : nb(nb_)
+    {
+        const int KO = N.KO;
+        const NetLayout& L = N.L;
+        ldt = round64(nb);
+        kol = round64(KO);
+        nchunk = (KO + SM_CHUNK - 1) / SM_CHUNK;
+        // one allocation, laid out in 256-byte steps: a first walk for its size
+        char* basep = nullptr;
+        size_t used = 0;
+        auto take = [&](size_t bytes) -> void* {
+            void* p = basep ? basep + used : nullptr;
+            used += (bytes + 255) & ~size_t(255);
+            return p;
+        };
+        auto f = [&](size_t n) { return (float*)take(n * sizeof(float)); };
+        for (int pass = 0; pass < 2; pass++) {
+            if (pass) {
+                basep = (char*)net_dalloc(mem, used);
+                used = 0;
+            }
+            bimg = f((size_t)nb * NET_NPIX);
+            a1 = f((size_t)nb * NET_C1 * NET_NPIX);
+            x0 = f((size_t)nb * NET_H0);
+            h1 = f((size_t)nb * NET_H1);
+            h2 = f((size_t)nb * NET_H2);
+            y = f((size_t)nb * KO);
+            dx0 = f((size_t)nb * NET_H0);
+            tgt_w = f((size_t)nb * NET_NTGT);
+            geo = f((size_t)nb * 10);
+            slices = f((size_t)MAX_SLICES * nb * NET_H0);
+            eulf = f((size_t)9 * tb.O);
+            colpart = f((size_t)COL_PARTS * NET_H0);
+            tgt_oc = (int*)take((size_t)nb * NET_NTGT * sizeof(int));
+            gcls = (int*)take((size_t)nb * sizeof(int));
+            err = (int*)take(sizeof(int));
+            loss = (double*)take(sizeof(double));
+            part = (SmPart*)take((size_t)nb * nchunk * sizeof(SmPart));
+            row = (SmRow*)take((size_t)nb * sizeof(SmRow));
+            X0.alloc(take, nb, NET_H0, NET_H0, ldt);
+            H1m.alloc(take, nb, NET_H1, NET_H1, ldt);
+            H2m.alloc(take, nb, NET_H2, NET_H2, ldt);
+            DY.alloc(take, nb, KO, kol, ldt);
+            D2.alloc(take, nb, NET_H2, NET_H2, ldt);
+            D1.alloc(take, nb, NET_H1, NET_H1, ldt);
+            w1t = (bf16*)take((size_t)NET_H0 * NET_H1 * sizeof(bf16));
+            w2t = (bf16*)take((size_t)NET_H1 * NET_H2 * sizeof(bf16));
+            w3t = (bf16*)take((size_t)NET_H2 * kol * sizeof(bf16));
+        }
+        X0.maps(nb, NET_H0, NET_H0, ldt);
+        H1m.maps(nb, NET_H1, NET_H1, ldt);
+        H2m.maps(nb, NET_H2, NET_H2, ldt);
+        DY.maps(nb, KO, kol, ldt);
+        D2.maps(nb, NET_H2, NET_H2, ldt);
+        D1.maps(nb, NET_H1, NET_H1, ldt);
+        bf16* thb = (bf16*)N.thb;
+        W1 = tg_operand(thb + L.w1, 1, NET_H1, NET_H0, NET_H0);
+        W2 = tg_operand(thb + L.w2, 1, NET_H2, NET_H1, NET_H1);
+        W3 = tg_operand(thb + L.w3, 1, KO, NET_H2, NET_H2);
+        W1T = tg_operand(w1t, 1, NET_H0, NET_H1, NET_H1);
+        W2T = tg_operand(w2t, 1, NET_H1, NET_H2, NET_H2);
+        W3T = tg_operand(w3t, 1, NET_H2, KO, kol);
+    }
+    ~TrainBufs() { free_list(mem); }
+    TrainBufs(const TrainBufs&) = delete;
+    TrainBufs& operator=(const TrainBufs&) = delete;
+    static constexpr int MAX_SLICES = 9;    // of the widest output (H0); 18 of the others
+    static constexpr int COL_PARTS = 8;     // row shares of the bias sums
+
+    // tables that follow the parameters and the sampling; the error flag
+    void begin(const ProposalNet& N, const Tables& tb, cudaStream_t st)
+    {
+        const bf16* thb = (const bf16*)N.thb;
+        auto tr = [&](const bf16* w, int R, int C, bf16* out, int ld) {
+            k_transpose_bf16<<<dim3((C + 31) / 32, (R + 31) / 32), 256, 0, st>>>(w, R, C, out, ld);
+        };
+        tr(thb + N.L.w1, NET_H1, NET_H0, w1t, NET_H1);
+        tr(thb + N.L.w2, NET_H2, NET_H1, w2t, NET_H2);
+        tr(thb + N.L.w3, N.KO, NET_H2, w3t, kol);
+        k_geo_table<<<(9 * tb.O + 255) / 256, 256, 0, st>>>(tb.eul_c, tb.O, eulf);
+        T2B_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
+        T2B_CUDA(cudaGetLastError());
+    }
+    // a bounded wait of a product ran out
+    void check(cudaStream_t st) const
+    {
+        int e = 0;
+        T2B_CUDA(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        T2B_CUDA(cudaStreamSynchronize(st));
+        T2B_REQUIRE(e == 0, T2B_ERR_TIMEOUT, "proposal training: a device-side wait ran out");
+    }
+};
+
 float inv2s2_of(double sigma_deg)
 {
     const double s = sigma_deg * PI / 180.;
     return (float)(1. / (2. * s * s));
 }
 
-void train_fwd_bwd(ProposalNet& N, TrainBufs& t, const Tables& tb, bool use_geo, float inv2s2, cudaStream_t st)
+// Forward and backward pass of one minibatch (bimg and targets filled), summed loss added to *t.loss;
+// use_geo: the rows' geometric targets count.  With `step` the weight matrices take their Adam step as
+// soon as their gradient tiles are ready and nothing later reads the old values (their transposes
+// are read by the backward product before); the gradients of the small parameters (below L.w1) are in N.g
+// and take theirs last.  Without it every gradient goes to N.g.
+void train_fwd_bwd(ProposalNet& N, TrainBufs& t, const Tables& tb, bool use_geo, float inv2s2, const AdamStep* step,
+                   cudaStream_t st)
 {
     const NetLayout& L = N.L;
     const int nb = t.nb, KO = N.KO;
-    const bf16* thb = (const bf16*)N.thb;
+    bf16* thb = (bf16*)N.thb;
     float* g = N.g;
+    const float* geo = use_geo ? t.geo : nullptr;
+    // K slices so that the tiles fill the SMs
+    auto slices = [&](int M) { return std::max(1, std::min(M > NET_H1 ? 9 : 18, 148 / tg_tiles(M, nb))); };
+    auto split = [&](const float* in, int ns, int C, const bf16* bias, int relu, const float* mask, float* out, SplitMat* m,
+                     float* colsum) {
+        const dim3 grid((C + 31) / 32, std::min(TrainBufs::COL_PARTS, (nb + 31) / 32));
+        k_split_parts<<<grid, 256, 0, st>>>(in, ns, nb, C, bias, relu, mask, out, m ? m->rp : nullptr, m ? m->tp : nullptr,
+                                            t.ldt, colsum ? t.colpart : nullptr);
+        if (colsum) k_colsum<<<(C + 255) / 256, 256, 0, st>>>(t.colpart, (int)grid.y, C, colsum);
+    };
+    auto product = [&](const TgOperand& w, const SplitMat& x, int M, int K) {
+        return tg_product(w, x.cols, true, M, nb, K, t.slices, M, slices(M), t.err, st);
+    };
+    auto gradient = [&](const SplitMat& in, const SplitMat& d, int M, int O, size_t off, bf16* wt, int ldt) {
+        if (step) {
+            const TgAdam w{N.th + off, N.m + off, N.v + off, thb + off, wt, M, ldt, *step};
+            tg_gradient_adam(in.t, d.t, M, O, nb, w, t.err, st);
+        } else {
+            tg_product(in.t, d.t, false, M, O, nb, g + off, M, 1, t.err, st);
+        }
+    };
+    T2B_CUDA(cudaMemsetAsync(g, 0, L.w1 * sizeof(float), st));
     k_conv_fwd<<<nb, 256, 0, st>>>(t.bimg, thb, L, nb, t.a1, t.x0, nullptr);
-    sgemm<false, true>(nb, NET_H1, NET_H0, t.x0, NET_H0, thb + L.w1, NET_H0, t.h1, NET_H1, 1, st);
-    k_bias_act<<<gridsz((size_t)nb * NET_H1), 256, 0, st>>>(t.h1, thb + L.b1, nb, NET_H1, 1, t.h1, nullptr);
-    sgemm<false, true>(nb, NET_H2, NET_H1, t.h1, NET_H1, thb + L.w2, NET_H1, t.h2, NET_H2, 1, st);
-    k_bias_act<<<gridsz((size_t)nb * NET_H2), 256, 0, st>>>(t.h2, thb + L.b2, nb, NET_H2, 1, t.h2, nullptr);
-    sgemm<false, true>(nb, KO, NET_H2, t.h2, NET_H2, thb + L.w3, NET_H2, t.y, KO, 1, st);
-    k_softmax_ce<<<nb, 1024, 0, st>>>(t.y, thb + L.b3, tb.skip, KO, t.tgt_oc, t.tgt_w, use_geo ? t.geo : nullptr,
-                                      t.gcls, tb.eul_c, tb.O, inv2s2, nb, t.loss);
-    // backward: t.y now holds dL/dlogits
-    T2B_CUDA(cudaMemsetAsync(g, 0, L.alloc * sizeof(float), st));
-    k_relu_back_bias<<<(KO + 255) / 256, 256, 0, st>>>(t.y, nullptr, nb, KO, 0, g + L.b3);
-    sgemm<true, false>(KO, NET_H2, nb, t.y, KO, t.h2, NET_H2, g + L.w3, NET_H2, 1, st);
-    sgemm<false, false>(nb, NET_H2, KO, t.y, KO, thb + L.w3, NET_H2, t.dh2, NET_H2, 32, st);
-    k_relu_back_bias<<<(NET_H2 + 255) / 256, 256, 0, st>>>(t.dh2, t.h2, nb, NET_H2, 1, g + L.b2);
-    sgemm<true, false>(NET_H2, NET_H1, nb, t.dh2, NET_H2, t.h1, NET_H1, g + L.w2, NET_H1, 1, st);
-    sgemm<false, false>(nb, NET_H1, NET_H2, t.dh2, NET_H2, thb + L.w2, NET_H1, t.dh1, NET_H1, 4, st);
-    k_relu_back_bias<<<(NET_H1 + 255) / 256, 256, 0, st>>>(t.dh1, t.h1, nb, NET_H1, 1, g + L.b1);
-    sgemm<true, false>(NET_H1, NET_H0, nb, t.dh1, NET_H1, t.x0, NET_H0, g + L.w1, NET_H0, 1, st);
-    sgemm<false, false>(nb, NET_H0, NET_H1, t.dh1, NET_H1, thb + L.w1, NET_H0, t.dx0, NET_H0, 4, st);
-    k_conv_bwd<<<nb, 256, 0, st>>>(t.bimg, t.a1, t.x0, t.dx0, thb, L, g);
+    split(t.x0, 1, NET_H0, nullptr, 0, nullptr, nullptr, &t.X0, nullptr);
+    split(t.slices, product(t.W1, t.X0, NET_H1, NET_H0), NET_H1, thb + L.b1, 1, nullptr, t.h1, &t.H1m, nullptr);
+    split(t.slices, product(t.W2, t.H1m, NET_H2, NET_H1), NET_H2, thb + L.b2, 1, nullptr, t.h2, &t.H2m, nullptr);
+    tg_product(t.W3, t.H2m.cols, true, KO, nb, NET_H2, t.y, KO, 1, t.err, st);
+    k_softmax_stats<<<dim3(t.nchunk, (nb + SM_ROWS - 1) / SM_ROWS), SM_THREADS, 0, st>>>(
+        t.y, thb + L.b3, tb.skip, KO, nb, geo, t.gcls, t.eulf, tb.O, inv2s2, t.part);
+    k_softmax_rows<<<nb, 32, 0, st>>>(t.part, t.nchunk, t.y, thb + L.b3, tb.skip, KO, t.tgt_oc, t.tgt_w, geo, t.row, t.loss);
+    k_softmax_split<<<(KO + 31) / 32, 256, 0, st>>>(t.y, thb + L.b3, tb.skip, KO, nb, t.tgt_oc, t.tgt_w, geo, t.gcls, t.eulf,
+                                                    tb.O, inv2s2, t.row, t.DY.rp, t.kol, t.DY.tp, t.ldt, g + L.b3);
+    split(t.slices, product(t.W3T, t.DY, NET_H2, KO), NET_H2, nullptr, 0, t.h2, nullptr, &t.D2, g + L.b2);
+    gradient(t.H2m, t.DY, NET_H2, KO, L.w3, t.w3t, t.kol);
+    split(t.slices, product(t.W2T, t.D2, NET_H1, NET_H2), NET_H1, nullptr, 0, t.h1, nullptr, &t.D1, g + L.b1);
+    gradient(t.H1m, t.D2, NET_H1, NET_H2, L.w2, t.w2t, NET_H2);
+    split(t.slices, product(t.W1T, t.D1, NET_H0, NET_H1), NET_H0, nullptr, 0, nullptr, t.dx0, nullptr, nullptr);
+    gradient(t.X0, t.D1, NET_H0, NET_H1, L.w1, t.w1t, NET_H1);
+    T2B_CUDA(cudaFuncSetAttribute(k_conv_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ConvBwdSmem)));
+    k_conv_bwd<<<nb, 256, sizeof(ConvBwdSmem), st>>>(t.bimg, t.a1, t.x0, t.dx0, thb, L, g);
+    if (step)
+        k_adam<<<gridsz(L.w1), 256, 0, st>>>(N.th, g, N.m, N.v, thb, L.w1, *step);
     T2B_CUDA(cudaGetLastError());
 }
 
@@ -1819,7 +2127,8 @@ void init_from_templates(t2b_ctx* c, ProposalNet& N, unsigned long long seed, co
     const Tables& tb = c->tb;
     std::vector<float> h;
     init_params_host(N.L, seed, h);
-    T2B_CUDA(cudaMemcpyAsync(N.th, h.data(), N.L.alloc * sizeof(float), cudaMemcpyHostToDevice, st));
+    T2B_CUDA(cudaMemcpyAsync(N.th, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+    T2B_CUDA(cudaMemsetAsync(N.th + h.size(), 0, (N.L.alloc - h.size()) * sizeof(float), st));
     DevBuf tmpl((size_t)N.KO * NET_NPIX * sizeof(float));
     for (int k = 0; k < tb.K; k++)
         k_features<<<tb.O, NET_NPIX, 0, st>>>(nullptr, nullptr, minv, tb.P, N.ring, N.ring_k, N.nring,
@@ -1998,7 +2307,8 @@ int t2b_proposal_train(t2b_ctx* c, const t2b_proposal_train_config* cfg, t2b_pro
             validate(&rep->val_mass_init, nullptr, nullptr, nullptr);
             // 4. Adam epochs over shuffled minibatches
             cudaEventRecord(e0, st);
-            TrainBufs t(f.batch, KO);
+            TrainBufs t(f.batch, N, tb);
+            t.begin(N, tb, st);
             std::vector<int> perm((size_t)ntr);
             std::iota(perm.begin(), perm.end(), 0);
             std::mt19937_64 rng(f.seed ^ 0x7261696eull);
@@ -2013,14 +2323,14 @@ int t2b_proposal_train(t2b_ctx* c, const t2b_proposal_train_config* cfg, t2b_pro
                     k_batch_gather<<<f.batch, 256, 0, st>>>(perm_d.as<int>() + i * f.batch, f.batch, imgs.as<float>(),
                                                             poses.as<float>(), pcls.as<int>(), poc.as<int>(),
                                                             pw.as<float>(), t.bimg, t.geo, t.gcls, t.tgt_oc, t.tgt_w);
-                    train_fwd_bwd(N, t, tb, true, inv2s2, st);
                     N.adam_t++;
-                    const float c1 = 1.f - std::pow(0.9f, (float)N.adam_t), c2 = 1.f - std::pow(0.999f, (float)N.adam_t);
-                    k_adam<<<gridsz(N.L.alloc), 256, 0, st>>>(N.th, N.g, N.m, N.v, (bf16*)N.thb, N.L.alloc, f.lr, c1, c2);
+                    const AdamStep step{(float)(f.lr / (1. - std::pow(0.9, (double)N.adam_t))),
+                                        (float)(1. / (1. - std::pow(0.999, (double)N.adam_t)))};
+                    train_fwd_bwd(N, t, tb, true, inv2s2, &step, st);
                 }
                 double l = 0.;
                 T2B_CUDA(cudaMemcpyAsync(&l, t.loss, sizeof(double), cudaMemcpyDeviceToHost, st));
-                T2B_CUDA(cudaStreamSynchronize(st));
+                t.check(st);
                 if (e < 64) rep->loss[e] = nbat > 0 ? l / ((double)nbat * f.batch) : 0.;
             }
             rep->train_ms = elapsed();
@@ -2165,12 +2475,14 @@ int t2b_proposal_grad(t2b_ctx* c, const float* imgs, const int* tgt_oc, const fl
         for (int i = 0; i < n * NET_NTGT; i++)
             T2B_REQUIRE(tgt_oc[i] >= -1 && tgt_oc[i] < KO, T2B_ERR_ARG, "target orientation out of range");
         cudaStream_t st = c->stream;
-        TrainBufs t(n, KO);
+        TrainBufs t(n, N, c->tb);
+        t.begin(N, c->tb, st);
         T2B_CUDA(cudaMemcpyAsync(t.bimg, imgs, (size_t)n * NET_NPIX * sizeof(float), cudaMemcpyHostToDevice, st));
         T2B_CUDA(cudaMemcpyAsync(t.tgt_oc, tgt_oc, (size_t)n * NET_NTGT * sizeof(int), cudaMemcpyHostToDevice, st));
         T2B_CUDA(cudaMemcpyAsync(t.tgt_w, tgt_w, (size_t)n * NET_NTGT * sizeof(float), cudaMemcpyHostToDevice, st));
         T2B_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(double), st));
-        train_fwd_bwd(N, t, c->tb, false, 0.f, st);
+        train_fwd_bwd(N, t, c->tb, false, 0.f, nullptr, st);
+        t.check(st);
         double l = 0.;
         T2B_CUDA(cudaMemcpyAsync(&l, t.loss, sizeof(double), cudaMemcpyDeviceToHost, st));
         T2B_CUDA(cudaMemcpyAsync(grad, N.g, N.L.total * sizeof(float), cudaMemcpyDeviceToHost, st));

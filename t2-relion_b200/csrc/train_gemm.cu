@@ -1,0 +1,338 @@
+// The dense products of the proposal network's training on the 5th-generation tensor cores, at FP32
+// accuracy.
+//
+// Weights are BF16 (as every forward pass reads them), activations and gradients FP32.  An FP32
+// value is split into three BF16 parts, x = p0 + p1 + p2 with p0 = bf16(x), p1 = bf16(x - p0),
+// p2 = bf16(x - p0 - p1): 24 bits, the whole significand.  BF16 products are exact in FP32, so
+//   activation x weight     3 products: every bit of the FP32 operand
+//   activation x gradient   6 products: p_i q_j with i + j <= 2 (the three left out are below 2^-24
+//                           of the product, less than the rounding of one FP32 accumulation)
+// accumulate in FP32.  The tensor core rounds its running sum towards zero: over the 192 steps of
+// a K of 1024 that came to 5e-6 of a gradient's norm, ten times what FP32 multiply-adds lose.  So
+// TMEM holds the sum of one 64-wide K block only, the leading product and the corrections (2^-8 of
+// it and less) apart, and the epilogue warps add both to registers, rounded to nearest, block by
+// block.
+//
+// k_train_gemm: persistent, one CTA per SM, 128 x 128 tiles.  Warp 0 issues the TMA loads of 64-wide K
+// blocks (all parts of both operands) into a ring of stages, warp 1 the tcgen05.mma, warps 2-17 collect
+// the double-buffered blocks: four warps per TMEM lane quarter, each 32 columns.  The accumulator's
+// lane is the output's contiguous axis, so loads and stores of the epilogue coalesce without a
+// transpose.
+//   store   out[n][m] (K slices side by side; the consumer sums them in order)
+//   Adam    the tile is the gradient of W[n][m]: the moments, the parameters, the BF16 copy and its
+//           transpose (the operand of the next backward pass) are updated here, so the gradient never
+//           goes to memory.  Bound by that traffic: 28 bytes a parameter, 1.06 GB for the output layer
+//           of 36,864 orientations (159 us at the copy bandwidth).
+#include "train_gemm.cuh"
+#include "tc_ptx.cuh"
+#include <algorithm>
+
+namespace t2b {
+namespace {
+
+constexpr int TG_TM = 128, TG_TN = 128, TG_TK = 64, TG_EPI_WARPS = 16, TG_THREADS = 32 * (2 + TG_EPI_WARPS);
+constexpr uint32_t TG_A_BYTES = TG_TM * TG_TK * 2, TG_B_BYTES = TG_TN * TG_TK * 2;
+constexpr uint32_t TG_TMEM = 512;   // two buffers of a leading and a correction accumulator
+enum { TG_STORE = 0, TG_ADAM = 1 };
+
+struct TgParams {
+    CUtensorMap a, b;
+    int a_rows, b_rows;       // rows of one part
+    int M, N, kblocks;
+    int m_tiles, n_tiles, ksplit;
+    float* out;
+    int ldo;
+    TgAdam w;
+    int* err;
+};
+
+constexpr int tg_stages(int na) { return na == 1 ? 3 : 2; }
+constexpr size_t tg_smem(int na, int nb)
+{
+    return (size_t)tg_stages(na) * (na * TG_A_BYTES + nb * TG_B_BYTES) + 1024;
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// One lane's 32 gradients of W[n0 .. n0 + 31][m]: four columns at a time, the next four loaded before
+// these are worked on, so that a warp always has 12 to 24 loads in flight
+__device__ __forceinline__ void adam_tile(const TgAdam& w, const float* acc, int m, int n0, int N)
+{
+    struct State {
+        float th[4], m[4], v[4];
+    } st[2];
+    const int last = N - 1;
+    const auto load = [&](State& s, int c) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const size_t i = (size_t)min(n0 + c + e, last) * w.ld + m;
+            s.th[e] = w.th[i];
+            s.m[e] = w.m[i];
+            s.v[e] = w.v[i];
+        }
+    };
+    load(st[0], 0);
+    __align__(16) __nv_bfloat16 tb[8];
+#pragma unroll
+    for (int c = 0; c < 32; c += 4) {
+        State& s = st[(c >> 2) & 1];
+        if (c + 4 < 32) load(st[((c >> 2) + 1) & 1], c + 4);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            adam_update(s.th[e], s.m[e], s.v[e], acc[c + e], w.step);
+            const __nv_bfloat16 t = __float2bfloat16_rn(s.th[e]);
+            tb[(c & 4) + e] = t;
+            if (n0 + c + e < N) {
+                const size_t i = (size_t)(n0 + c + e) * w.ld + m;
+                w.m[i] = s.m[e];
+                w.v[i] = s.v[e];
+                w.th[i] = s.th[e];
+                static_cast<__nv_bfloat16*>(w.thb)[i] = t;
+            }
+        }
+        if ((c & 4) == 4) {
+            // transposed copy: 8 consecutive n of this lane's m (ldt a multiple of 8)
+            const int nb = n0 + c - 4;
+            __nv_bfloat16* tt = static_cast<__nv_bfloat16*>(w.tht) + (size_t)m * w.ldt + nb;
+            if (nb + 8 <= N) {
+                *reinterpret_cast<uint4*>(tt) = *reinterpret_cast<const uint4*>(tb);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    if (nb + e < N) tt[e] = tb[e];
+            }
+        }
+    }
+}
+
+// NA, NB: parts of the operands
+template <int NA, int NB, int EPI>
+__global__ void __launch_bounds__(TG_THREADS, 1) k_train_gemm(const __grid_constant__ TgParams p)
+{
+    constexpr int NST = tg_stages(NA);
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t full_bar[NST], empty_bar[NST], tfull_bar[2], tempty_bar[2], drain_bar;
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ volatile int abort_flag;
+    constexpr uint32_t SBYTES = NA * TG_A_BYTES + NB * TG_B_BYTES;
+    // D f32, A/B bf16, both K-major, M = 128, N = 128
+    constexpr uint32_t IDESC =
+        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TG_TN >> 3) << 17) | ((uint32_t)(TG_TM >> 4) << 24);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t base = (su32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* gbase = smem_raw + (base - su32(smem_raw));
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NST; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+        for (int s = 0; s < 2; s++) { mbar_init(&tfull_bar[s], 1); mbar_init(&tempty_bar[s], TG_EPI_WARPS); }
+        mbar_init(&drain_bar, 1);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&tmem_base_slot)),
+                     "r"(TG_TMEM));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_slot;
+    const int ksp = p.ksplit, ntiles = p.m_tiles * p.n_tiles * ksp;
+    const int kper = (p.kblocks + ksp - 1) / ksp;
+
+    if (warp == 0 && lane == 0) {
+        // ---------------- TMA producer
+        int it = 0;
+        int issued[NST] = {};
+        uint32_t last_par[NST] = {};
+        for (int tile = blockIdx.x; tile < ntiles && !abort_flag; tile += gridDim.x) {
+            const int mn = tile / ksp, kb0 = (tile % ksp) * kper, kb1 = min(p.kblocks, kb0 + kper);
+            const int ya = (mn % p.m_tiles) * TG_TM, yb = (mn / p.m_tiles) * TG_TN;
+            for (int kb = kb0; kb < kb1; kb++, it++) {
+                const int s = it % NST;
+                const uint32_t ph = (uint32_t)(it / NST) & 1u;
+                if (!mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag)) { abort_flag = 1; break; }
+                uint8_t* st = gbase + s * SBYTES;
+                mbar_expect_tx(&full_bar[s], SBYTES);
+#pragma unroll
+                for (int i = 0; i < NA; i++) tma_load(st + i * TG_A_BYTES, &p.a, &full_bar[s], kb * TG_TK, i * p.a_rows + ya);
+#pragma unroll
+                for (int i = 0; i < NB; i++)
+                    tma_load(st + NA * TG_A_BYTES + i * TG_B_BYTES, &p.b, &full_bar[s], kb * TG_TK, i * p.b_rows + yb);
+                issued[s] = 1;
+                last_par[s] = ph;
+            }
+        }
+        if (abort_flag) {
+            // let the copies already in flight land before the CTA exits
+            volatile int never = 0;
+            for (int s = 0; s < NST; s++)
+                if (issued[s]) mbar_wait(&full_bar[s], last_par[s], &never);
+        }
+    } else if (warp == 1 && lane == 0) {
+        // ---------------- MMA issuer: K block `it` into buffer it & 1
+        int it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < ntiles && !abort_flag; tile += gridDim.x) {
+            const int kb0 = (tile % ksp) * kper, kb1 = min(p.kblocks, kb0 + kper);
+            for (int kb = kb0; kb < kb1; kb++, it++) {
+                const int s = it % NST, buf = it & 1;
+                if (!mbar_wait(&tempty_bar[buf], ((uint32_t)(it >> 1) & 1u) ^ 1u, &abort_flag) ||
+                    !mbar_wait(&full_bar[s], (uint32_t)(it / NST) & 1u, &abort_flag)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t sa = base + s * SBYTES, sb = sa + NA * TG_A_BYTES;
+                const uint32_t lead = tmem + (uint32_t)(buf * 2 * TG_TN), corr = lead + TG_TN;
+#pragma unroll
+                for (int k = 0; k < TG_TK / 16; k++) {
+                    const uint64_t ko = (uint64_t)(k * 32) >> 4;   // 32 bytes per K = 16 step
+                    umma(lead, sdesc(sa) + ko, sdesc(sb) + ko, IDESC, k != 0);
+#pragma unroll
+                    for (int i = 0; i < NA; i++)
+#pragma unroll
+                        for (int j = 0; j < NB; j++) {
+                            if (i + j == 0 || (NA == 3 && i + j > 2)) continue;   // beyond: below 2^-24 of the product
+                            umma(corr, sdesc(sa + i * TG_A_BYTES) + ko, sdesc(sb + j * TG_B_BYTES) + ko, IDESC,
+                                 k != 0 || !(i == 0 && j == 1));
+                        }
+                }
+                umma_commit(&empty_bar[s]);
+                umma_commit(&tfull_bar[buf]);
+            }
+        }
+        if (!ok) abort_flag = 1;
+        // drain: every MMA issued by this thread has retired before TMEM is freed
+        umma_commit(&drain_bar);
+        volatile int never = 0;
+        mbar_wait(&drain_bar, 0, &never);
+    } else if (warp >= 2) {
+        // ---------------- epilogue
+        const int q = warp & 3, part = (warp - 2) >> 2;   // TMEM lane quarter, 32 columns
+        int it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < ntiles && !abort_flag; tile += gridDim.x) {
+            const int mn = tile / ksp, kb0 = (tile % ksp) * kper, kb1 = min(p.kblocks, kb0 + kper);
+            const int m = (mn % p.m_tiles) * TG_TM + q * 32 + lane;
+            const int n0 = (mn / p.m_tiles) * TG_TN + part * 32;
+            if (EPI == TG_ADAM && n0 + lane < p.N && m - lane < p.M) {
+                // the state that this warp updates at the end, a line a lane, on its way to L2 meanwhile
+                const size_t i = (size_t)(n0 + lane) * p.w.ld + (m - lane);
+                for (const float* x : {p.w.th + i, p.w.m + i, p.w.v + i})
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(x));
+            }
+            float acc[32];
+#pragma unroll
+            for (int e = 0; e < 32; e++) acc[e] = 0.f;
+            for (int kb = kb0; kb < kb1; kb++, it++) {
+                const int buf = it & 1;
+                if (!mbar_wait(&tfull_bar[buf], (uint32_t)(it >> 1) & 1u, &abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 2 * TG_TN + part * 32);
+#pragma unroll
+                for (int c = 0; c < 32; c += 16) {
+                    uint32_t hi[16], lo[16];
+                    tmem_ld16(ta + c, hi);
+                    tmem_ld16(ta + TG_TN + c, lo);
+#pragma unroll
+                    for (int e = 0; e < 16; e++) acc[c + e] += __uint_as_float(hi[e]) + __uint_as_float(lo[e]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+            }
+            if (!ok) { abort_flag = 1; break; }
+            if (m < p.M) {
+                if (EPI == TG_STORE) {
+                    float* out = p.out + ((size_t)(tile % ksp) * p.N + n0) * p.ldo + m;
+#pragma unroll
+                    for (int e = 0; e < 32; e++)
+                        if (n0 + e < p.N) out[(size_t)e * p.ldo] = acc[e];
+                } else if (n0 < p.N) {
+                    adam_tile(p.w, acc, m, n0, p.N);
+                }
+            }
+            __syncwarp();   // the next tile's TMEM loads take the whole warp
+        }
+    }
+    __syncthreads();
+    if (abort_flag && threadIdx.x == 0) atomicExch(p.err, T2B_ERR_TIMEOUT);
+    tc_fence_after();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TG_TMEM));
+}
+
+template <int NA, int NB, int EPI>
+void launch(const TgParams& p, cudaStream_t st)
+{
+    const auto kern = k_train_gemm<NA, NB, EPI>;
+    const size_t smem = tg_smem(NA, NB);
+    T2B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int dev = 0, sms = 0;
+    T2B_CUDA(cudaGetDevice(&dev));
+    T2B_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    kern<<<std::min(sms, p.m_tiles * p.n_tiles * p.ksplit), TG_THREADS, smem, st>>>(p);
+    T2B_CUDA(cudaGetLastError());
+}
+
+// tiles, operands and K blocks of a product
+TgParams shape(const TgOperand& a, const TgOperand& b, int M, int N, int K, int ksplit, int* err)
+{
+    TgParams p{};
+    p.a = a.map;
+    p.b = b.map;
+    p.a_rows = a.rows;
+    p.b_rows = b.rows;
+    p.M = M;
+    p.N = N;
+    p.kblocks = (K + TG_TK - 1) / TG_TK;
+    p.m_tiles = (M + TG_TM - 1) / TG_TM;
+    p.n_tiles = (N + TG_TN - 1) / TG_TN;
+    const int kper = (p.kblocks + std::max(1, ksplit) - 1) / std::max(1, ksplit);
+    p.ksplit = (p.kblocks + kper - 1) / kper;   // no empty slice
+    p.err = err;
+    return p;
+}
+
+}  // namespace
+
+TgOperand tg_operand(void* ptr, int parts, int rows, int K, int ld)
+{
+    T2B_REQUIRE(ld % 8 == 0 && ld >= K, T2B_ERR_STATE, "training operand stride");
+    TgOperand o;
+    o.map = make_map(ptr, parts * rows, K, 128, ld);
+    o.rows = rows;
+    return o;
+}
+
+int tg_tiles(int M, int N) { return (M + TG_TM - 1) / TG_TM * ((N + TG_TN - 1) / TG_TN); }
+
+int tg_product(const TgOperand& a, const TgOperand& b, bool weights, int M, int N, int K, float* out, int ldo, int ksplit,
+               int* err, cudaStream_t st)
+{
+    TgParams p = shape(a, b, M, N, K, ksplit, err);
+    p.out = out;
+    p.ldo = ldo;
+    if (weights) launch<1, 3, TG_STORE>(p, st);
+    else launch<3, 3, TG_STORE>(p, st);
+    return p.ksplit;
+}
+
+void tg_gradient_adam(const TgOperand& a, const TgOperand& b, int M, int N, int K, const TgAdam& w, int* err,
+                      cudaStream_t st)
+{
+    T2B_REQUIRE(w.ldt % 8 == 0, T2B_ERR_STATE, "transposed weight stride");
+    TgParams p = shape(a, b, M, N, K, 1, err);
+    p.w = w;
+    launch<3, 3, TG_ADAM>(p, st);
+}
+
+}  // namespace t2b

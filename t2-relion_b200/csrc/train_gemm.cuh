@@ -1,0 +1,46 @@
+// Tensor-core products of the proposal network's training (train_gemm.cu).
+#pragma once
+#include "t2b_internal.cuh"
+#include <cuda.h>
+
+namespace t2b {
+
+// A row-major BF16 operand of `parts` matrices of rows x K, one after the other: one part for the
+// weights (BF16 already), three for an FP32 matrix split into x = p0 + p1 + p2 (24 bits)
+struct TgOperand {
+    CUtensorMap map;
+    int rows = 0;   // of one part
+};
+TgOperand tg_operand(void* ptr, int parts, int rows, int K, int ld);
+// tiles of an M x N product (one CTA each and K slice)
+int tg_tiles(int M, int N);
+
+// One Adam step (bias-corrected): rate lr / c1 and 1 / c2 with c = 1 - beta^t, formed on the host
+struct AdamStep {
+    float rate, ic2;
+};
+__device__ __forceinline__ void adam_update(float& th, float& m, float& v, float g, AdamStep s)
+{
+    m = 0.9f * m + 0.1f * g;
+    v = 0.999f * v + 0.001f * g * g;
+    th -= s.rate * m / (sqrtf(v * s.ic2) + 1e-8f);
+}
+
+// Adam state of one weight matrix W[n][m] (row length ld): parameters, moments, the BF16 copy and its
+// transpose WT[m][n] (row length ldt)
+struct TgAdam {
+    float *th, *m, *v;
+    void *thb, *tht;
+    int ld, ldt;
+    AdamStep step;
+};
+
+// out[n * ldo + m] = sum_k A[m][k] B[n][k]; A the weights (weights = true: A one part, B three) or both split.
+// K in up to `ksplit` slices, slice s at out + s * N * ldo (to be summed in order); returns their number.
+int tg_product(const TgOperand& a, const TgOperand& b, bool weights, int M, int N, int K, float* out, int ldo, int ksplit,
+               int* err, cudaStream_t st);
+// the same sum (both split) as the gradient of W[n][m]: one Adam step of W in the epilogue
+void tg_gradient_adam(const TgOperand& a, const TgOperand& b, int M, int N, int K, const TgAdam& w, int* err,
+                      cudaStream_t st);
+
+}  // namespace t2b

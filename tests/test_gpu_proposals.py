@@ -74,6 +74,40 @@ def test_gradient_matches_oracle(o2):
         assert err <= 1e-4, (name, err)
 
 
+@pytest.mark.parametrize("n", [1, 17, 128, 129, 300], ids=lambda n: f"n{n}")
+def test_gradient_products_at_tile_edges(o2, n):
+    """The training products (three BF16 parts of an FP32 operand on the tensor cores) at minibatches around
+    their tiles: 1 and 17 rows, 128 and 129 (column tiles of 128, then of 256), 300 (two column tiles, a
+    ragged K block in the weight gradients), against the FP64 oracle.  Bound: FP32 sums of up to 2048 terms
+    of one size differ from 64 bits by about sqrt(2048) 2^-24 = 3e-6 of their norm, through three layers;
+    images with an activation within rounding of zero (where a ReLU's gradient is rounding's choice) are left out."""
+    es, KO = o2["es"], _KO(o2)
+    L, th = _random_params(KO, 11)
+    es.proposal_params(set_to=th)
+    rng = np.random.default_rng(n)
+    imgs = rng.normal(size=(2 * n + 8, 256)).astype(np.float32)
+    _, c = po.forward(th, imgs, KO)
+    z1 = po._conv(c["x"], c["p"]["wc1"], c["p"]["bc1"], 1)[0]
+    z2 = po._conv(c["a1"], c["p"]["wc2"], c["p"]["bc2"], 2)[0]
+    z3 = c["x0"] @ c["p"]["w1"].T + c["p"]["b1"]
+    z4 = c["h1"] @ c["p"]["w2"].T + c["p"]["b2"]
+    near = np.any([np.abs(z).reshape(len(imgs), -1).min(1) < 2e-5 * z.std() for z in (z1, z2, z3, z4)], axis=0)
+    imgs = np.ascontiguousarray(imgs[~near][:n])
+    assert len(imgs) == n
+    to = np.full((n, 9), -1, np.int32)
+    tw = np.zeros((n, 9), np.float32)
+    to[:, :3] = rng.integers(0, KO, (n, 3))
+    tw[:, :3] = [0.5, 0.3, 0.2]
+    skip = np.zeros(KO, bool)
+    loss, g = es.proposal_grad(imgs, to, tw)
+    rloss, rg = po.loss_grad(th, imgs, to, tw, skip, KO)
+    assert loss == pytest.approx(rloss, rel=1e-6)
+    for name, size in (("wc1", 144), ("wc2", 4608), ("w1", 1024 * 2048), ("b1", 1024), ("w2", 1024 * 1024),
+                       ("b2", 1024), ("w3", KO * 1024), ("b3", KO)):
+        a, b = g[L[name]:L[name] + size], rg[L[name]:L[name] + size]
+        assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b), name
+
+
 def test_tensor_core_logits_match_oracle(o2):
     """Inference path (tcgen05, BF16 activations) vs the FP64 forward pass."""
     es, KO = o2["es"], _KO(o2)
