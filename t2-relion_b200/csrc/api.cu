@@ -466,6 +466,9 @@ int t2b_configure(t2b_ctx* c, const t2b_config* cfg)
         w.pair_off = dalloc<long long>(c, B + 1);
         w.max_chunks = (int)((KOT + 4095) / 4096);
         w.chunk_cnt = dalloc<int>(c, (size_t)B * w.max_chunks);
+        // (proposals: up to 128 x T hypotheses a particle)
+        w.max_dchunks = (int)((std::max<long long>(KOT, 128LL * T) + 511) / 512);
+        w.cmin = dalloc<float>(c, (size_t)B * w.max_dchunks);
         w.d2f = dalloc<float>(c, (size_t)w.pair_cap * R * V);
         w.wf = dalloc<double>(c, (size_t)w.pair_cap * R * V);
         w.groups = dalloc<long long>(c, w.pair_cap);

@@ -158,6 +158,8 @@ struct Work {
     long long pair_cap;
     int* chunk_cnt;           // n x max_chunks
     int max_chunks;
+    float* cmin;              // n x max_dchunks: smallest coarse diff2 of each 512 hypotheses
+    int max_dchunks;
     float* d2f;               // pair_cap * R*V
     double* wf;               // pair_cap * R*V (final weights when ovs; coarse gathered otherwise)
     long long* groups;        // pair_cap: first pair of each orientation group
