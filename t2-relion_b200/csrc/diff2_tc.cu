@@ -623,10 +623,12 @@ bool tc_supported() { return true; }
 size_t tc_kdim(int nk) { return (size_t)((2 * nk + TK - 1) / TK) * TK; }
 size_t tc_kn(int nk) { return (size_t)((nk + TK - 1) / TK) * TK; }
 
-// descriptor slots in op.maps (TC_MAP_SLOTS of 128 bytes)
+// descriptor slots in op.maps (TC_MAP_SLOTS of 128 bytes).  The image and w2 operands have one pair for each
+// box height below 256: MAP_IHN + 2 (rows / 32 - 1) and MAP_WHN + 2 (rows / 32 - 1).
+constexpr int BOXES = TN / 32 - 1;
 enum { MAP_PH = 0, MAP_PL, MAP_IH, MAP_IL, MAP_NH, MAP_NL, MAP_WH, MAP_WL,
        MAP_IAH, MAP_IAL, MAP_RAH, MAP_RAL, MAP_RBH, MAP_RBL,
-       MAP_IH128, MAP_IL128, MAP_WAH, MAP_WAL, MAP_IAH_N, MAP_IAL_N, MAP_COUNT };
+       MAP_WAH, MAP_WAL, MAP_IAH_N, MAP_IAL_N, MAP_IHN, MAP_WHN = MAP_IHN + 2 * BOXES, MAP_COUNT = MAP_WHN + 2 * BOXES };
 static_assert(MAP_COUNT <= TC_MAP_SLOTS, "tensor-map slots");
 static_assert(sizeof(CUtensorMap) == 128, "tensor-map size");
 
@@ -650,10 +652,16 @@ void tc_prepare_projections(const Tables& tb, TcOperands& op, cudaStream_t st)
     h[MAP_WL] = make_map(op.wl, op.b_pad, op.kn, TN);
     T2B_CUDA(cudaStreamSynchronize(st));
     T2B_CUDA(cudaMemcpy(op.maps, h, sizeof(h), cudaMemcpyHostToDevice));  // slots MAP_PH..MAP_WL
-    // and with a 128-row box: dense coarse tiles of 128 columns (t2b_autotune)
-    CUtensorMap h128[2] = {make_map(op.ah, op.n_pad, op.kdim, 128), make_map(op.al, op.n_pad, op.kdim, 128)};
-    T2B_CUDA(cudaMemcpy(static_cast<unsigned char*>(op.maps) + 128 * MAP_IH128, h128, sizeof(h128),
-                        cudaMemcpyHostToDevice));
+    // and with the lower boxes of narrow column tiles
+    CUtensorMap nar[4 * BOXES];
+    for (int i = 0; i < BOXES; i++) {
+        const int box = 32 * (i + 1);
+        nar[2 * i] = make_map(op.ah, op.n_pad, op.kdim, box);
+        nar[2 * i + 1] = make_map(op.al, op.n_pad, op.kdim, box);
+        nar[2 * BOXES + 2 * i] = make_map(op.wh, op.b_pad, op.kn, box);
+        nar[2 * BOXES + 2 * i + 1] = make_map(op.wl, op.b_pad, op.kn, box);
+    }
+    T2B_CUDA(cudaMemcpy(static_cast<unsigned char*>(op.maps) + 128 * MAP_IHN, nar, sizeof(nar), cudaMemcpyHostToDevice));
     const int rows = op.chunk > 0 ? op.chunk : tb.K * tb.O;
     // sizes were fixed when the operand buffers were allocated
     T2B_REQUIRE(op.m_pad == (rows + TM - 1) / TM * TM && op.kdim == (int)tc_kdim(tb.nk), T2B_ERR_STATE,
@@ -703,6 +711,16 @@ static void launch_gemm(const TcOperands& op, int ia, int ib, TcParams& p, cudaS
     T2B_CUDA(cudaGetLastError());
 }
 
+// Column tiles of `cols` columns: the fewest of at most 256, each narrowed to a multiple of 32, so that little
+// of the contraction goes into padding (32 particles x 49 shifts: 7 tiles of 224 columns, not of
+// 256; one particle x 29: one of 32).  Batches of 21 and 16 particles at boxes 176 and 220 in chunks of 1,000
+// orientations took 8.96 and 9.02 ms at 256, 6.48 and 6.52 so.
+static void column_tiles(int cols, int& n_tiles, int& tn)
+{
+    n_tiles = (cols + TN - 1) / TN;
+    tn = ((cols + n_tiles - 1) / n_tiles + 31) / 32 * 32;
+}
+
 // N[b][oc] = sum_p w2[b][p] |P_oc[p]|^2 with the same split-BF16 tensor-core kernel
 void tc_launch_norms(const Tables& tb, const Work& w, TcOperands& op, cudaStream_t st, const int* gate, int gate_run,
                      RowChunk ch, bool split_w2)
@@ -716,7 +734,9 @@ void tc_launch_norms(const Tables& tb, const Work& w, TcOperands& op, cudaStream
     }
     TcParams p{};
     p.m_tiles = ch.rows ? (ch.rows + TM - 1) / TM : op.m_pad / TM;
-    p.n_tiles = b_pad / TN;
+    int tn = TN;
+    column_tiles(w.n, p.n_tiles, tn);
+    p.tn = tn == TN ? 0 : tn;
     p.kblocks = op.kn / TK;
     p.raw = 1;
     p.KO = ch.rows ? ch.rows : tb.K * tb.O;
@@ -731,7 +751,7 @@ void tc_launch_norms(const Tables& tb, const Work& w, TcOperands& op, cudaStream
     p.products = 3;
     p.gate = gate;
     p.gate_run = gate_run;
-    launch_gemm(op, MAP_NH, MAP_WH, p, st);
+    launch_gemm(op, MAP_NH, tn == TN ? (int)MAP_WH : MAP_WHN + 2 * (tn / 32 - 1), p, st);
 }
 
 void tc_split_images(const Tables& tb, const Work& w, TcOperands& op, cudaStream_t st, const int* gate)
@@ -764,8 +784,10 @@ void tc_launch_diff2(const Tables& tb, const Work& w, TcOperands& op, cudaStream
     TcParams p{};
     p.raw = 0;
     p.m_tiles = ch.rows ? (ch.rows + TM - 1) / TM : op.m_pad / TM;
-    p.n_tiles = (ncols + op.dense_tn - 1) / op.dense_tn;
-    p.tn = op.dense_tn == TN ? 0 : op.dense_tn;
+    int tn = op.dense_tn;
+    if (tn == TN) column_tiles(ncols, p.n_tiles, tn);
+    else p.n_tiles = (ncols + tn - 1) / tn;
+    p.tn = tn == TN ? 0 : tn;
     p.group = op.group_m;
     p.kblocks = op.kdim / TK;
     p.KO = ch.rows ? ch.rows : tb.K * tb.O;
@@ -782,7 +804,7 @@ void tc_launch_diff2(const Tables& tb, const Work& w, TcOperands& op, cudaStream
     p.products = 3;
     p.gate = gate;
     p.gate_run = gate_run;
-    launch_gemm(op, MAP_PH, op.dense_tn == TN ? MAP_IH : MAP_IH128, p, st);
+    launch_gemm(op, MAP_PH, tn == TN ? (int)MAP_IH : MAP_IHN + 2 * (tn / 32 - 1), p, st);
 }
 
 void tc_set_map(TcOperands& op, int slot, void* ptr, int rows, int kdim, bool a_side)
@@ -921,16 +943,10 @@ void tc_launch_audit_norms(const Tables& tb, TcOperands& op, int na_max, float* 
 // batch of fewer audited particles runs the narrower variant (na_max - 1 slots,
 // MAP_IAH_N/IAL_N) when its tiles cover fewer columns, a batch of na_max the full one;
 // each launch returns at once unless the count is its own.
-static void audit_shape(int cols, int& n_tiles, int& tn)
-{
-    n_tiles = (cols + TN - 1) / TN;
-    tn = ((cols + n_tiles - 1) / n_tiles + 31) / 32 * 32;
-}
-
 int tc_audit_tn(int na, int T)
 {
     int nt, tn;
-    audit_shape(na * T, nt, tn);
+    column_tiles(na * T, nt, tn);
     return tn;
 }
 
@@ -938,8 +954,8 @@ int tc_audit_narrow_tn(int na_max, int T)
 {
     if (na_max < 2) return 0;
     int nf, tf, nn, tnn;
-    audit_shape(na_max * T, nf, tf);
-    audit_shape((na_max - 1) * T, nn, tnn);
+    column_tiles(na_max * T, nf, tf);
+    column_tiles((na_max - 1) * T, nn, tnn);
     return nn * tnn < nf * tf ? tnn : 0;
 }
 
@@ -949,7 +965,7 @@ void tc_launch_audit(const Tables& tb, TcOperands& op, int na_max, const int* na
     TcParams p{};
     int tf = TN;
     p.m_tiles = op.m_pad / TM;
-    audit_shape(na_max * tb.T, p.n_tiles, tf);
+    column_tiles(na_max * tb.T, p.n_tiles, tf);
     p.tn = tf == TN ? 0 : tf;
     p.kblocks = op.kdim / TK;
     p.KO = tb.K * tb.O;
@@ -967,7 +983,7 @@ void tc_launch_audit(const Tables& tb, TcOperands& op, int na_max, const int* na
     if (tn_n > 0 && na) {
         TcParams q = p;
         int tq = TN;
-        audit_shape((na_max - 1) * tb.T, q.n_tiles, tq);
+        column_tiles((na_max - 1) * tb.T, q.n_tiles, tq);
         q.ncols = (na_max - 1) * tb.T;
         q.tn = tq == TN ? 0 : tq;
         q.cnt = na;

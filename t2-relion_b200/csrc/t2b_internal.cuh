@@ -232,7 +232,7 @@ struct TcOperands {
 struct RowChunk {
     int row0 = 0, rows = 0;   // rows == 0: every row (the resident operands)
 };
-constexpr int TC_MAP_SLOTS = 24;
+constexpr int TC_MAP_SLOTS = 48;
 size_t tc_kdim(int nk);
 void tc_prepare_projections(const Tables& tb, TcOperands& op, cudaStream_t st);
 // resident tables: split rows [0, rows) of tb.proj_c into the projection operands
