@@ -1228,7 +1228,10 @@ def main():
     # the contraction runs over the nk window pixels inside the projection radius only
     # (projections are zero outside); "executed" counts what the tensor cores did
     nk = int(sum(1 for n in range(P) if (lambda i, x: x * x + (i if i < s // 2 + 1 else i - s) ** 2)(n // (s // 2 + 1), n % (s // 2 + 1)) <= (s // 2) ** 2))
-    kdim = (2 * nk + 63) // 64 * 64
+    # split-BF16: orientations half a turn apart in plane share their products (an even number of angles): half
+    # the rows, the real and imaginary parts in 64-wide blocks
+    pair = 2 if mode == t2b.DIFF2_SPLIT_BF16 and samp["n_psi"] % 2 == 0 else 1
+    kdim = 2 * ((nk + 63) // 64 * 64) if pair == 2 else (2 * nk + 63) // 64 * 64
     if learned is None:
         flops = 8.0 * K * O * T * P * B
         gemm = float(stages[2])
@@ -1240,7 +1243,7 @@ def main():
             bound = "fp32_simt"
             src, peak_kind = "nominal", "FP32 FMA nominal"
         achieved = flops / (gemm / 1000.0) / 1e12
-        executed = (12.0 if mode == t2b.DIFF2_SPLIT_BF16 else 4.0) * K * O * T * nk * B / (gemm / 1000.0) / 1e12
+        executed = (12.0 if mode == t2b.DIFF2_SPLIT_BF16 else 4.0) / pair * K * O * T * nk * B / (gemm / 1000.0) / 1e12
         traffic = None   # no capture of the dense pass of this kernel source
         roof = {"bound": bound, "kernel": "k_diff2_tc" if mode else "k_diff2_simt", "achieved": achieved,
                 "executed_tflops": executed, "contraction_pixels": nk,
@@ -1271,7 +1274,7 @@ def main():
             if na == 0:
                 return 0.0
             nt, tn = narrow if (na < na_max and narrow[0] * narrow[1] < full[0] * full[1]) else full
-            return ((K * O + 127) // 128) * nt * tn
+            return ((K * O // pair + 127) // 128) * nt * tn
         # proposal tiles: 128 rows of 128 / kslot particles x T phase rows padded to 32 columns
         ppt = 2 if PROP["topk"] <= 64 else 1
         prop_exec = ((B + ppt - 1) // ppt) * 128 * ((T + 31) // 32 * 32) * kdim * 2 * 3.0

@@ -114,7 +114,8 @@ typedef struct t2b_config {
                                   (built once here) when the coarse and fine tables and their
                                   split-BF16 operands fit in 60 % of the free device memory,
                                   else chunks of 16384; > 0: chunks of this many rows (at most
-                                  nr_classes * n_dir * n_psi).  Chunked: split-BF16 contraction
+                                  nr_classes * n_dir * n_psi; a row serves two orientations
+                                  half a turn apart in plane where the sampling has both).  Chunked: split-BF16 contraction
                                   only, the fine pass and the weighted sums interpolate their
                                   projections from the models on the fly (the same FP64
                                   interpolation, so the same values), no learned proposals.

@@ -361,7 +361,7 @@ int t2b_configure(t2b_ctx* c, const t2b_config* cfg)
         // resident projection tables, or one chunk of the coarse orientations per batch step
         int chunk = 0;
         {
-            const double kd = (double)tc_kdim(tb.nk), kn = (double)tc_kn(tb.nk);
+            const double kd = (double)tc_kdim(tb.nk, 0), kn = (double)tc_kn(tb.nk);
             const double resident = (double)KO * P * 8. * (1 + (tb.ovs ? R : 0)) +
                                     (f.diff2_mode == T2B_DIFF2_SPLIT_BF16 ? (double)KO * (kd + kn) * 4. : 0.);
             size_t fr = 0, tot = 0;
@@ -376,6 +376,22 @@ int t2b_configure(t2b_ctx* c, const t2b_config* cfg)
                     "projection tables do not fit (or orientation_chunk was set): the chunked coarse pass "
                     "runs on the split-BF16 contraction only");
         tb.chunk = chunk;
+        // Orientations half a turn apart in plane share an operand row where the sampling has all of them
+        // (any even number of psi steps over the full turn) and the models are transforms of real maps
+        // (x = 0 planes Hermitian), checked here; their two products then cost one, and a chunk's
+        // projections serve both.  (Not the plain FP32 contraction, whose sums keep their order.)
+        tb.half = 0;
+        if (f.diff2_mode == T2B_DIFF2_SPLIT_BF16 && f.n_psi % 2 == 0) {
+            const int half = f.n_psi / 2;
+            bool paired = true;
+            for (int o = 0; paired && o < O; o++) {
+                if (o % f.n_psi >= half) continue;
+                const double *a = f.eul_coarse + 9 * (size_t)o, *b = f.eul_coarse + 9 * (size_t)(o + half);
+                for (int i = 0; i < 6; i++) paired = paired && std::fabs(a[i] + b[i]) <= 1e-13;
+            }
+            for (int k = 0; paired && k < K; k++) paired = tc_planes_hermitian(c->mvol[k], c->mdl[k], st);
+            if (paired) tb.half = half;
+        }
         tb.eul_c = (const double*)up(f.eul_coarse, (size_t)O * 9 * sizeof(double));
         tb.trans_c = (const double*)up(f.trans_px, (size_t)T * 2 * sizeof(double));
         tb.trans_prior = (const double*)up(f.trans_prior, (size_t)T * 2 * sizeof(double));
@@ -542,9 +558,9 @@ int t2b_configure(t2b_ctx* c, const t2b_config* cfg)
         c->tc.group_m = c->tune.group_m;
         if (f.diff2_mode == T2B_DIFF2_SPLIT_BF16) {
             TcOperands& op = c->tc;
-            op.kdim = (int)tc_kdim(tb.nk);
-            op.chunk = chunk;
-            op.m_pad = (int)(((chunk ? chunk : KO) + 127) / 128 * 128);
+            op.kdim = (int)tc_kdim(tb.nk, tb.half);
+            op.chunk = chunk ? std::min(chunk, tb.half ? O / 2 : O) : 0;   // operand rows
+            op.m_pad = (int)(((chunk ? op.chunk : tb.half ? KO / 2 : KO) + 127) / 128 * 128);
             op.n_pad = (B * T + 255) / 256 * 256;
             op.bh = dalloc<uint16_t>(c, (size_t)op.m_pad * op.kdim);
             op.bl = dalloc<uint16_t>(c, (size_t)op.m_pad * op.kdim);
@@ -612,13 +628,14 @@ void enqueue_estep(t2b_ctx* c, Work& w, cudaStream_t st, bool stage_events, bool
         // chunked coarse pass: per chunk of one class's orientations, its projections, their
         // split-BF16 operands, the norms and the contraction into the batch's diff2 rows
         if (stage_events) cudaEventRecord(c->ev[2], st);
+        const int rows = tb.half ? tb.O / 2 : tb.O, step = tc_chunk_rows(c->tc, w.n * tb.T);
         bool first = true;
         for (int k = 0; k < tb.K; k++)
-            for (int o0 = 0; o0 < tb.O; o0 += tb.chunk) {
-                const int n = std::min(tb.chunk, tb.O - o0);
-                tc_project_split(tb, c->tc, c->mtex[k], c->mvol[k], tb.eul_c + 9 * (size_t)o0, n, st);
+            for (int h0 = 0; h0 < rows; h0 += step) {
+                const int n = std::min(step, rows - h0);
+                tc_project_split(tb, c->tc, c->mtex[k], c->mvol[k], tb.eul_c, h0, n, st);
                 RowChunk ch;
-                ch.row0 = k * tb.O + o0;
+                ch.row0 = k * rows + h0;
                 ch.rows = n;
                 tc_launch_norms(tb, w, c->tc, st, nullptr, 0, ch, first);
                 tc_launch_diff2(tb, w, c->tc, st, nullptr, 0, ch);

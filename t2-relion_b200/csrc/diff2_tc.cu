@@ -7,17 +7,23 @@
 //     C[oc][b*T+t] = sum_k Proj[oc][k] * Img[b*T+t][k]
 // Every FP32 operand x is split as hi = bf16(x), lo = bf16(x - hi), and
 //     C ~= Ph.Ih + Ph.Il + Pl.Ih      (the lo.lo term is below FP32 resolution)
-// The three products accumulate into one FP32 TMEM accumulator.
+// The three products accumulate into one FP32 TMEM accumulator; of paired orientations (pair_row), whose
+// products are the sum and the difference of the real and the imaginary parts' sums, into one for either.
 //
-// Kernel: persistent, one CTA per SM, 192 threads.
+// Kernel: persistent, one CTA per SM, 320 threads.
 //   warp 0      TMA producer: per 64-wide K block loads Ph, Pl (128 x 64) and
 //               Ih, Il (256 x 64) with 128-byte swizzle into a 2-stage ring
 //   warp 1      MMA issuer: 12 x tcgen05.mma (M128 N256 K16) per K block (4 per
-//               product; the network GEMMs use one product, BF16 x BF16) into a
-//               double-buffered 2 x 256-column TMEM accumulator
-//   warps 2-5   epilogue: tcgen05.ld 32x32b, transpose through shared memory,
-//               diff2 = c0 + norm - C written coalesced along t, per-particle
-//               minimum by shared + global atomics
+//               product; the network GEMMs use one product, BF16 x BF16) into
+//               512 TMEM columns: two tiles of 256, or one paired tile of 256
+//               (two of 128 or less)
+//   warps 2-9   epilogue, two warps a TMEM lane quarter: tcgen05.ld 32x32b, diff2 = c0 + norm - C
+//               rounded once, per-particle minimum by global atomics, transpose
+//               through shared memory, stores coalesced along t
+// 36,864 orientations x 64 particles x 81 shifts (K = 5,104): 4.14 ms a row per orientation (1.41 PFLOP/s),
+// 2.60 paired (1.13: a paired tile's epilogue has no second tile to hide behind; with four epilogue warps
+// that read their norms row by row it was 3.07).  Tiles of half the width would hide it, at a third more
+// shared-memory reads per product; t2b_autotune tries them.
 // Every mbarrier wait is bounded (2 s); on expiry the CTA records
 // T2B_ERR_TIMEOUT in a device flag, waits (bounded) for its own copies and
 // MMAs, frees TMEM and returns.
@@ -25,6 +31,7 @@
 #include "tc_ptx.cuh"
 #include "project_pixel.cuh"
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 namespace t2b {
@@ -40,10 +47,11 @@ constexpr int L2_AHEAD = T2B_L2_AHEAD;  // k-blocks between an A tile's L2 prefe
 constexpr uint32_t A_BYTES = TM * TK * 2;              // 16 KB
 constexpr uint32_t B_BYTES = TN * TK * 2;              // 32 KB
 constexpr uint32_t STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // 96 KB
-constexpr int NTHREADS = 192;
+constexpr int EPI_WARPS = 8, NTHREADS = 32 * (2 + EPI_WARPS);
 constexpr uint32_t TMEM_COLS = 512;
-constexpr int EPI_LD = 33;
-constexpr size_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 4 * 32 * EPI_LD * 4 + 4 * (TN + 2) * 4;
+constexpr size_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + EPI_WARPS * 32 * 32 * 4 + 4 * 2 * 4;
+// element (r, c) of an epilogue warp's 32 x 32 transpose buffer: rows and columns both on 32 banks
+__device__ __forceinline__ int epi_at(int r, int c) { return r * 32 + (c ^ r); }
 
 // instruction descriptor: D f32, A/B bf16, both K-major, M = 128; N (bits 17-22, N/8)
 // is set per launch (256, or 96 for one particle's translations)
@@ -76,7 +84,11 @@ struct TcParams {
     int ksplit;               // raw GEMMs: K split into this many slices (0/1: none); slice s writes
                               // its partial product at out + s * ncols * KO
     int raw;                  // 1: store the contraction itself (norm and network GEMMs), 0: diff2 epilogue
-    int KO, T, ncols;
+    int KO, T, ncols;         // (mode 0: KO operand rows)
+    int half;                 // mode 0: paired orientations (Tables::half).  A row's even k-blocks hold the real
+                              // parts and its odd ones the imaginary; their sums go to two accumulators,
+                              // whose sum is the first orientation's product and whose difference
+                              // the second's
     const float* c0;
     const float* norms;
     const unsigned char* skip;
@@ -151,12 +163,12 @@ k_diff2_tc(const CUtensorMap* __restrict__ maps, int ia, int ib, TcParams p)
     const int nst = min(MAXSTAGES, (int)((uint32_t)(STAGES * STAGE_BYTES) / sbytes));
     const uint32_t base = (su32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (base - su32(smem_raw));
-    float* epi = reinterpret_cast<float*>(gbase + STAGES * STAGE_BYTES);          // 4 x 32 x 33
-    unsigned* smin = reinterpret_cast<unsigned*>(epi + 4 * 32 * EPI_LD);          // 4 x (TN+2)
+    float* epi = reinterpret_cast<float*>(gbase + STAGES * STAGE_BYTES);          // EPI_WARPS x 32 x 32
+    unsigned* smin = reinterpret_cast<unsigned*>(epi + EPI_WARPS * 32 * 32);       // 4 x 2 (mode 1)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAXSTAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        for (int s = 0; s < 2; s++) { mbar_init(&tfull_bar[s], 1); mbar_init(&tempty_bar[s], 4); }
+        for (int s = 0; s < 2; s++) { mbar_init(&tfull_bar[s], 1); mbar_init(&tempty_bar[s], EPI_WARPS); }
         mbar_init(&drain_bar, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -173,6 +185,11 @@ k_diff2_tc(const CUtensorMap* __restrict__ maps, int ia, int ib, TcParams p)
     const int ksp = p.ksplit > 1 ? p.ksplit : 1;
     const int ntiles = p.m_tiles * p.n_tiles * ksp;
     const int kper = (p.kblocks + ksp - 1) / ksp;   // k-blocks per slice
+    // paired products take two accumulators a tile: 512 columns at 256, so one tile at a time
+    const bool two = p.half && !p.raw;
+    const int accw = tn_l <= TN / 2 ? TN / 2 : TN;           // columns of an accumulator
+    const int nbuf = two && accw == TN ? 1 : 2;              // tiles in TMEM
+    const uint32_t bufw = (uint32_t)(two ? 2 * accw : TN);   // columns of a tile
 
     if (warp == 0 && lane == 0) {
         // ---------------- TMA producer
@@ -248,11 +265,11 @@ k_diff2_tc(const CUtensorMap* __restrict__ maps, int ia, int ib, TcParams p)
         const uint32_t idesc = idesc_for(p.tn ? p.tn : TN);
         int it = 0, tl = 0;
         for (int tile = blockIdx.x; tile < ntiles && !abort_flag; tile += gridDim.x, tl++) {
-            const int abuf = tl & 1;
-            const uint32_t aph = (uint32_t)(tl >> 1) & 1u;
+            const int abuf = tl % nbuf;
+            const uint32_t aph = (uint32_t)(tl / nbuf) & 1u;
             if (!mbar_wait(&tempty_bar[abuf], aph ^ 1u, &abort_flag)) { abort_flag = 1; break; }
             tc_fence_after();
-            const uint32_t dt = tmem + (uint32_t)(abuf * TN);
+            const uint32_t dt0 = tmem + abuf * bufw;
             bool ok = true;
             const int kb0 = (tile % ksp) * kper, kb1 = min(p.kblocks, kb0 + kper);
             for (int kb = kb0; kb < kb1; kb++, it++) {
@@ -263,10 +280,12 @@ k_diff2_tc(const CUtensorMap* __restrict__ maps, int ia, int ib, TcParams p)
                 const uint32_t sa = base + s * sbytes;
                 const uint64_t dPh = sdesc(sa), dPl = sdesc(sa + A_BYTES);
                 const uint64_t dIh = sdesc(sa + a_st), dIl = sdesc(sa + a_st + bbytes);
+                const uint32_t dt = two && (kb & 1) ? dt0 + (uint32_t)accw : dt0;
+                const bool fresh = kb - kb0 < (two ? 2 : 1);   // the accumulator's first k-block
 #pragma unroll
                 for (int k = 0; k < TK / 16; k++) {
                     const uint64_t ko = (uint64_t)(k * 32) >> 4;  // 32 bytes per K=16 step
-                    umma(dt, dPh + ko, dIh + ko, idesc, (kb != kb0 || k != 0));
+                    umma(dt, dPh + ko, dIh + ko, idesc, (!fresh || k != 0));
                     if (p.products >= 2) umma(dt, dPh + ko, dIl + ko, idesc, 1);
                     if (p.products == 3) umma(dt, dPl + ko, dIh + ko, idesc, 1);
                 }
@@ -283,23 +302,46 @@ k_diff2_tc(const CUtensorMap* __restrict__ maps, int ia, int ib, TcParams p)
         // ---------------- epilogue (warps 2..5 -> TMEM lane quarters 2,3,0,1)
         const int q = warp & 3;
         const int ew = warp - 2;
-        float* sbuf = epi + ew * 32 * EPI_LD;
-        unsigned* wmin = smin + ew * (TN + 2);
+        const int grp = ew >> 2;   // of the two warps of a quarter: this one's chunks of 32 columns (modes 1, 2: the first's)
+        float* sbuf = epi + ew * 32 * 32;
+        unsigned* wmin = smin + (ew & 3) * 2;
         int tl = 0;
         for (int tile = blockIdx.x; tile < ntiles && !abort_flag; tile += gridDim.x, tl++) {
             int mt = 0, nt = 0;
             if (p.mode == 0) tile_coords(tile / ksp, p.m_tiles, p.n_tiles, p.group ? p.group : 16, mt, nt);
             float* const outp = p.d2c + (size_t)(tile % ksp) * p.ncols * p.KO * p.T;   // raw: the slice's partial
-            const int abuf = tl & 1;
-            const uint32_t aph = (uint32_t)(tl >> 1) & 1u;
+            const int abuf = tl % nbuf;
+            const uint32_t aph = (uint32_t)(tl / nbuf) & 1u;
+            // mode 0, diff2: this lane's row and the c0, norm of its next chunk's first two particles, fetched
+            // while the tile is still contracted
+            const size_t ks = p.ko_stride ? (size_t)p.ko_stride : (size_t)p.KO;
+            const bool dense = p.mode == 0 && !p.raw;
+            const int rl = mt * TM + q * 32 + lane;
+            const bool rok = dense && rl < p.KO;
+            const size_t og = rok ? (size_t)pair_row(p.row0 + rl, p.half) : 0;
+            const bool skipped = rok && p.skip[og];
+            float bc[2], bn[2];
+            const auto fetch = [&](int b0) {
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const bool in = rok && (b0 + i) * p.T < p.ncols;
+                    bc[i] = in ? p.c0[b0 + i] : 0.f;
+                    bn[i] = in ? p.norms[(size_t)(b0 + i) * ks + og] : 0.f;
+                }
+            };
+            if (dense) fetch((nt * tn_l + grp * 32) / p.T);
             if (!mbar_wait(&tfull_bar[abuf], aph, &abort_flag)) { abort_flag = 1; break; }
             tc_fence_after();
+            if (p.mode != 0 && grp != 0) {
+                if (lane == 0) mbar_arrive(&tempty_bar[abuf]);
+                continue;
+            }
             const int n0 = nt * tn_l;
             const int mtp = p.mtp ? p.mtp : 1;
             const int tt = tile / ksp;   // the m-tile (modes 1, 2)
             const int bfirst = p.mode == 0 ? n0 / p.T : (tt / mtp) * p.ppt;
             const int jbase = p.mode == 0 ? 0 : (tt % mtp) * TM;
-            for (int i = lane; i < TN + 2; i += 32) wmin[i] = 0xffffffffu;
+            if (p.mode == 1 && lane < 2) wmin[lane] = 0xffffffffu;
             // proposal tiles: the per-row data of the warp's 32 rows (orientation skip flag
             // and norm), one row per lane, broadcast by shuffles in the chunk loop below
             int my_skip = 1;
@@ -388,22 +430,95 @@ k_diff2_tc(const CUtensorMap* __restrict__ maps, int ia, int ib, TcParams p)
             // the TMEM lane is the row, which is the contiguous axis of the output, so each of
             // the 32 columns of a load is one coalesced 128-byte store, no transpose
             const bool raw_rows = p.mode == 0 && p.raw && p.T == 1;
-            const size_t ks = p.ko_stride ? (size_t)p.ko_stride : (size_t)p.KO;
             if (raw_rows) {
                 const int oc = mt * TM + q * 32 + lane;
-                for (int c = 0; c < nchunk; c++) {
+                const size_t og = (size_t)pair_row(p.row0 + oc, p.half);
+                for (int c = grp; c < nchunk; c += 2) {
                     uint32_t v[32];
                     tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(abuf * TN + c * 32), v);
                     if (oc < p.KO) {
 #pragma unroll
                         for (int e = 0; e < 32; e++) {
                             const int col = n0 + c * 32 + e;
-                            if (col < p.ncols) outp[(size_t)col * ks + p.row0 + oc] = __uint_as_float(v[e]);
+                            if (col < p.ncols) outp[(size_t)col * ks + og] = __uint_as_float(v[e]);
                         }
                     }
                 }
             }
-            for (int c = 0; c < (p.mode == 2 || !emit || raw_rows ? 0 : nchunk); c++) {
+            if (p.mode == 0 && !raw_rows) {
+                // diff2 in the TMEM layout (lane = row), then through shared memory to lane = column for
+                // coalesced stores
+                const unsigned rows = __ballot_sync(0xffffffffu, rok);
+                for (int c = grp; c < nchunk && n0 + c * 32 < p.ncols; c += 2) {
+                    const int col0 = n0 + c * 32;
+                    const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)abuf * bufw + (uint32_t)(c * 32);
+                    uint32_t v[32], u[32];
+                    tmem_ld32(ta, v);
+                    if (two) tmem_ld32(ta + (uint32_t)accw, u);
+                    const float fc[2] = {bc[0], bc[1]}, fn[2] = {bn[0], bn[1]};
+                    if (c + 2 < nchunk) fetch((col0 + 64) / p.T);
+                    // particle by particle; c0 + norm and its difference from the product keep their rounding
+                    // errors (two-sum), so that diff2 is rounded once
+                    const int b0 = col0 / p.T;
+                    for (int b = b0, lo = 0; lo < 32 && col0 + lo < p.ncols; b++) {
+                        const int hi = min(32, (b + 1) * p.T - col0);
+                        float x, y;
+                        if (b - b0 < 2) {
+                            x = b == b0 ? fc[0] : fc[1];
+                            y = b == b0 ? fn[0] : fn[1];
+                        } else {
+                            x = rok ? p.c0[b] : 0.f;
+                            y = rok ? p.norms[(size_t)b * ks + og] : 0.f;
+                        }
+                        const float base_d = x + y, yy = base_d - x, low = (x - (base_d - yy)) + (y - yy);
+                        const bool finite = fabsf(base_d) < INFINITY;
+                        const auto diff = [&](float cross) {
+                            const float t = base_d - cross;
+                            return finite ? t + (((base_d - t) - cross) + low) : t;
+                        };
+                        float least = __int_as_float(0x7fffffff);   // NaN: below nothing
+#pragma unroll
+                        for (int e = 0; e < 32; e++) {
+                            if (e < lo || e >= hi) continue;
+                            const float re = __uint_as_float(v[e]), im = two ? __uint_as_float(u[e]) : 0.f;
+                            const float d = diff(two ? re + im : re);
+                            least = fminf(least, d);
+                            v[e] = __float_as_uint(skipped ? -999.f : d);
+                            if (two) {
+                                const float d2 = diff(re - im);
+                                least = fminf(least, d2);
+                                u[e] = __float_as_uint(skipped ? -999.f : d2);
+                            }
+                        }
+                        const unsigned m = __reduce_min_sync(0xffffffffu, rok && !skipped ? f2key(least) : 0xffffffffu);
+                        if (lane == 0) atomicMin(&p.minkey[b], m);
+                        lo = hi;
+                    }
+                    const int col = col0 + lane;
+                    const bool cok = col < p.ncols;
+                    const int sb = cok ? col / p.T : 0;
+                    float* const dst = outp + (size_t)sb * ks * p.T + (col - sb * p.T);
+#pragma unroll 1
+                    for (int set = 0; set < (two ? 2 : 1); set++) {
+                        if (set == 0) {
+#pragma unroll
+                            for (int j = 0; j < 32; j++) sbuf[epi_at(lane, j)] = __uint_as_float(v[j]);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; j++) sbuf[epi_at(lane, j)] = __uint_as_float(u[j]);
+                        }
+                        __syncwarp();
+                        const int oo = (int)og + (set ? p.half : 0);
+#pragma unroll 8
+                        for (int r = 0; r < 32; r++) {
+                            const int o = __shfl_sync(0xffffffffu, oo, r);
+                            if (cok && (rows >> r & 1u)) dst[(size_t)o * p.T] = sbuf[epi_at(r, lane)];
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+            for (int c = 0; c < (p.mode == 1 && emit ? nchunk : 0); c++) {
                 uint32_t v[32];
                 tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(abuf * TN + c * 32), v);
                 if (other) {
@@ -412,54 +527,29 @@ k_diff2_tc(const CUtensorMap* __restrict__ maps, int ia, int ib, TcParams p)
                         v[e] = __float_as_uint(__uint_as_float(v[e]) + __ldcg(other + (size_t)c * 1024 + e * 32 + lane));
                 }
 #pragma unroll
-                for (int j = 0; j < 32; j++) sbuf[lane * EPI_LD + j] = __uint_as_float(v[j]);
+                for (int j = 0; j < 32; j++) sbuf[epi_at(lane, j)] = __uint_as_float(v[j]);
                 __syncwarp();
                 unsigned lmin = 0xffffffffu;
-                int b;
-                if (p.mode == 0) {
-                    // lane = column within the chunk; rows walk the warp's 32 TMEM lanes
-                    const int col = n0 + c * 32 + lane;
-                    const bool cok = col < p.ncols;
-                    b = cok ? col / p.T : 0;
-                    const int t = cok ? col - b * p.T : 0;
-                    const float c0 = (cok && !p.raw) ? p.c0[b] : 0.f;  // raw mode has no c0 array
-                    for (int r = 0; r < 32; r++) {
-                        const int oc = mt * TM + q * 32 + r;
-                        if (!cok || oc >= p.KO) continue;
-                        const size_t og = (size_t)p.row0 + oc;
-                        float d;
-                        if (p.raw) {
-                            d = sbuf[r * EPI_LD + lane];
-                        } else if (p.skip[og]) {
-                            d = -999.f;
-                        } else {
-                            d = c0 + p.norms[(size_t)b * ks + og] - sbuf[r * EPI_LD + lane];
-                            lmin = min(lmin, f2key(d));
-                        }
-                        outp[((size_t)b * ks + og) * p.T + t] = d;
+                // proposal tile: column = translation; the warp's 32 rows are proposals of
+                // one particle (kslot a multiple of 32)
+                const int t = c * 32 + lane;
+                const int bp = (q * 32) / p.kslot;
+                const int b = bfirst + bp;
+                const bool cok = t < p.T && bp < p.ppt && b < p.ncols;
+                for (int r = 0; r < 32; r++) {
+                    const int j = q * 32 + r - bp * p.kslot;
+                    const int skip_r = __shfl_sync(0xffffffffu, my_skip, r);
+                    const float cn_r = __shfl_sync(0xffffffffu, my_norm, r);
+                    if (!cok || j >= p.KO) continue;
+                    const size_t pj = (size_t)b * p.KO + j;
+                    float d;
+                    if (skip_r) {
+                        d = -999.f;
+                    } else {
+                        d = cn_r - sbuf[epi_at(r, lane)];
+                        lmin = min(lmin, f2key(d));
                     }
-                } else {
-                    // proposal tile: column = translation; the warp's 32 rows are proposals of
-                    // one particle (kslot a multiple of 32)
-                    const int t = c * 32 + lane;
-                    const int bp = (q * 32) / p.kslot;
-                    b = bfirst + bp;
-                    const bool cok = t < p.T && bp < p.ppt && b < p.ncols;
-                    for (int r = 0; r < 32; r++) {
-                        const int j = q * 32 + r - bp * p.kslot;
-                        const int skip_r = __shfl_sync(0xffffffffu, my_skip, r);
-                        const float cn_r = __shfl_sync(0xffffffffu, my_norm, r);
-                        if (!cok || j >= p.KO) continue;
-                        const size_t pj = (size_t)b * p.KO + j;
-                        float d;
-                        if (skip_r) {
-                            d = -999.f;
-                        } else {
-                            d = cn_r - sbuf[r * EPI_LD + lane];
-                            lmin = min(lmin, f2key(d));
-                        }
-                        p.d2c[pj * p.T + t] = d;
-                    }
+                    p.d2c[pj * p.T + t] = d;
                 }
                 if (lmin != 0xffffffffu) atomicMin(&wmin[b - bfirst], lmin);
                 __syncwarp();
@@ -467,11 +557,8 @@ k_diff2_tc(const CUtensorMap* __restrict__ maps, int ia, int ib, TcParams p)
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty_bar[abuf]);
-            for (int i = lane; i < TN + 2; i += 32) {
-                const int b = bfirst + i;
-                if (wmin[i] != 0xffffffffu && (p.mode == 0 ? b * p.T < p.ncols : b < p.ncols))
-                    atomicMin(&p.minkey[b], wmin[i]);
-            }
+            if (p.mode == 1 && lane < 2 && wmin[lane] != 0xffffffffu && bfirst + lane < p.ncols)
+                atomicMin(&p.minkey[bfirst + lane], wmin[lane]);
             __syncwarp();
         }
     }
@@ -494,40 +581,52 @@ __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bflo
 // to rpad and elements beyond nk zero.  The same values as k_project followed by k_split_proj
 // and k_split_norm_proj (one project_window_pixel each), without the FP32 table in between.
 __global__ void __launch_bounds__(256) k_project_split(cudaTextureObject_t mdl, Volume v,
-                                                       const double* __restrict__ eul, int rows, int rpad, int s,
-                                                       const int* __restrict__ kpix, int nk, int kh, int kn,
-                                                       __nv_bfloat162* __restrict__ ph, __nv_bfloat162* __restrict__ pl,
+                                                       const double* __restrict__ eul, int h0, int rows, int rpad, int s,
+                                                       const int* __restrict__ kpix, int nk, int kh, int kn, int half,
+                                                       __nv_bfloat16* __restrict__ ph, __nv_bfloat16* __restrict__ pl,
                                                        __nv_bfloat16* __restrict__ nh, __nv_bfloat16* __restrict__ nl)
 {
     const int r = blockIdx.y;
     const int kk = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rpad || kk >= kn) return;
     float2 z = make_float2(0.f, 0.f);
-    if (r < rows && kk < nk) z = project_window_pixel(mdl, v, eul + 9 * (size_t)r, kpix[kk], s);
+    if (r < rows && kk < nk) z = project_window_pixel(mdl, v, eul + 9 * (size_t)pair_row(h0 + r, half), kpix[kk], s);
     if (kk < kh) {
-        __nv_bfloat16 h0, l0, h1, l1;
-        split_bf16(z.x, h0, l0);
+        const size_t o = (size_t)r * 2 * kh;
+        __nv_bfloat16 h0_, l0, h1, l1;
+        split_bf16(z.x, h0_, l0);
         split_bf16(z.y, h1, l1);
-        ph[(size_t)r * kh + kk] = __halves2bfloat162(h0, h1);
-        pl[(size_t)r * kh + kk] = __halves2bfloat162(l0, l1);
+        if (half) {
+            ph[o + pair_elem(kk, 0, half)] = h0_;
+            ph[o + pair_elem(kk, 1, half)] = h1;
+            pl[o + pair_elem(kk, 0, half)] = l0;
+            pl[o + pair_elem(kk, 1, half)] = l1;
+        } else {
+            *reinterpret_cast<__nv_bfloat162*>(ph + o + 2 * kk) = __halves2bfloat162(h0_, h1);
+            *reinterpret_cast<__nv_bfloat162*>(pl + o + 2 * kk) = __halves2bfloat162(l0, l1);
+        }
     }
     split_bf16(z.x * z.x + z.y * z.y, nh[(size_t)r * kn + kk], nl[(size_t)r * kn + kk]);
 }
 
 // projections (K*O x P complex) -> Ph/Pl (m_pad x kdim bf16), zero padded
 __global__ void k_split_proj(const float2* __restrict__ proj, int rows, int P, const int* __restrict__ kpix, int nk,
-                             int kdim, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, long long total)
+                             int kdim, int half, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
+                             long long total)
 {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long r = i / (kdim / 2);
         const int kk = (int)(i - r * (kdim / 2));
         float2 v = make_float2(0.f, 0.f);
-        if (r < rows && kk < nk) v = proj[r * P + kpix[kk]];
+        if (r < rows && kk < nk) v = proj[(size_t)pair_row((int)r, half) * P + kpix[kk]];
         __nv_bfloat16 h0, l0, h1, l1;
         split_bf16(v.x, h0, l0);
         split_bf16(v.y, h1, l1);
-        reinterpret_cast<__nv_bfloat162*>(hi)[i] = __halves2bfloat162(h0, h1);
-        reinterpret_cast<__nv_bfloat162*>(lo)[i] = __halves2bfloat162(l0, l1);
+        const size_t e0 = (size_t)r * kdim + pair_elem(kk, 0, half), e1 = (size_t)r * kdim + pair_elem(kk, 1, half);
+        hi[e0] = h0;
+        hi[e1] = h1;
+        lo[e0] = l0;
+        lo[e1] = l1;
     }
 }
 
@@ -538,7 +637,7 @@ __global__ void k_split_proj(const float2* __restrict__ proj, int rows, int P, c
 __global__ void __launch_bounds__(128) k_split_img(const float2* __restrict__ cvec, const float2* __restrict__ ab,
                                                    int ncols, int nrows, int T, int P, const int* __restrict__ kpix,
                                                    int nk, int kdim, __nv_bfloat16* __restrict__ hi,
-                                                   __nv_bfloat16* __restrict__ lo, const int* gate, int swz)
+                                                   __nv_bfloat16* __restrict__ lo, const int* gate, int swz, int half)
 {
     if (gate && *gate != 0) return;
     const int nv = kdim / 8;  // groups of 4 complex values
@@ -551,7 +650,7 @@ __global__ void __launch_bounds__(128) k_split_img(const float2* __restrict__ cv
         uint4* dh = reinterpret_cast<uint4*>(hi);
         uint4* dl = reinterpret_cast<uint4*>(lo);
         for (int g = threadIdx.x; g < nv; g += blockDim.x) {
-            __nv_bfloat162 h[4], l[4];
+            __align__(16) __nv_bfloat162 h[4], l[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const int kk = 4 * g + e;
@@ -569,8 +668,26 @@ __global__ void __launch_bounds__(128) k_split_img(const float2* __restrict__ cv
                 __nv_bfloat16 h0, l0, h1, l1;
                 split_bf16(v.x, h0, l0);
                 split_bf16(v.y, h1, l1);
-                h[e] = __halves2bfloat162(h0, h1);
-                l[e] = __halves2bfloat162(l0, l1);
+                if (half) {   // h, l: four real parts, four imaginary
+                    reinterpret_cast<__nv_bfloat16*>(h)[e] = h0;
+                    reinterpret_cast<__nv_bfloat16*>(h)[4 + e] = h1;
+                    reinterpret_cast<__nv_bfloat16*>(l)[e] = l0;
+                    reinterpret_cast<__nv_bfloat16*>(l)[4 + e] = l1;
+                } else {
+                    h[e] = __halves2bfloat162(h0, h1);
+                    l[e] = __halves2bfloat162(l0, l1);
+                }
+            }
+            if (half) {
+                const size_t o = ((size_t)col * kdim + pair_elem(4 * g, 0, half)) / 4;
+                const uint4 hv = *reinterpret_cast<const uint4*>(h), lv = *reinterpret_cast<const uint4*>(l);
+                uint2* eh = reinterpret_cast<uint2*>(hi) + o;
+                uint2* el = reinterpret_cast<uint2*>(lo) + o;
+                eh[0] = make_uint2(hv.x, hv.y);
+                eh[16] = make_uint2(hv.z, hv.w);   // 64 elements on
+                el[0] = make_uint2(lv.x, lv.y);
+                el[16] = make_uint2(lv.z, lv.w);
+                continue;
             }
             const size_t o = swz ? swz_offset(col, 8 * g, nrows) / 8 : (size_t)col * (kdim / 8) + g;
             dh[o] = *reinterpret_cast<const uint4*>(h);
@@ -581,15 +698,15 @@ __global__ void __launch_bounds__(128) k_split_img(const float2* __restrict__ cv
 
 // |projection|^2 (K*O x P) -> hi/lo (m_pad x kn), zero padded
 __global__ void k_split_norm_proj(const float2* __restrict__ proj, int rows, int P, const int* __restrict__ kpix,
-                                  int nk, int kn, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
-                                  long long total)
+                                  int nk, int kn, int half, __nv_bfloat16* __restrict__ hi,
+                                  __nv_bfloat16* __restrict__ lo, long long total)
 {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long r = i / kn;
         const int kk = (int)(i - r * kn);
         float v = 0.f;
         if (r < rows && kk < nk) {
-            const float2 z = proj[r * P + kpix[kk]];
+            const float2 z = proj[(size_t)pair_row((int)r, half) * P + kpix[kk]];
             v = z.x * z.x + z.y * z.y;
         }
         split_bf16(v, hi[i], lo[i]);
@@ -620,8 +737,43 @@ int sms()
 
 bool tc_supported() { return true; }
 
-size_t tc_kdim(int nk) { return (size_t)((2 * nk + TK - 1) / TK) * TK; }
 size_t tc_kn(int nk) { return (size_t)((nk + TK - 1) / TK) * TK; }
+size_t tc_kdim(int nk, int half) { return half ? 2 * tc_kn(nk) : (size_t)((2 * nk + TK - 1) / TK) * TK; }
+
+// largest |m(0, y, z) - conj m(0, -y, -z)| and |m| of the x = 0 plane, as keys of positive floats
+__global__ void k_plane_asym(const float2* __restrict__ mdl, Volume v, unsigned* out)
+{
+    const int n = v.ydim * v.zdim;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int y = i % v.ydim + v.inity, z = v.ref_dim == 3 ? i / v.ydim + v.initz : 0;
+        const int my = -y - v.inity, mz = v.ref_dim == 3 ? -z - v.initz : 0;
+        if (my < 0 || my >= v.ydim || mz < 0 || mz >= v.zdim) continue;
+        const float2 a = mdl[(size_t)i * v.xdim], c = mdl[((size_t)mz * v.ydim + my) * v.xdim];
+        const float d = fmaxf(fabsf(a.x - c.x), fabsf(a.y + c.y)), m = fmaxf(fabsf(a.x), fabsf(a.y));
+        atomicMax(&out[0], d == d ? __float_as_uint(d) : 0x7f800000u);
+        atomicMax(&out[1], m == m ? __float_as_uint(m) : 0x7f800000u);
+    }
+}
+
+bool tc_planes_hermitian(const Volume& v, const float2* mdl, cudaStream_t st)
+{
+    unsigned* d = nullptr;
+    unsigned h[2] = {0, 0};
+    T2B_CUDA(cudaMalloc(&d, sizeof(h)));
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(h), st);
+    if (e == cudaSuccess) {
+        k_plane_asym<<<64, 256, 0, st>>>(mdl, v, d);
+        e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, st);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d);
+    T2B_CUDA(e);
+    float asym, most;
+    std::memcpy(&asym, &h[0], sizeof(float));
+    std::memcpy(&most, &h[1], sizeof(float));
+    return std::isfinite(most) && asym <= 1e-6f * most;
+}
+
 
 // descriptor slots in op.maps (TC_MAP_SLOTS of 128 bytes).  The image and w2 operands have one pair for each
 // box height below 256: MAP_IHN + 2 (rows / 32 - 1) and MAP_WHN + 2 (rows / 32 - 1).
@@ -637,6 +789,9 @@ void tc_encode(void* ptr, int rows, int kdim, bool a_side, void* out128, int box
     const CUtensorMap m = make_map(ptr, rows, kdim, box_rows > 0 ? box_rows : (a_side ? TM : TN));
     std::memcpy(out128, &m, sizeof(m));
 }
+
+// operand rows of every orientation
+static int op_rows(const Tables& tb) { return tb.half ? tb.K * tb.O / 2 : tb.K * tb.O; }
 
 void tc_prepare_projections(const Tables& tb, TcOperands& op, cudaStream_t st)
 {
@@ -662,23 +817,23 @@ void tc_prepare_projections(const Tables& tb, TcOperands& op, cudaStream_t st)
         nar[2 * BOXES + 2 * i + 1] = make_map(op.wl, op.b_pad, op.kn, box);
     }
     T2B_CUDA(cudaMemcpy(static_cast<unsigned char*>(op.maps) + 128 * MAP_IHN, nar, sizeof(nar), cudaMemcpyHostToDevice));
-    const int rows = op.chunk > 0 ? op.chunk : tb.K * tb.O;
+    const int rows = op.chunk > 0 ? op.chunk : op_rows(tb);
     // sizes were fixed when the operand buffers were allocated
-    T2B_REQUIRE(op.m_pad == (rows + TM - 1) / TM * TM && op.kdim == (int)tc_kdim(tb.nk), T2B_ERR_STATE,
+    T2B_REQUIRE(op.m_pad == (rows + TM - 1) / TM * TM && op.kdim == (int)tc_kdim(tb.nk, tb.half), T2B_ERR_STATE,
                 "tensor-core operand sizes do not match their allocation");
     if (op.chunk == 0) tc_split_chunk(tb, op, rows, st);   // chunked: split per chunk in each batch
 }
 
 void tc_project_split(const Tables& tb, TcOperands& op, cudaTextureObject_t mtex, const Volume& v, const double* eul,
-                      int rows, cudaStream_t st)
+                      int h0, int rows, cudaStream_t st)
 {
     T2B_REQUIRE(op.bh && op.nh && rows >= 1 && rows <= op.m_pad && op.kn >= op.kdim / 2, T2B_ERR_STATE,
                 "tensor-core operands not allocated");
     const int rpad = (rows + TM - 1) / TM * TM;
     dim3 grid((op.kn + 255) / 256, rpad);
-    k_project_split<<<grid, 256, 0, st>>>(mtex, v, eul, rows, rpad, tb.s, tb.kpix, tb.nk,
-                                          op.kdim / 2, op.kn,
-                                          (__nv_bfloat162*)op.bh, (__nv_bfloat162*)op.bl, (__nv_bfloat16*)op.nh,
+    k_project_split<<<grid, 256, 0, st>>>(mtex, v, eul, h0, rows, rpad, tb.s, tb.kpix, tb.nk,
+                                          op.kdim / 2, op.kn, tb.half,
+                                          (__nv_bfloat16*)op.bh, (__nv_bfloat16*)op.bl, (__nv_bfloat16*)op.nh,
                                           (__nv_bfloat16*)op.nl);
     T2B_CUDA(cudaGetLastError());
 }
@@ -689,10 +844,10 @@ void tc_split_chunk(const Tables& tb, TcOperands& op, int rows, cudaStream_t st)
 {
     T2B_REQUIRE(op.bh && op.bl && rows >= 1 && rows <= op.m_pad, T2B_ERR_STATE, "tensor-core operands not allocated");
     const long long rpad = (rows + TM - 1) / TM * TM;
-    k_split_proj<<<4 * sms(), 256, 0, st>>>(tb.proj_c, rows, tb.P, tb.kpix, tb.nk, op.kdim, (__nv_bfloat16*)op.bh,
+    k_split_proj<<<4 * sms(), 256, 0, st>>>(tb.proj_c, rows, tb.P, tb.kpix, tb.nk, op.kdim, tb.half, (__nv_bfloat16*)op.bh,
                                             (__nv_bfloat16*)op.bl, rpad * op.kdim / 2);
     T2B_REQUIRE(op.nh && op.nl && op.kn == (int)tc_kn(tb.nk), T2B_ERR_STATE, "norm operands not allocated");
-    k_split_norm_proj<<<4 * sms(), 256, 0, st>>>(tb.proj_c, rows, tb.P, tb.kpix, tb.nk, op.kn, (__nv_bfloat16*)op.nh,
+    k_split_norm_proj<<<4 * sms(), 256, 0, st>>>(tb.proj_c, rows, tb.P, tb.kpix, tb.nk, op.kn, tb.half, (__nv_bfloat16*)op.nh,
                                                  (__nv_bfloat16*)op.nl, rpad * op.kn);
     T2B_CUDA(cudaGetLastError());
 }
@@ -721,6 +876,16 @@ static void column_tiles(int cols, int& n_tiles, int& tn)
     tn = ((cols + n_tiles - 1) / n_tiles + 31) / 32 * 32;
 }
 
+// As many rows as fill whole waves of tiles, one tile an SM (32 particles x 49 shifts: 7 column tiles, so
+// 126 orientation tiles of 16,128 rows are 5.96 waves, the 16,384 that would fit 6.05).
+int tc_chunk_rows(const TcOperands& op, int cols)
+{
+    int n_tiles, tn;
+    column_tiles(cols, n_tiles, tn);
+    const int fit = op.chunk / TM, waves = fit * n_tiles / sms();
+    return waves >= 1 ? std::min(op.chunk, std::max(1, waves * sms() / n_tiles) * TM) : op.chunk;
+}
+
 // N[b][oc] = sum_p w2[b][p] |P_oc[p]|^2 with the same split-BF16 tensor-core kernel
 void tc_launch_norms(const Tables& tb, const Work& w, TcOperands& op, cudaStream_t st, const int* gate, int gate_run,
                      RowChunk ch, bool split_w2)
@@ -739,9 +904,10 @@ void tc_launch_norms(const Tables& tb, const Work& w, TcOperands& op, cudaStream
     p.tn = tn == TN ? 0 : tn;
     p.kblocks = op.kn / TK;
     p.raw = 1;
-    p.KO = ch.rows ? ch.rows : tb.K * tb.O;
+    p.KO = ch.rows ? ch.rows : op_rows(tb);
+    p.half = tb.half;
     p.row0 = ch.row0;
-    p.ko_stride = ch.rows ? tb.K * tb.O : 0;
+    p.ko_stride = tb.K * tb.O;
     p.T = 1;
     p.ncols = w.n;
     p.skip = tb.skip;
@@ -761,7 +927,7 @@ void tc_split_images(const Tables& tb, const Work& w, TcOperands& op, cudaStream
     T2B_REQUIRE(n_pad <= op.n_pad, T2B_ERR_ARG, "batch larger than the tensor-core workspace");
     k_split_img<<<std::min(n_pad, 16 * sms()), 128, 0, st>>>(w.cvec, tb.ab_c, ncols, n_pad, tb.T, tb.P, tb.kpix, tb.nk,
                                                             op.kdim, (__nv_bfloat16*)op.ah, (__nv_bfloat16*)op.al,
-                                                            gate, 0);
+                                                            gate, 0, tb.half);
     T2B_CUDA(cudaGetLastError());
 }
 
@@ -770,7 +936,7 @@ void tc_split_phases(const Tables& tb, const TcOperands& op, int rows, void* hi,
     T2B_REQUIRE(rows >= tb.T, T2B_ERR_ARG, "phase operand rows");
     T2B_REQUIRE(rows % 8 == 0, T2B_ERR_ARG, "phase operand rows");
     k_split_img<<<std::min(rows, 16 * sms()), 128, 0, st>>>(nullptr, tb.ab_c, tb.T, rows, tb.T, tb.P, tb.kpix, tb.nk,
-                                                           op.kdim, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, nullptr, 1);
+                                                           op.kdim, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, nullptr, 1, 0);
     T2B_CUDA(cudaGetLastError());
 }
 
@@ -790,9 +956,10 @@ void tc_launch_diff2(const Tables& tb, const Work& w, TcOperands& op, cudaStream
     p.tn = tn == TN ? 0 : tn;
     p.group = op.group_m;
     p.kblocks = op.kdim / TK;
-    p.KO = ch.rows ? ch.rows : tb.K * tb.O;
+    p.KO = ch.rows ? ch.rows : op_rows(tb);
+    p.half = tb.half;
     p.row0 = ch.row0;
-    p.ko_stride = ch.rows ? tb.K * tb.O : 0;
+    p.ko_stride = tb.K * tb.O;
     p.T = tb.T;
     p.ncols = ncols;
     p.c0 = w.c0;
@@ -923,7 +1090,9 @@ void tc_launch_audit_norms(const Tables& tb, TcOperands& op, int na_max, float* 
     p.n_tiles = (na_max + 31) / 32;
     p.kblocks = op.kn / TK;
     p.raw = 1;
-    p.KO = tb.K * tb.O;
+    p.KO = op_rows(tb);
+    p.half = tb.half;
+    p.ko_stride = tb.K * tb.O;
     p.T = 1;
     p.ncols = na_max;
     p.skip = tb.skip;
@@ -968,7 +1137,9 @@ void tc_launch_audit(const Tables& tb, TcOperands& op, int na_max, const int* na
     column_tiles(na_max * tb.T, p.n_tiles, tf);
     p.tn = tf == TN ? 0 : tf;
     p.kblocks = op.kdim / TK;
-    p.KO = tb.K * tb.O;
+    p.KO = op_rows(tb);
+    p.half = tb.half;
+    p.ko_stride = tb.K * tb.O;
     p.T = tb.T;
     p.ncols = na_max * tb.T;
     p.c0 = c0a;

@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(1024) k_rescore_select(const int* __restrict__
 // tensor-core tile of 128 rows and one k-block is one contiguous 16 KB block).
 // Runs while *gate != 0.
 __global__ void __launch_bounds__(128) k_prop_gather(Work w, int P, const int* __restrict__ kpix, int nk, int kslot,
-                                                     int rows, int kdim,
+                                                     int rows, int kdim, int half,
                                                      const bf16* __restrict__ bh, const bf16* __restrict__ bl,
                                                      bf16* __restrict__ ph, bf16* __restrict__ pl, float* __restrict__ nprop)
 {
@@ -575,17 +575,40 @@ __global__ void __launch_bounds__(128) k_prop_gather(Work w, int P, const int* _
     const size_t row = (size_t)b * kslot + j;
     float acc = 0.f;
     {
-        const uint4* sh = reinterpret_cast<const uint4*>(bh + oc * kdim);
-        const uint4* sl = reinterpret_cast<const uint4*>(bl + oc * kdim);
+        // the operand's row of this orientation; half a turn on, its conjugate
+        const bool conj = half && oc % (2 * half) >= (size_t)half;
+        const size_t src = (half ? oc / (2 * half) * half + oc % half : oc) * kdim;
+        const uint4* sh = reinterpret_cast<const uint4*>(bh + src);
+        const uint4* sl = reinterpret_cast<const uint4*>(bl + src);
+        const uint2* ph2 = reinterpret_cast<const uint2*>(bh + src);
+        const uint2* pl2 = reinterpret_cast<const uint2*>(bl + src);
         const int4* kp4 = reinterpret_cast<const int4*>(kpix);
         const float2* cb = w.cvec + (size_t)b * P;
         const float* w2b = w.w2 + (size_t)b * P;
         uint4* dh = reinterpret_cast<uint4*>(ph);
         uint4* dl = reinterpret_cast<uint4*>(pl);
         for (int v = threadIdx.x; v < kdim / 8; v += blockDim.x) {
-            const uint4 hv = sh[v], lv = sl[v];
-            const __nv_bfloat162* hp = reinterpret_cast<const __nv_bfloat162*>(&hv);
-            const __nv_bfloat162* lp = reinterpret_cast<const __nv_bfloat162*>(&lv);
+            __align__(16) float2 pvs[4];
+            if (half) {
+                const int g = pair_elem(4 * v, 0, half) / 4;
+                const uint2 hv[2] = {ph2[g], ph2[g + 16]}, lv[2] = {pl2[g], pl2[g + 16]};   // real, imaginary
+                const bf16* hp = reinterpret_cast<const bf16*>(hv);
+                const bf16* lp = reinterpret_cast<const bf16*>(lv);
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float im = __bfloat162float(hp[4 + e]) + __bfloat162float(lp[4 + e]);
+                    pvs[e] = make_float2(__bfloat162float(hp[e]) + __bfloat162float(lp[e]), conj ? -im : im);
+                }
+            } else {
+                const uint4 hv = sh[v], lv = sl[v];
+                const __nv_bfloat162* hp = reinterpret_cast<const __nv_bfloat162*>(&hv);
+                const __nv_bfloat162* lp = reinterpret_cast<const __nv_bfloat162*>(&lv);
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float2 hf = __bfloat1622float2(hp[e]), lf = __bfloat1622float2(lp[e]);
+                    pvs[e] = make_float2(hf.x + lf.x, hf.y + lf.y);
+                }
+            }
             // pixel indices of these 4 values: one 16-byte load when all are in radius
             int kk[4];
             if (4 * v + 3 < nk) {
@@ -600,8 +623,7 @@ __global__ void __launch_bounds__(128) k_prop_gather(Work w, int P, const int* _
             for (int e = 0; e < 4; e++) {
                 float2 a = make_float2(0.f, 0.f);
                 if (4 * v + e < nk) {
-                    const float2 hf = __bfloat1622float2(hp[e]), lf = __bfloat1622float2(lp[e]);
-                    const float2 pv = make_float2(hf.x + lf.x, hf.y + lf.y);
+                    const float2 pv = pvs[e];
                     const float2 c = cb[kk[e]];
                     a = make_float2(pv.x * c.x + pv.y * c.y, pv.y * c.x - pv.x * c.y);
                     acc += w2b[kk[e]] * (pv.x * pv.x + pv.y * pv.y);
@@ -651,7 +673,7 @@ __global__ void k_audit_begin(PropState* ps, int* audit_b, int n, int every, int
 // audit slots
 __global__ void __launch_bounds__(256) k_audit_operands(const PropState* ps, const int* audit_b, Work w, int T, int P,
                                                         const int* __restrict__ kpix, int nk, int kn,
-                                                        int kdim, const float2* __restrict__ ab,
+                                                        int kdim, int half, const float2* __restrict__ ab,
                                                         bf16* __restrict__ iah, bf16* __restrict__ ial,
                                                         bf16* __restrict__ wah, bf16* __restrict__ wal,
                                                         float* __restrict__ c0a)
@@ -664,8 +686,6 @@ __global__ void __launch_bounds__(256) k_audit_operands(const PropState* ps, con
         const size_t dst = ((size_t)a * T + t) * kdim;
         const float2* cb = w.cvec + (size_t)b * P;
         const float2* at = ab + (size_t)t * P;
-        __nv_bfloat162* dh = reinterpret_cast<__nv_bfloat162*>(iah + dst);
-        __nv_bfloat162* dl = reinterpret_cast<__nv_bfloat162*>(ial + dst);
         for (int k = threadIdx.x; k < kdim / 2; k += blockDim.x) {
             float2 v = make_float2(0.f, 0.f);
             if (k < nk) {
@@ -674,9 +694,11 @@ __global__ void __launch_bounds__(256) k_audit_operands(const PropState* ps, con
                 v = make_float2(c.x * e.x - c.y * e.y, c.x * e.y + c.y * e.x);
             }
             const bf16 hx = __float2bfloat16_rn(v.x), hy = __float2bfloat16_rn(v.y);
-            dh[k] = __halves2bfloat162(hx, hy);
-            dl[k] = __halves2bfloat162(__float2bfloat16_rn(v.x - __bfloat162float(hx)),
-                                       __float2bfloat16_rn(v.y - __bfloat162float(hy)));
+            const size_t e0 = dst + pair_elem(k, 0, half), e1 = dst + pair_elem(k, 1, half);
+            iah[e0] = hx;
+            iah[e1] = hy;
+            ial[e0] = __float2bfloat16_rn(v.x - __bfloat162float(hx));
+            ial[e1] = __float2bfloat16_rn(v.y - __bfloat162float(hy));
         }
     } else {
         for (int k = threadIdx.x; k < kn; k += blockDim.x) {
@@ -2052,7 +2074,7 @@ void proposal_audit_contract(t2b_ctx* c, const Work& w, cudaStream_t st, cudaEve
     TcOperands& op = c->tc;
     k_audit_begin<<<1, 256, 0, st>>>(N.ps, N.audit_b, w.n, N.every, N.na_max, N.minkeya, N.asum, w.r_audit);
     k_audit_operands<<<dim3(tb.T + 1, N.na_max), 256, 0, st>>>(N.ps, N.audit_b, w, tb.T, tb.P, tb.kpix, tb.nk, op.kn,
-                                                               op.kdim, tb.ab_c, (bf16*)N.ia_h,
+                                                               op.kdim, tb.half, tb.ab_c, (bf16*)N.ia_h,
                                                                (bf16*)N.ia_l, (bf16*)N.wa_h, (bf16*)N.wa_l, N.c0a);
     tc_launch_audit_norms(tb, op, N.na_max, N.norma, w.err, st);
     T2B_CUDA(cudaGetLastError());
@@ -2078,7 +2100,7 @@ void proposal_coarse(t2b_ctx* c, const Work& w, cudaStream_t st, cudaEvent_t* ev
     ProposalNet& N = *c->net;
     const Tables& tb = c->tb;
     const TcOperands& op = c->tc;
-    k_prop_gather<<<dim3(N.kprop, w.n), 128, 0, st>>>(w, tb.P, tb.kpix, tb.nk, N.kslot, N.pg_rows, op.kdim,
+    k_prop_gather<<<dim3(N.kprop, w.n), 128, 0, st>>>(w, tb.P, tb.kpix, tb.nk, N.kslot, N.pg_rows, op.kdim, tb.half,
                                                       (const bf16*)op.bh, (const bf16*)op.bl, (bf16*)N.pg_h,
                                                       (bf16*)N.pg_l, N.nprop);
     T2B_CUDA(cudaGetLastError());

@@ -122,6 +122,7 @@ struct Tables {
     const unsigned long long* mtex; // K: texture objects over the models' 3D arrays (on-the-fly
                                     // projection, project_pixel.cuh)
     const Volume* mvol;       // K: their geometry
+    int half;                 // split-BF16: orientation o and o + half (of 2 half in-plane angles) are half a turn apart; 0: unpaired
 };
 
 // Device views of the batch workspace.
@@ -228,22 +229,36 @@ struct TcOperands {
     int group_m = 16;         // orientation tiles per raster group of the dense and audit tiles
     int chunk = 0;            // > 0: the projection operands hold one chunk of this many rows
 };
-// One chunk of the coarse orientations: rows [row0, row0 + rows) of the K*O layout.
+// One chunk of the coarse orientations: operand rows [row0, row0 + rows) (of K*O, paired K*O / 2).
 struct RowChunk {
     int row0 = 0, rows = 0;   // rows == 0: every row (the resident operands)
 };
 constexpr int TC_MAP_SLOTS = 48;
-size_t tc_kdim(int nk);
+// Paired orientations (Tables::half > 0): the in-plane angle half a turn on sees the same slice with every
+// pixel's sign reversed, the complex conjugate, so one operand row serves both.  Operand row h belongs to
+// the orientations pair_row(h) and pair_row(h) + half; a row alternates 64 real parts and the
+// same pixels' 64 imaginary parts.  Unpaired (half == 0): row h is orientation h, parts interleaved.
+__host__ __device__ inline int pair_row(int h, int half) { return half ? h + h / half * half : h; }
+__host__ __device__ inline int pair_elem(int kk, int part, int half)
+{
+    return half ? (kk >> 6) * 128 + part * 64 + (kk & 63) : 2 * kk + part;
+}
+size_t tc_kdim(int nk, int half);
+// the models' x = 0 planes are Hermitian to rounding (what makes paired orientations conjugate there too)
+bool tc_planes_hermitian(const Volume& v, const float2* mdl, cudaStream_t st);
 void tc_prepare_projections(const Tables& tb, TcOperands& op, cudaStream_t st);
 // resident tables: split rows [0, rows) of tb.proj_c into the projection operands
 void tc_split_chunk(const Tables& tb, TcOperands& op, int rows, cudaStream_t st);
 // chunked: the projections of `rows` orientations (eul) of one model straight into the operands
+// (operand rows h0 .. h0 + rows of its orientations)
 void tc_project_split(const Tables& tb, TcOperands& op, cudaTextureObject_t mtex, const Volume& v, const double* eul,
-                      int rows, cudaStream_t st);
+                      int h0, int rows, cudaStream_t st);
 void tc_split_images(const Tables& tb, const Work& w, TcOperands& op, cudaStream_t st, const int* gate);
 void tc_launch_norms(const Tables& tb, const Work& w, TcOperands& op, cudaStream_t st, const int* gate = nullptr,
                      int gate_run = 0, RowChunk ch = RowChunk{}, bool split_w2 = true);
 size_t tc_kn(int nk);
+// chunked: operand rows of a chunk at `cols` columns
+int tc_chunk_rows(const TcOperands& op, int cols);
 void tc_launch_diff2(const Tables& tb, const Work& w, TcOperands& op, cudaStream_t st, const int* gate = nullptr,
                      int gate_run = 0, RowChunk ch = RowChunk{});
 bool tc_supported();
