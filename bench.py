@@ -1295,7 +1295,7 @@ def main():
             "scaling": "weak", "vs_baseline": None, "dtype": "f32+bf16x3/f64" if mode else "f32/f64",
             "data": "synthetic (seeded blob map, CTF, white noise; stands in for the reference's datasets)",
             "config": workload_config(), "particles_per_step": B,
-            "run": {"diff2": args.mode, "l2": "working set > L2 (bf16 hi/lo projection operands 0.97 GB per step)"},
+            "run": {"diff2": args.mode, "l2": "working set > L2 (projection operands per step: split-BF16 0.57 GB, plain FP32 table 0.97 GB)"},
             "e2e": e2e, "gpu_launches": timing["gpu_launches"], "clocks": clocks, "roofline": roof,
             "stage_ms": {n: float(v) for n, v in zip(
                 ["prep_network", "operands_audit_norms", "coarse_diff2", "coarse_weights", "fine", "fine_weights",
